@@ -16,8 +16,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmako_b200.so")
 SYNTH = os.path.join(HERE, "libmk_synth.so")
 
-CUDA_SOURCES = ["row_pipeline.cu", "aux_kernels.cu", "capi.cu", "row_sampler.cu"]
-CUDA_DEPS = ["row_pipeline.h", "device_expf.cuh", "ptx.cuh", "exp2_table.inc", "../../include/mako_b200.h"]
+CUDA_SOURCES = ["row_pipeline.cu", "flat_rows.cu", "aux_kernels.cu", "capi.cu", "row_sampler.cu"]
+CUDA_DEPS = ["row_pipeline.h", "device_expf.cuh", "list_chain.cuh", "row_common.cuh", "ptx.cuh", "exp2_table.inc", "../../include/mako_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -37,7 +37,9 @@
 #include "row_pipeline.h"
 
 #include "device_expf.cuh"
+#include "list_chain.cuh"
 #include "ptx.cuh"
+#include "row_common.cuh"
 
 #include <cfloat>
 #include <type_traits>
@@ -61,7 +63,6 @@ constexpr int kBmWords = 5120;  // history bitmap: one bit per column, vocabular
 constexpr uint32_t kMaxBitmapVocab = kBmWords * 32u;
 constexpr int kSortCap = 8192;  // 64-bit sort keys: they take the ring (64 KB) once the streaming is over
 constexpr uint32_t kBarSort = 3;         // named barrier of the sorting warps
-constexpr uint32_t kNucleusGuess = 24;  // top_p alone, first launch: the largest elements kept (the one-warp finish takes 32 candidates)
 #ifndef MK_PREFIX_TILES
 #define MK_PREFIX_TILES 4
 #endif
@@ -97,7 +98,9 @@ constexpr uint32_t kOffKeys = 0;                                  // kSortCap 64
 constexpr uint32_t kOffFinBitmap = kSortCap * 8u;                 // kBmWords words (also: the mass histogram)
 constexpr uint32_t kOffFinWpre = kOffFinBitmap + kBmWords * 4u;   // kBmWords 16-bit ranks
 constexpr uint32_t kOffFinOrd = kOffFinWpre + kBmWords * 2u;      // kSortCap 16-bit slots
-static_assert(kOffFinOrd + kSortCap * 2u <= kDynBytes, "finish layout fits");
+constexpr uint32_t kOffChain = kOffFinOrd + kSortCap * 2u;        // what the chains of a long list share
+using RowChain = ChainSmem<kThreads>;
+static_assert(kOffChain + sizeof(RowChain) <= kDynBytes, "finish layout fits");
 static_assert(kBins * 4u <= kBmWords * 4u, "mass histogram fits the finish bitmap area");
 
 // Bins of the histogram that bounds the k-th largest element of a row: monotone in the float order, fine where
@@ -134,118 +137,12 @@ __device__ __forceinline__ float hist_bin_floor(uint32_t b)
     return -__uint_as_float((((q >> 5) + 117u) << 23) | ((q & 31u) << 18));
 }
 
-struct RowCfg {
-    float temperature, inv_t, minp_eff, top_p;
-    uint32_t top_k;
-    uint32_t hist_k;    // the histogram bound keeps the hist_k largest elements
-    float rep, presence, frequency;
-    bool greedy, hist_mode, need_sum, use_topp, pen_active, optimistic;
-    float delta_w;      // keep elements with l >= running max - delta_w
-    bool force_none;    // inv_t is inf/NaN: no finite weight can exist
-};
-
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ float warp_max(float v)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
-}
-
-__device__ __forceinline__ RowCfg make_cfg(const mk_sampling_params& p, uint32_t n_vocab, int mode, uint32_t vp_k, int pass)
-{
-    RowCfg c;
-    c.temperature = p.temperature;
-    c.greedy = p.temperature <= 0.0f;                       // sampler.hpp:26
-    c.inv_t = __fdiv_rn(1.0f, p.temperature);               // sampler.cpp:29
-    c.minp_eff = (1.0f < p.min_p) ? 1.0f : p.min_p;         // std::min(min_p, 1.0f), sampler.cpp:34
-    c.top_p = p.top_p;
-    c.top_k = p.top_k;
-    c.rep = p.repetition_penalty;
-    c.presence = p.presence_penalty;
-    c.frequency = p.frequency_penalty;
-    c.pen_active = !(c.rep == 1.0f && c.presence == 0.0f && c.frequency == 0.0f);
-    c.use_topp = p.top_p < 1.0f;
-    c.hist_mode = !c.greedy && p.top_k > 0 && p.top_k < n_vocab;
-    // One more than top_k is kept, so that "more candidates than top_k" (which decides whether the reference
-    // truncates, and with it the order of the list, sampler.cpp:39) can be told from the kept elements alone.
-    c.hist_k = p.top_k + 1u;
-    const bool minp_on = c.minp_eff > 0.0f;
-    // The float total over "all candidates" is only needed when top_p is the only truncation.
-    c.need_sum = !c.greedy && c.use_topp && !minp_on && !c.hist_mode;
-    c.force_none = !c.greedy && (!(c.inv_t < __int_as_float(0x7f800000)) || !(c.inv_t == c.inv_t));
-    // top_p alone: the first launch bets that the nucleus lies within the kNucleusGuess largest elements and keeps
-    // only those (the top_k histogram bound, with no top_k cut afterwards); a row whose nucleus does not close within
-    // what was kept asks for the second pass, which keeps everything the mass bound allows.
-    c.optimistic = c.need_sum && pass == 0 && mode != kModeVpLocal && kNucleusGuess < n_vocab;
-    if (c.optimistic) {
-        c.hist_mode = true;
-        c.hist_k = kNucleusGuess;
-    }
-    if (mode == kModeVpLocal) {
-        c.hist_mode = vp_k < n_vocab;
-        c.top_k = vp_k;
-        c.hist_k = vp_k;
-        c.need_sum = true;
-        c.use_topp = false;
-        c.minp_eff = 0.0f;
-    }
-    // Distance below the row maximum, in units of (l - max) * inv_t, past which an element cannot be kept:
-    //   q == 0 below about -103.98 (float underflow of expf);
-    //   q < min_p below ln(min_p);
-    //   with top_p alone, an element with q < (1 - top_p) / n_vocab is outside the nucleus, because all such
-    //   elements together weigh less than (1 - top_p) * total (total >= 1: the maximum itself has q = 1).
-    float d = 104.2f;
-    if (mode != kModeVpLocal) {
-        if (minp_on)
-            d = fminf(d, -logf(c.minp_eff));
-        if (c.need_sum) {
-            float a = (1.0f - c.top_p) / (float)n_vocab;
-            a = fminf(a, 1.0f);
-            if (a > 0.0f)
-                d = fminf(d, -logf(a));
-        }
-    }
-    d = d * 1.001f + 1e-3f;
-    c.delta_w = d * fmaxf(c.temperature, 0.0f);
-    if (!(c.delta_w == c.delta_w))
-        c.delta_w = __int_as_float(0x7f800000);
-    return c;
-}
-
-// Threshold on the (edited) logit for the current running maximum; never -inf, so masked elements never pass.
-__device__ __forceinline__ float keep_threshold(const RowCfg& c, float m_run)
-{
-    if (c.force_none || !(m_run < __int_as_float(0x7f800000)))
-        return __int_as_float(0x7f800000); // no finite weight can exist (an infinite maximum makes l - max NaN or -inf)
-    const float t = m_run - c.delta_w - fabsf(m_run) * 1e-6f;
-    return fmaxf(t, -FLT_MAX);
-}
-
-// Penalties of one generated token with count n, exactly as sampler.cpp:24-27.
-__device__ __forceinline__ float penalise(float l, uint32_t n, const RowCfg& c)
-{
-    if (c.rep != 1.0f)
-        l = (l > 0.0f) ? __fdiv_rn(l, c.rep) : __fmul_rn(l, c.rep);
-    const float step = __fadd_rn(c.presence, __fmul_rn(c.frequency, (float)n));
-    return __fsub_rn(l, step);
-}
-
-__device__ __forceinline__ unsigned long long pack_by_weight(float q, uint32_t col)
-{
-    // ascending key order = (q descending, column ascending); q > 0 so its bit pattern is monotone
-    return ((unsigned long long)(~__float_as_uint(q)) << 32) | col;
-}
-__device__ __forceinline__ unsigned long long pack_by_column(float q, uint32_t col)
-{
-    return ((unsigned long long)col << 32) | __float_as_uint(q);
 }
 
 // Position of the n-th set bit (n = 0: the lowest) of a word that has more than n bits set: five halvings by
@@ -417,27 +314,10 @@ __device__ void merge_pass(const unsigned long long* src, unsigned long long* ds
     }
 }
 
-// Where a row's results go (the output pointers of the launch), for the steps that live out of line.
-struct RowOut {
-    int32_t* token;
-    float* prob;
-    uint32_t* flags;
-    uint32_t* n_cand;
-    int32_t* accepted;
-    float* total_out;
-    int32_t* cand_ids;
-    float* cand_q;
-    uint32_t cand_cap;
-    int32_t id_offset;
-    unsigned long long* timing;
-    int mode;
-};
-
 // More candidates than the shared-memory sort holds, and no truncation orders them: the draw walks them in ascending
-// id (sampler.cpp:64-73). The exact weights are laid out by column in scratch (`qrow`) and one thread adds and walks
-// them in the reference's order and precision; the other threads stage tiles for it (`stage`: two tiles of shared
-// memory). Writes the row's results. Whole CTA.
-__device__ __noinline__ void wide_id_ordered(Smem& s, float* stage, const uint2* scratch, float* qrow, uint32_t n_raw,
+// id (sampler.cpp:64-73). The exact weights are laid out by column in scratch (`qrow`, zero where there is no candidate)
+// and the chains run over all columns. Writes the row's results. Whole CTA.
+__device__ __noinline__ void wide_id_ordered(Smem& s, RowChain& cs, const uint2* scratch, float* qrow, uint32_t n_raw,
                                              uint32_t n, uint32_t V, float thr_final, float m, float inv_t, float minp_eff,
                                              uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
                                              const RowOut o)
@@ -454,116 +334,67 @@ __device__ __noinline__ void wide_id_ordered(Smem& s, float* stage, const uint2*
         if (q >= minp_eff && q > 0.0f)
             qrow[c.y] = q;
     }
-    __threadfence_block();
     __syncthreads();
-    const int32_t draft_col = (o.mode == kModeVerify) ? (draft_row - o.id_offset) : -1;
-    float total = 0.0f, q_draft = 0.0f;
-    // pass 0: float total (and the draft's weight); pass 1: the walk
-    float r = 0.0f, walk_total = 0.0f, eps = 0.0f;
-    int32_t tok = -1, last = -1, acc = 0;
-    float prob = 0.0f, last_q = 0.0f;
-    bool first = true, done = false, skip_draft = false;
-    uint32_t emitted = 0;
-    for (int pass = 0; pass < 2 && !done; ++pass) {
-        for (uint32_t t = 0; t * kTile < V && !done; ++t) {
-            const uint32_t base = t * kTile, n_t = min((uint32_t)kTile, V - base);
-            float* buf = stage + (t & 1) * kTile;
-            for (uint32_t e = tid; e < n_t; e += kThreads)
-                buf[e] = qrow[base + e];
-            __syncthreads();
-            if (tid == 0) {
-                if (pass == 0) {
-                    for (uint32_t e = 0; e < n_t; ++e) {
-                        const float q = buf[e];
-                        if (q > 0.0f) {
-                            total = __fadd_rn(total, q);
-                            if ((int32_t)(base + e) == draft_col)
-                                q_draft = q;
-                            if (emitted < o.cand_cap) {
-                                if (o.cand_ids) o.cand_ids[(size_t)row * o.cand_cap + emitted] = (int32_t)(base + e) + o.id_offset;
-                                if (o.cand_q) o.cand_q[(size_t)row * o.cand_cap + emitted] = q;
-                            }
-                            ++emitted;
-                        }
-                    }
-                } else {
-                    for (uint32_t e = 0; e < n_t && !done; ++e) {
-                        const float q = buf[e];
-                        if (!(q > 0.0f) || (skip_draft && (int32_t)(base + e) == draft_col))
-                            continue;
-                        last = (int32_t)(base + e);
-                        last_q = q;
-                        if (r < q) {
-                            tok = last;
-                            prob = __fdiv_rn(q, walk_total);
-                            if ((!first && r < eps) || __fsub_rn(q, r) < eps)
-                                s.flags = 1; // upper boundary: cleared below if this was the last candidate
-                            s.n_final = (!first && r < eps) ? 2u : 0u;
-                            done = true;
-                        } else {
-                            r = __fsub_rn(r, q);
-                            first = false;
-                        }
-                    }
-                }
+    if ((o.cand_ids || o.cand_q) && tid < 32u) { // the candidate list, as far as the caller wants it
+        uint32_t at = 0;
+        for (uint32_t c0 = 0; c0 < V && at < o.cand_cap; c0 += 32u) {
+            const float q = (c0 + tid < V) ? qrow[c0 + tid] : 0.0f;
+            const uint32_t have = __ballot_sync(0xffffffffu, q > 0.0f);
+            const uint32_t slot = at + (uint32_t)__popc(have & ((1u << tid) - 1u));
+            if (q > 0.0f && slot < o.cand_cap) {
+                if (o.cand_ids) o.cand_ids[(size_t)row * o.cand_cap + slot] = (int32_t)(c0 + tid) + o.id_offset;
+                if (o.cand_q) o.cand_q[(size_t)row * o.cand_cap + slot] = q;
             }
-            __syncthreads();
-            if (pass == 1) {
-                // the walking thread publishes "done" through shared memory
-                if (tid == 0)
-                    s.nsurv = done ? 0xffffffffu : n;
-                __syncthreads();
-                done = s.nsurv == 0xffffffffu;
-            }
-        }
-        if (pass == 0) {
-            // decide what the walk does (sampler.cpp:100-106 for verify)
-            if (tid == 0) {
-                walk_total = total;
-                if (o.mode == kModeVerify) {
-                    acc = __fmul_rn(u_row, total) < q_draft;
-                    if (acc) {
-                        tok = draft_col + o.id_offset;
-                        prob = __fdiv_rn(q_draft, total);
-                    } else {
-                        skip_draft = true;
-                        walk_total = __fsub_rn(total, q_draft);
-                    }
-                }
-                const float uu = (o.mode == kModeVerify) ? u2_row : u_row;
-                r = __fmul_rn(uu, walk_total);
-                eps = 1e-6f * walk_total;
-                s.n_final = 0;
-                s.flags = 0;
-                s.nsurv = (o.mode == kModeDistOnly || acc) ? 0xffffffffu : n;
-            }
-            __syncthreads();
-            done = s.nsurv == 0xffffffffu;
+            at += (uint32_t)__popc(have);
         }
     }
-    if (tid == 0) {
-        if (o.mode == kModeDistOnly) {
-            tok = -1;
-        } else if (tok < 0) { // rounding: the last candidate
-            tok = last;
-            prob = __fdiv_rn(last_q, walk_total);
-        } else if (!acc && o.mode != kModeDistOnly) {
-            // near-boundary report: lower boundary always counts; the upper one only if a candidate follows
-            bool more = false;
-            for (uint32_t c = (uint32_t)tok + 1; c < V && !more; ++c)
-                if (qrow[c] > 0.0f && !(skip_draft && (int32_t)c == draft_col))
-                    more = true;
-            if (s.n_final == 2u || (s.flags && more))
-                flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
-        }
-        if (o.token) o.token[row] = (tok >= 0 && !(acc)) ? tok + o.id_offset : tok;
-        if (o.prob) o.prob[row] = prob;
-        if (o.flags) o.flags[row] = flags;
-        if (o.n_cand) o.n_cand[row] = n;
-        if (o.accepted) o.accepted[row] = acc;
-        if (o.total_out) o.total_out[row] = total;
-        if (o.timing) o.timing[(size_t)row * 64 + 3] = global_ns();
+    const int64_t d = (int64_t)draft_row - o.id_offset;
+    const uint32_t draft_idx = (o.mode == kModeVerify && draft_row >= 0 && d >= 0 && d < (int64_t)V) ? (uint32_t)d : 0xffffffffu;
+    draw_long<kThreads>(cs, V, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, [&](uint32_t i) -> float { return qrow[i]; },
+              [](uint32_t i) -> uint32_t { return i; });
+}
+
+// How a long list names its candidates.
+enum ListOrder : int {
+    kByWeight = 0, // keys in order: (~weight bits, column)
+    kByRank = 1,   // keys through an index list: (weight bits, column)
+    kByColumn = 2  // keys in order: (column, weight bits)
+};
+
+// Total and walk of a list of more than one warp's worth of candidates. Whole CTA.
+__device__ __noinline__ void draw_list(Smem& s, RowChain& cs, const unsigned long long* keys, const uint16_t* ord, ListOrder order,
+                                       uint32_t n, uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
+                                       const RowOut o)
+{
+    const auto q_of = [&](uint32_t i) -> float {
+        if (order == kByWeight)
+            return __uint_as_float(~(uint32_t)(keys[i] >> 32));
+        if (order == kByRank)
+            return __uint_as_float((uint32_t)(keys[ord[i]] >> 32));
+        return __uint_as_float((uint32_t)(keys[i] & 0xffffffffull));
+    };
+    const auto col_of = [&](uint32_t i) -> uint32_t {
+        if (order == kByWeight)
+            return (uint32_t)(keys[i] & 0xffffffffull);
+        if (order == kByRank)
+            return (uint32_t)(keys[ord[i]] & 0xffffffffull);
+        return (uint32_t)(keys[i] >> 32);
+    };
+    uint32_t draft_idx = 0xffffffffu;
+    if (o.mode == kModeVerify && draft_row >= 0) {
+        if (threadIdx.x == 0)
+            cs.hit = 0xffffffffu;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += kThreads)
+            if ((int32_t)col_of(i) + o.id_offset == draft_row)
+                cs.hit = i;
+        __syncthreads();
+        draft_idx = cs.hit;
+        __syncthreads();
     }
+    if (threadIdx.x == 0)
+        s.n_final = n;
+    draw_long<kThreads>(cs, n, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, q_of, col_of);
 }
 
 // sampler.cpp:44-61 for a list longer than one warp walks: the shortest prefix of the sorted list whose double sum
@@ -1762,7 +1593,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             bool done = n <= 32u;
             if (!kRowTotal && n > 32u && n <= kWideCand) {
                 const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                                  a.cand_cap, id_off, a.timing, mode};
+                                  a.cand_cap, id_off, a.timing, mode, nullptr};
                 wide_finish(s, fkeys, n, cfg.top_k, cfg.use_topp, cfg.top_p, cfg.inv_t, m, flags, draft_row, u_row, u2_row, row, o);
                 done = true;
             }
@@ -1840,10 +1671,15 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     }
                     if ((row_total && run < want) ||
                         (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))) {
-                        if (cfg.optimistic)
+                        if (cfg.optimistic) {
                             retry = true; // what was kept does not settle the nucleus: the second pass will
-                        else
+                            if (lane == 0) {
+                                again[1] = __float_as_uint(m);
+                                *reinterpret_cast<double*>(again + 2) = total_d;
+                            }
+                        } else {
                             fl |= MK_FLAG_GUARD_BAND;
+                        }
                     }
                     n = max(k, 1u);
                 }
@@ -2071,6 +1907,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 total_approx += s.warp_sum[i];
             total_need = sum + total_approx;
             band_need = 1e-5 * total_approx + 0x1p-40 * total_need;
+            if (cfg.optimistic && tid == 0) { // for the second pass, should the row ask for it
+                again[1] = __float_as_uint(m);
+                *reinterpret_cast<double*>(again + 2) = total_need;
+            }
         }
     }
     __syncthreads();
@@ -2082,8 +1922,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     }
     if (!overflow && n > (uint32_t)kSortCap && !cfg.use_topp && !(cfg.top_k > 0 && cfg.top_k < n)) {
         const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                          a.cand_cap, id_off, a.timing, mode};
-        wide_id_ordered(s, reinterpret_cast<float*>(dyn + kOffKeys), scratch, qrow, n_raw, n, V,
+                          a.cand_cap, id_off, a.timing, mode, nullptr};
+        wide_id_ordered(s, *reinterpret_cast<RowChain*>(dyn + kOffChain), scratch, qrow, n_raw, n, V,
                         fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key)), m, cfg.inv_t, cfg.minp_eff, row,
                         flags, u_row, u2_row, draft_row, o);
         return;
@@ -2102,7 +1942,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         pre_sorted = true;
         // The float total and the walk below are sequential chains that take 32 candidates per step: fed from global
         // memory they run at the pace of its latency, so a list that fits is staged in shared memory first.
-        if (n <= kDynBytes / 8u) {
+        if (n <= kOffChain / 8u) {
             unsigned long long* const staged = reinterpret_cast<unsigned long long*>(dyn);
             for (uint32_t i = tid; i < n; i += kThreads)
                 staged[i] = P[i];
@@ -2227,8 +2067,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 
     if (a.timing && tid == 0)
         a.timing[(size_t)row * 64 + 13] = global_ns();
-    // Float total and the walk, left to right in the reference's order and precision (sampler.cpp:64-73, 80-83,
-    // 100-106), by one warp: every lane loads one candidate, the values go round by shuffle and every lane runs
+    if (!short_list) {
+        const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
+                          a.cand_cap, id_off, a.timing, mode, retry ? again : nullptr};
+        draw_list(s, *reinterpret_cast<RowChain*>(dyn + kOffChain), ksrc, ord, sorted ? kByWeight : (by_rank ? kByRank : kByColumn),
+                  n, row, flags, u_row, u2_row, draft_row, o);
+    } else
+    // A short list: float total and the walk, left to right in the reference's order and precision (sampler.cpp:64-73,
+    // 80-83, 100-106), by one warp: every lane loads one candidate, the values go round by shuffle and every lane runs
     // the same sequential chain, so the chain never waits for memory.
     if (warp == 0) {
         const uint32_t full = 0xffffffffu;
@@ -2479,7 +2325,13 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     const bool host_need_sum = !(p.temperature <= 0.0f) && p.top_p < 1.0f && !(minp_eff > 0.0f) &&
                                !(p.top_k > 0 && p.top_k < a.n_vocab);
     if (a.mode != kModeVpLocal && kNucleusGuess < a.n_vocab && (a.params_dev || host_need_sum)) {
-        RowKernelArgs second = a;
+        const int take = flat_rows_take(a);
+        if (take) {
+            e = launch_flat_rows(a, batch, stream);
+            if (e != cudaSuccess || take == 2)
+                return e;
+        }
+        RowKernelArgs second = a; // what is left
         second.pass = 1;
         e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, second)
                  : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false>, second);

@@ -70,11 +70,16 @@ struct RowKernelArgs {
 };
 
 // Words of handle scratch per row: 4 per column of capacity, then 4 of per-row state (word 0: the row asks for the
-// second pass).
+// second pass; with it word 1 its maximum, words 2-3 its total weight as a double).
 __host__ __device__ inline size_t row_scratch_words(uint32_t cap) { return 4ull * cap + 4ull; }
 
 size_t row_kernel_smem_bytes();
 cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream_t stream);
+
+// The rows of `a` that the first launch marked (top_p alone, nucleus not settled), one CTA of 1024 threads each.
+// flat_rows_take says which rows that can be: 2 all, 1 those whose history is short enough (the others stay marked), 0 none.
+int flat_rows_take(const RowKernelArgs& a);
+cudaError_t launch_flat_rows(const RowKernelArgs& a, uint32_t batch, cudaStream_t stream);
 
 struct VpMergeArgs {
     const unsigned char* gathered; // [n_shards][batch] records

@@ -1,0 +1,62 @@
+"""Rows of top_p alone whose nucleus runs to many tokens (flat_rows.cu): sizes at the edges of its groups, tables and
+lists, rows on every alignment, weights that crowd one bucket, cuts from a sample that has nothing to say. Token ids,
+candidate lists and weights against the reference, bit for bit, except in rows that report a guard band."""
+import numpy as np
+import pytest
+
+from helpers import Inputs, oracle_sample_rows
+from mako_b200.sampler import SamplingParams
+
+pytestmark = pytest.mark.gpu
+
+P = dict(repetition_penalty=1.1, presence_penalty=0.5, frequency_penalty=0.3)
+CASES = {  # vocabulary, batch, parameters, inputs, what is done to the logits
+    "ragged_small": (4099, 5, dict(temperature=1.0, top_p=0.9), dict(n_spikes=0), None),
+    "smallest": (33, 3, dict(temperature=1.0, top_p=0.97), dict(n_spikes=0, sigma=0.3), None),
+    "everything_edited": (20001, 6, dict(temperature=1.0, top_p=0.9, **P), dict(n_history=4000, n_bias=96, with_mask=True,
+                                                                             mask_fraction=0.5, n_spikes=2), None),
+    "aligned_history": (129280, 3, dict(temperature=0.8, top_p=0.95, **P), dict(n_history=4096, n_spikes=2), None),
+    "history_too_long_for_the_tables": (32000, 4, dict(temperature=1.0, top_p=0.9, **P), dict(n_history=4096, n_bias=8, n_spikes=0), None),
+    "longer_than_shared_memory": (151552, 3, dict(temperature=1.5, top_p=0.97), dict(n_spikes=0), None),
+    "ties_of_sixteenths": (65536, 3, dict(temperature=1.0, top_p=0.9), dict(n_spikes=0), lambda x: np.round(x * 16) / 16),
+    "ties_of_halves": (50257, 3, dict(temperature=1.0, top_p=0.9), dict(n_spikes=2), lambda x: np.round(x * 2) / 2),
+    "all_equal": (10000, 2, dict(temperature=1.0, top_p=0.50005), dict(n_spikes=0), lambda x: np.zeros_like(x)),
+    "low_top_p": (100003, 4, dict(temperature=1.5, top_p=0.3), dict(n_spikes=8), None),
+    "sample_misses_the_heavy": (131072, 2, dict(temperature=1.0, top_p=0.5), dict(n_spikes=0),
+                                lambda x: np.where((np.arange(x.shape[1]) % 512 >= 128) & (np.arange(x.shape[1]) % 1700 < 3), 7.0, x * 0.1)),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_flat_rows_equal_the_reference(gpu_sampler_factory, ref, name):
+    import torch
+    v, batch, p, kw, change = CASES[name]
+    p, cap = SamplingParams(**p), 256
+    inp = Inputs(7000 + len(name), batch, v, **kw)
+    if change is not None:
+        inp.logits = np.ascontiguousarray(change(inp.logits).astype(np.float32))
+    s = gpu_sampler_factory(v, 8, cap)
+    g = inp.to_gpu()
+    res = s.sample(g["logits"], p, g["u"], **g["kw"])
+    torch.cuda.synchronize()
+    tok, n, flags = res.token.cpu().numpy(), res.n_cand.cpu().numpy(), res.flags.cpu().numpy()
+    ids, qs = res.cand_ids.cpu().numpy(), res.cand_q.cpu().numpy()
+    sure = 0
+    for b, w in enumerate(oracle_sample_rows(ref, p, inp, cap=cap)):
+        assert not flags[b] & 0x50
+        if flags[b] & 0x2:
+            continue
+        sure += 1
+        k = min(w["n_cand"], cap)
+        assert (tok[b], n[b]) == (w["token"], w["n_cand"]), f"row {b}"
+        assert np.array_equal(ids[b, :k], w["cand_ids"][:k])
+        assert np.array_equal(qs[b, :k].view(np.uint32), w["cand_q"][:k].view(np.uint32))
+    assert sure
+    # the same rows as verification rows: drafts in the list and outside it
+    draft = np.where(np.arange(batch) % 2 == 0, ids[:, 0], (tok + 1) % v).astype(np.int32)
+    ver = s.verify(g["logits"], p, torch.from_numpy(draft).cuda(), g["u2"], g["u3"], **g["kw"])
+    torch.cuda.synchronize()
+    for b in range(batch):
+        if not ver.flags[b].item() & 0x2:
+            want = ref.verify(p, inp.logits[b], int(draft[b]), inp.u2[b], inp.u3[b], **inp.row_kwargs(b))
+            assert (ver.token[b].item(), bool(ver.accepted[b].item())) == (want[0], bool(want[1])), f"row {b}"
