@@ -23,7 +23,9 @@ __device__ __constant__ unsigned long long kExp2Tab[32] = {
 #include "exp2_table.inc"
 };
 
-__device__ __forceinline__ float expf_host_exact(float x)
+// `table`: kExp2Tab, or a copy of it in shared memory — lanes that want different entries of constant memory are served one
+// after the other.
+__device__ __forceinline__ float expf_host_exact(float x, const unsigned long long* table = kExp2Tab)
 {
     if (!(x >= -0x1.9fe368p6f)) {       // below log(2^-150), -inf, or NaN
         return (x != x) ? x : 0.0f;
@@ -41,7 +43,7 @@ __device__ __forceinline__ float expf_host_exact(float x)
     const unsigned long long ki = (unsigned long long)__double_as_longlong(kd);
     kd = __dsub_rn(kd, shift);
     const double r = __fma_rn(inv_ln2_n, xd, -kd);
-    const unsigned long long t = kExp2Tab[ki & 31ull] + (ki << 47);
+    const unsigned long long t = table[ki & 31ull] + (ki << 47);
     const double s = __longlong_as_double((long long)t);
     const double zz = __fma_rn(c0, r, c1);
     const double r2 = __dmul_rn(r, r);

@@ -4,12 +4,12 @@
 //
 // One CTA of 1024 threads takes a marked row; the others return. What the first launch leaves is the row's maximum and its
 // total weight (exact for what it kept, approximate for the rest), so the cut is known before the row is read again:
-//   sample    a quarter of the columns counted by weight class (sixteenths of an octave) says below which weight the elements
+//   sample    an eighth of the columns counted by weight class (sixteenths of an octave) says below which weight the elements
 //             sum up to a little less than the mass top_p leaves out;
 //   collect   one pass over the row keeps everything above that weight — the nucleus and a few per cent more — and sums
 //             the approximate weights of the rest;
-//   order     exact weights; the list is dealt into buckets of about eight, of equal counts rather than equal widths, each sorted
-//             by one thread (a warp or the CTA where equal weights crowd a bucket);
+//   order     exact weights; the list is dealt into buckets of about eight, of equal counts rather than equal widths, each whose
+//             members rank themselves, a lane each (a warp or the CTA sorts where equal weights crowd a bucket);
 //   draw      double prefix sums for top_p, then the float total and the walk as scans (list_chain.cuh).
 // A cut that proves too tight (a list that ends before the nucleus does) is replaced by the bound that cannot be, and the row
 // is read once more. The generated and biased columns are edited apart: a bitmap takes them out of the row's stream, and their
@@ -30,8 +30,7 @@ constexpr uint32_t kSpecialCap = 4096;      // generated and biased columns of a
 constexpr uint32_t kFlatVocab = 163840;
 constexpr uint32_t kFlatBmWords = kFlatVocab / 32 + 2;
 constexpr uint32_t kMaxBuckets = 8192;
-constexpr uint32_t kThreadSort = 24;        // a bucket up to this size is sorted by one thread
-constexpr uint32_t kWarpSort = 4096;        // ... by one warp
+constexpr uint32_t kWarpSort = 4096;        // a bucket of more than 32 and up to this size is sorted by one warp
 constexpr uint32_t kBigBuckets = 1024;
 
 // Shared memory: the tables of the edits while the row is read, the list and its buckets afterwards.
@@ -46,11 +45,11 @@ constexpr uint32_t kOffBuckets = kOffKeysEnd;                  // kMaxBuckets en
 constexpr uint32_t kOffClass = kOffBuckets + kMaxBuckets * 4u; // kClasses (first bucket, buckets); sampling: the counts
 constexpr uint32_t kOffBig = kOffClass + kClasses * 8u;        // buckets too large for one thread
 constexpr uint32_t kFlatDyn = kOffBig + kBigBuckets * 4u;
-constexpr uint32_t kDenseCap = (kFlatDyn - kOffBuckets) / 4u;  // weights in order that fit behind the list
 static_assert(kOffVal + kSpecialCap * 4u <= kOffBuckets, "the edits' tables lie below the classes");
 
 struct FlatSmem {
     ChainSmem<kFlatThreads> chain;
+    unsigned long long exp2_table[32];
     double sum[2][kFlatWarps];
     uint32_t wsum[kFlatWarps];
     uint32_t rows[16], n_rows;
@@ -160,6 +159,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
     uint32_t* const big = reinterpret_cast<uint32_t*>(dyn + kOffBig);
     const uint32_t V = a.n_vocab;
 
+    if (tid < 32u)
+        s.exp2_table[tid] = kExp2Tab[tid];
     uint32_t seen = 0; // marked rows of earlier chunks
     for (uint32_t chunk = 0; chunk < batch; chunk += (uint32_t)kFlatThreads) {
         // which marked rows of this chunk are this CTA's
@@ -210,23 +211,25 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             if (hlen + nb > kSpecialCap)
                 continue; // stays marked: the row pipeline's own second launch takes it
             const bool special = hlen > 0u || nb > 0u;
-            // four places of the row; those that are not the row's own, not allowed, or edited apart read as -inf
-            auto load4 = [&](uint32_t g, float (&w)[4]) {
+            // Four places of the row: fetched (nothing is, for a group that reaches past the row's ends), and edited; those that
+            // are not the row's own, not allowed, or edited apart read as -inf.
+            auto fetch4 = [&](uint32_t g) -> float4 {
                 const uint32_t p = 4u * g;
+                return (p >= shift && p + 4u <= V + shift) ? __ldg(l4 + g) : make_float4(ninf, ninf, ninf, ninf);
+            };
+            auto edit4 = [&](uint32_t g, const float4& v, float (&w)[4]) {
+                const uint32_t p = 4u * g;
+                w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+                if (g >= n4)
+                    return;
                 uint32_t off = special ? (bitmap[p >> 5] >> (p & 31u)) & 15u : 0u;
-                if (p < shift)
-                    off |= (1u << shift) - 1u;
-                if (p + 4u > V + shift)
-                    off |= 15u & ~((1u << (V + shift - p)) - 1u);
                 if (mrow)
                     off |= ~(shift == 0u ? __ldg(mrow + (p >> 5)) >> (p & 31u) : mask_nibble(mrow, (int32_t)p - (int32_t)shift, V));
-                if (p >= shift && p + 4u <= V + shift) {
-                    const float4 v = __ldg(l4 + g);
-                    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
-                } else {
+                if (p < shift || p + 4u > V + shift) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        w[j] = ((off >> j) & 1u) ? ninf : __ldg(lrow + (p + (uint32_t)j - shift));
+                    for (uint32_t j = 0; j < 4u; ++j)
+                        if (p + j >= shift && p + j < V + shift)
+                            w[j] = __ldg(lrow + (p + j - shift));
                 }
                 if (off & 15u) {
 #pragma unroll
@@ -235,6 +238,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                             w[j] = ninf;
                 }
             };
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 14] = global_ns();
             // ---- the edited columns --------------------------------------------------------------------------------
             uint32_t n_special = 0;
             if (special) {
@@ -243,19 +248,25 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     bitmap[i] = 0u;
                 for (uint32_t i = tid; i < kSpecialCap; i += kFlatThreads)
                     count[i] = 0u;
-                __syncthreads();
-                // place of a token id, or none: unsigned, an id below the row's first column wraps past V
-                auto place = [&](int32_t id) -> uint32_t {
-                    const uint32_t c = (uint32_t)id - (uint32_t)a.id_offset;
-                    return c < V ? c + shift : 0xffffffffu;
-                };
-                for (uint32_t j = tid; j < hlen + nb; j += kFlatThreads) {
-                    const bool h = j < hlen;
-                    const int32_t id = h ? __ldg(hrow + j) : brow[j - hlen].id;
-                    const uint32_t p = (h || id >= 0) ? place(id) : 0xffffffffu;
-                    if (p != 0xffffffffu)
-                        atomicOr(&bitmap[p >> 5], 1u << (p & 31u));
+                constexpr uint32_t kMine = kSpecialCap / kFlatThreads;
+                uint32_t place[kMine]; // of this thread's entries, or none
+#pragma unroll
+                for (uint32_t i = 0; i < kMine; ++i) {
+                    const uint32_t j = tid + i * kFlatThreads;
+                    place[i] = 0xffffffffu;
+                    if (j < hlen + nb) {
+                        const bool h = j < hlen;
+                        const int32_t id = h ? __ldg(hrow + j) : brow[j - hlen].id;
+                        const uint32_t c = (uint32_t)id - (uint32_t)a.id_offset; // an id below the first column wraps past V
+                        if ((h || id >= 0) && c < V)
+                            place[i] = c + shift;
+                    }
                 }
+                __syncthreads();
+#pragma unroll
+                for (uint32_t i = 0; i < kMine; ++i)
+                    if (place[i] != 0xffffffffu)
+                        atomicOr(&bitmap[place[i] >> 5], 1u << (place[i] & 31u));
                 __syncthreads();
                 constexpr uint32_t kPer = (kFlatBmWords + kFlatThreads - 1u) / kFlatThreads;
                 uint32_t pc[kPer], mine = 0;
@@ -274,15 +285,14 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     before += pc[i];
                 }
                 __syncthreads();
-                for (uint32_t j = tid; j < hlen + nb; j += kFlatThreads) {
-                    const bool h = j < hlen;
-                    const int32_t id = h ? __ldg(hrow + j) : brow[j - hlen].id;
-                    const uint32_t p = (h || id >= 0) ? place(id) : 0xffffffffu;
+#pragma unroll
+                for (uint32_t i = 0; i < kMine; ++i) {
+                    const uint32_t j = tid + i * kFlatThreads, p = place[i];
                     if (p == 0xffffffffu)
                         continue;
                     const uint32_t r = ranks[p >> 5] + __popc(bitmap[p >> 5] & ((1u << (p & 31u)) - 1u));
                     scol[r] = p - shift;
-                    if (h) {
+                    if (j < hlen) {
                         atomicAdd(&count[r], 1u);
                     } else {
                         sval[r] = brow[j - hlen].value;
@@ -302,27 +312,32 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     sval[r] = l;
                 }
             }
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 15] = global_ns();
             // ---- the cut ---------------------------------------------------------------------------------------------
             // Elements counted by weight class; a class's heaviest weight stands for all of its elements, so the mass below a
-            // class is never taken for less than the sample says. A quarter of the row is counted, in runs of 128 columns.
+            // class is never taken for less than the sample says. An eighth of a long row is counted, in runs of 128 columns.
             for (uint32_t i = tid; i < kClasses; i += kFlatThreads)
                 cls[i] = 0u;
             __syncthreads();
-            const uint32_t every = n4 >= 8192u ? 4u : 1u;
+            const uint32_t every = n4 >= 24576u ? 8u : n4 >= 8192u ? 4u : 1u;
             auto enter = [&](float w, uint32_t n) {
                 const float x = (m - w) * (c2 * 16.0f);
                 if (x < (float)kClasses) // false for NaN and for what is not there
                     atomicAdd(&cls[min((uint32_t)fmaxf(x, 0.0f), kClasses - 1u)], n);
             };
-            for (uint32_t b = warp; b * 32u * every < n4; b += kFlatWarps) {
-                const uint32_t g = b * 32u * every + ((b * 5u) % every) * 32u + lane;
-                float w[4];
-                if (g < n4) {
-                    load4(g, w);
+            for (uint32_t b0 = warp * 4u; b0 * 32u * every < n4; b0 += kFlatWarps * 4u) { // four loads in flight
+                float w[4][4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k) {
+                    const uint32_t b = b0 + k, g = b * 32u * every + (b % every) * 32u + lane;
+                    edit4(g, fetch4(g), w[k]);
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < 4u; ++k)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        enter(w[j], every);
-                }
+                        enter(w[k][j], every);
             }
             for (uint32_t r = tid; r < n_special; r += kFlatThreads)
                 enter(sval[r], 1u);
@@ -368,6 +383,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             }
             __syncthreads();
             float thr = s.cut;
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 16] = global_ns();
             // ---- collect, order, cut at top_p; once more with the loose bound if the list ends too early ---------------
             unsigned long long* keys = nullptr;
             uint32_t n = 0, n_take = 0;
@@ -379,27 +396,26 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 __syncthreads();
                 double tail = 0.0;
                 for (uint32_t g0 = warp * 128u; g0 < n4; g0 += kFlatThreads * 4u) {
+                    float4 v[4];
                     float w[4][4];
-                    uint32_t mine = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        v[k] = fetch4(g0 + k * 32u + lane);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        edit4(g0 + k * 32u + lane, v[k], w[k]);
+                    uint32_t keep = 0u; // one bit an element; nothing below branches on an element's own value
                     float part = 0.0f;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint32_t g = g0 + (uint32_t)k * 32u + lane;
-                        if (g < n4)
-                            load4(g, w[k]);
-                        else
-                            w[k][0] = w[k][1] = w[k][2] = w[k][3] = ninf;
-                    }
+                    for (uint32_t k = 0; k < 4u; ++k)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            if (w[k][j] >= thr)
-                                ++mine;
-                            else if (w[k][j] < thr) // not a NaN
-                                part += ex2_approx((w[k][j] - m) * c2);
+                        for (uint32_t j = 0; j < 4u; ++j) {
+                            keep |= w[k][j] >= thr ? 1u << (4u * k + j) : 0u;
+                            const float e = ex2_approx((w[k][j] - m) * c2); // (not w * c2 - m * c2: that rounds m * c2)
+                            part += w[k][j] < thr ? e : 0.0f; // a NaN is neither
                         }
                     tail += (double)part;
+                    const uint32_t mine = (uint32_t)__popc(keep);
                     if (__any_sync(full, mine != 0u)) {
                         uint32_t inc = mine;
 #pragma unroll
@@ -411,17 +427,14 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                         uint32_t slot = 0;
                         if (lane == 31u)
                             slot = atomicAdd(&s.n_list, inc);
-                        slot = __shfl_sync(full, slot, 31) + inc - mine;
-                        if (mine) {
+                        uint2* at_list = list + (__shfl_sync(full, slot, 31) + inc - mine);
+                        const uint32_t col = 4u * (g0 + lane) - shift;
 #pragma unroll
-                            for (int k = 0; k < 4; ++k)
+                        for (uint32_t k = 0; k < 4u; ++k)
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    if (w[k][j] >= thr) {
-                                        const uint32_t p = 4u * (g0 + (uint32_t)k * 32u + lane) + (uint32_t)j;
-                                        list[slot++] = make_uint2(__float_as_uint(w[k][j]), p - shift);
-                                    }
-                        }
+                            for (uint32_t j = 0; j < 4u; ++j)
+                                if ((keep >> (4u * k + j)) & 1u)
+                                    *at_list++ = make_uint2(__float_as_uint(w[k][j]), col + 128u * k + j);
                     }
                 }
                 for (uint32_t r = tid; r < n_special; r += kFlatThreads) {
@@ -433,24 +446,36 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 }
                 const double rest = block_sum(s, tail, 0);
                 n = s.n_list;
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 17] = global_ns();
                 // exact weights, in place of the logits; their sum; how many there are in each class of the float's own octaves
                 for (uint32_t i = tid; i < kClasses; i += kFlatThreads)
                     cls2[i] = make_uint2(0u, 0u);
                 __syncthreads();
                 double exact = 0.0;
-                for (uint32_t i = tid; i < n; i += kFlatThreads) {
-                    const uint2 c = list[i];
-                    const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t));
-                    const bool in = q >= cfg.minp_eff && q > 0.0f;
-                    exact += (double)q;
-                    const uint32_t d = in ? 0x3f800000u - __float_as_uint(q) : 0xffffffffu; // 0 for the maximum
-                    list[i].x = d;
-                    if (in)
-                        atomicAdd(&cls2[min(d >> 19, kClasses - 1u)].y, 1u);
+                for (uint32_t i0 = tid; i0 < n; i0 += 4u * kFlatThreads) {
+                    uint32_t x[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        x[k] = i0 + k * kFlatThreads < n ? list[i0 + k * kFlatThreads].x : 0u;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k) {
+                        if (i0 + k * kFlatThreads >= n)
+                            break;
+                        const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(x[k]), m), cfg.inv_t), s.exp2_table);
+                        const bool in = q >= cfg.minp_eff && q > 0.0f;
+                        exact += (double)q;
+                        const uint32_t d = in ? 0x3f800000u - __float_as_uint(q) : 0xffffffffu; // 0 for the maximum
+                        list[i0 + k * kFlatThreads].x = d;
+                        if (in)
+                            atomicAdd(&cls2[min(d >> 19, kClasses - 1u)].y, 1u);
+                    }
                 }
                 const double sum = block_sum(s, exact, 1);
                 const double total = sum + rest;
                 const double band = 1e-5 * rest + 0x1p-36 * total, want = (double)cfg.top_p * total;
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 18] = global_ns();
                 // buckets: each class gets as many as its count asks for
                 uint32_t in_class = tid < kClasses ? cls2[tid].y : 0u, n_in, n_buckets;
                 block_exclusive(s, in_class, n_in);
@@ -469,10 +494,15 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                         return b.x;
                     return b.x + (uint32_t)(((unsigned long long)(d & 0x7ffffu) * b.y) >> 19);
                 };
-                for (uint32_t i = tid; i < n; i += kFlatThreads) {
-                    const uint32_t d = list[i].x;
-                    if (d != 0xffffffffu)
-                        atomicAdd(&ends[bucket(d)], 1u);
+                for (uint32_t i0 = tid; i0 < n; i0 += 4u * kFlatThreads) {
+                    uint32_t d[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        d[k] = i0 + k * kFlatThreads < n ? list[i0 + k * kFlatThreads].x : 0xffffffffu;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        if (d[k] != 0xffffffffu)
+                            atomicAdd(&ends[bucket(d[k])], 1u);
                 }
                 __syncthreads();
                 {
@@ -505,27 +535,59 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                         keep[r] = make_uint2(__float_as_uint(sval[r]), scol[r]);
                     __syncthreads();
                 }
-                for (uint32_t i = tid; i < n; i += kFlatThreads) {
-                    const uint2 c = list[i];
-                    if (c.x != 0xffffffffu)
-                        keys[atomicAdd(&ends[bucket(c.x)], 1u)] =
-                            ((unsigned long long)(c.x + ~0x3f800000u) << 32) | c.y; // pack_by_weight's key
+                for (uint32_t i0 = tid; i0 < n; i0 += 4u * kFlatThreads) {
+                    uint2 c[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        c[k] = i0 + k * kFlatThreads < n ? list[i0 + k * kFlatThreads] : make_uint2(0xffffffffu, 0u);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        if (c[k].x != 0xffffffffu)
+                            keys[atomicAdd(&ends[bucket(c[k].x)], 1u)] =
+                                ((unsigned long long)(c[k].x + ~0x3f800000u) << 32) | c[k].y; // pack_by_weight's key
                 }
                 __syncthreads();
-                for (uint32_t b = tid; b < n_buckets; b += kFlatThreads) {
-                    const uint32_t i0 = b ? ends[b - 1u] : 0u, i1 = ends[b];
-                    if (i1 - i0 > kThreadSort) {
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 19] = global_ns();
+                for (uint32_t b = tid; b < n_buckets; b += kFlatThreads)
+                    if (ends[b] - (b ? ends[b - 1u] : 0u) > 32u) {
                         const uint32_t at_big = atomicAdd(&s.n_big, 1u);
                         if (at_big < kBigBuckets)
                             big[at_big] = b;
-                    } else {
-                        for (uint32_t i = i0 + 1u; i < i1; ++i) {
-                            const unsigned long long key = keys[i];
-                            uint32_t j = i;
-                            for (; j > i0 && keys[j - 1u] > key; --j)
-                                keys[j] = keys[j - 1u];
-                            keys[j] = key;
+                    }
+                // Every warp takes the buckets that start in its share of the list, as many as 32 lanes hold at a time: a
+                // lane counts the smaller keys of its bucket and puts its own there.
+                {
+                    const uint32_t share = (n_in + kFlatWarps - 1u) / kFlatWarps, p_end = min((warp + 1u) * share, n_in);
+                    uint32_t p = min(warp * share, n_in);
+                    bool whole = p == 0u; // whether p is the start of a bucket
+                    while (p < p_end) {
+                        const uint32_t i = p + lane;
+                        unsigned long long key = 0ull;
+                        uint32_t i0 = 0u, i1 = 0u;
+                        if (i < n_in) {
+                            key = keys[i];
+                            const uint32_t b = bucket((uint32_t)(key >> 32) - ~0x3f800000u);
+                            i0 = b ? ends[b - 1u] : 0u;
+                            i1 = ends[b];
                         }
+                        const uint32_t b0 = __shfl_sync(full, i0, 0), b1 = __shfl_sync(full, i1, 0);
+                        if ((!whole && b0 != p) || b1 - b0 > 32u) { // another warp's, or a large one
+                            p = b1;
+                            whole = true;
+                            continue;
+                        }
+                        const bool mine = i < n_in && i1 <= p + 32u && i0 < p_end;
+                        uint32_t below = 0u;
+                        if (mine)
+                            for (uint32_t j = i0; j < i1; ++j)
+                                below += keys[j] < key ? 1u : 0u;
+                        __syncwarp();
+                        if (mine)
+                            keys[i0 + below] = key;
+                        __syncwarp();
+                        p = __reduce_max_sync(full, mine ? i1 : 0u);
+                        whole = true;
                     }
                 }
                 __syncthreads();
@@ -545,6 +607,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     }
                     __syncthreads();
                 }
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 20] = global_ns();
                 // ---- top_p (sampler.cpp:44-61): the shortest prefix whose double sum is not below `want` --------------------
                 auto q_key = [&](uint32_t i) -> float { return __uint_as_float(~(uint32_t)(keys[i] >> 32)); };
                 const uint32_t run_len = ((n_in + kFlatThreads - 1u) / kFlatThreads) | 1u;
@@ -617,6 +681,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 thr = loose;
                 __syncthreads();
             }
+            if (a.timing && tid == 0)
+                a.timing[(size_t)row * 64 + 21] = global_ns();
             // ---- the draw --------------------------------------------------------------------------------------------
             uint32_t draft_idx = 0xffffffffu;
             if (a.mode == kModeVerify && draft_row >= 0) {
@@ -629,9 +695,15 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 __syncthreads();
                 draft_idx = s.n_big;
             }
+            if (a.timing && tid == 0) {
+                a.timing[(size_t)row * 64 + 9] = n;
+                a.timing[(size_t)row * 64 + 10] = n_take;
+            }
             // the weights alone, in order, for the chains
-            float* const q = n_take <= kDenseCap ? reinterpret_cast<float*>(dyn + kOffBuckets)
-                                                 : reinterpret_cast<float*>(row_scratch); // the raw list is dead
+            const bool on_chip = reinterpret_cast<unsigned char*>(keys) == dyn;
+            const uint32_t q_off = on_chip ? (n * 8u + 15u) & ~15u : 0u;
+            float* const q = q_off + n_take * 4u <= kFlatDyn ? reinterpret_cast<float*>(dyn + q_off)
+                                                             : reinterpret_cast<float*>(row_scratch); // the raw list is dead
             for (uint32_t i = tid; i < n_take; i += kFlatThreads)
                 q[i] = __uint_as_float(~(uint32_t)(keys[i] >> 32));
             const uint32_t n_out = min(n_take, a.cand_cap);
@@ -641,9 +713,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             }
             __syncthreads();
             const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                              a.cand_cap, a.id_offset, a.timing, a.mode, nullptr};
-            draw_long<kFlatThreads>(s.chain, n_take, n_take, draft_idx, row, flags, u_row, u2_row, draft_row, o,
-                                    [&](uint32_t i) -> float { return q[i]; },
+                              a.cand_cap, a.id_offset, a.timing, a.mode};
+            draw_long<kFlatThreads>(s.chain, q, n_take, n_take, draft_idx, row, flags, u_row, u2_row, draft_row, o,
                                     [&](uint32_t i) -> uint32_t { return (uint32_t)(keys[i] & 0xffffffffull); });
             if (tid == 0)
                 state[0] = 0u;

@@ -11,7 +11,9 @@
 
 namespace mk {
 
-constexpr uint32_t kNucleusGuess = 24;  // top_p alone, first launch: the largest elements kept (the one-warp finish takes 32 candidates)
+// top_p alone, first launch: the largest elements kept. The bound that keeps them is the edge of a histogram bin and lets
+// about 1.4 times as many through; the one-warp finish takes 32.
+constexpr uint32_t kNucleusGuess = 20;
 
 struct RowCfg {
     float temperature, inv_t, minp_eff, top_p;
@@ -133,22 +135,21 @@ struct RowOut {
     int32_t id_offset;
     unsigned long long* timing;
     int mode;
-    uint32_t* again; // set: what was kept does not settle the row, the second pass will (the row's mark), else null
 };
 
-// What the draw leaves behind once its chains are known (sampler.cpp:64-73, 80-83, 100-106), for a list of n candidates
-// that the whole CTA walks: q_of(i), col_of(i) in draw order. Zero weights (gaps of a list laid out by column) never
-// win. Returns through o; n_out is the number of candidates. Whole CTA.
-template <int kThreads, class Q, class Col>
-__device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, uint32_t n, uint32_t n_out, uint32_t draft_idx, uint32_t row, uint32_t flags,
-                                          float u_row, float u2_row, int32_t draft_row, const RowOut& o, Q&& q_of, Col&& col_of)
+// What the draw leaves behind once its chains are known (sampler.cpp:64-73, 80-83, 100-106), for a list of n weights q in draw
+// order (16-byte aligned; zeros, the gaps of a list laid out by column, never win; a rejected draft's weight is zeroed).
+// col_of(i) names a weight's column; n_out is the number of candidates. Whole CTA; the caller synchronises before.
+template <int kThreads, class Col>
+__device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, float* q, uint32_t n, uint32_t n_out, uint32_t draft_idx,
+                                          uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
+                                          const RowOut& o, Col&& col_of)
 {
     const uint32_t none = 0xffffffffu;
-    const float total = chain_total<kThreads>(cs, n, q_of);
-    const float q_draft = (draft_idx != none) ? q_of(draft_idx) : 0.0f;
+    const float total = chain<kThreads, false>(cs, q, n, 0.0f);
+    const float q_draft = (draft_idx != none) ? q[draft_idx] : 0.0f;
     int32_t tok = -1, acc = 0;
     float prob = 0.0f, walk_total = total;
-    uint32_t skip = none;
     if (o.mode == kModeDistOnly) {
         tok = -2; // nothing is drawn: the first candidate stands for the row below
     } else if (o.mode == kModeVerify) {
@@ -157,20 +158,22 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, uint32_t n, u
             tok = draft_row;
             prob = __fdiv_rn(q_draft, total);
         } else {
-            skip = draft_idx;
             walk_total = __fsub_rn(total, q_draft);
         }
     }
     uint32_t hit = none, first = none, last = none;
     float r_hit = 0.0f, q_hit = 0.0f;
-    const auto q_walk = [&](uint32_t i) -> float { return (i == skip) ? 0.0f : q_of(i); };
     if (tok == -1) {
-        const float r = __fmul_rn((o.mode == kModeVerify) ? u2_row : u_row, walk_total);
-        if (chain_walk<kThreads>(cs, n, r, q_walk)) {
-            hit = cs.hit;
-            r_hit = cs.r_hit;
-            q_hit = cs.q_hit;
+        if (draft_idx != none && o.mode == kModeVerify) {
+            __syncthreads(); // everyone has read the draft's weight
+            if (threadIdx.x == 0)
+                q[draft_idx] = 0.0f;
+            __syncthreads();
         }
+        chain<kThreads, true>(cs, q, n, __fmul_rn((o.mode == kModeVerify) ? u2_row : u_row, walk_total));
+        hit = cs.hit;
+        r_hit = cs.r_hit;
+        q_hit = cs.q_hit;
     }
     // the first and the last candidate that could win: the edges of the CDF have no neighbour beyond them
     __syncthreads();
@@ -180,12 +183,12 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, uint32_t n, u
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += kThreads)
-        if (q_walk(i) > 0.0f) {
+        if (q[i] > 0.0f) {
             atomicMin(&cs.warp0[0], i);
             break;
         }
     for (uint32_t i = threadIdx.x; i < n; i += kThreads)
-        if (q_walk(n - 1u - i) > 0.0f) {
+        if (q[n - 1u - i] > 0.0f) {
             atomicMax(&cs.warp1[0], n - 1u - i);
             break;
         }
@@ -196,7 +199,7 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, uint32_t n, u
         return;
     if (tok == -2) {
         tok = (int32_t)col_of(first) + o.id_offset;
-        prob = __fdiv_rn(q_of(first), total);
+        prob = __fdiv_rn(q[first], total);
     } else if (tok == -1 && first == none) { // nothing but the rejected draft
         tok = draft_row;
         prob = 1.0f;
@@ -207,14 +210,12 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, uint32_t n, u
                 flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
         } else { // rounding: the last candidate (sampler.cpp:72)
             hit = last;
-            q_hit = q_of(last);
+            q_hit = q[last];
         }
         tok = (int32_t)col_of(hit) + o.id_offset;
         prob = __fdiv_rn(q_hit, walk_total);
     }
-    if (o.token) o.token[row] = o.again ? -1 : tok;
-    if (o.again)
-        o.again[0] = 1u; // every output of this row is written again by the second pass
+    if (o.token) o.token[row] = tok;
     if (o.prob) o.prob[row] = prob;
     if (o.flags) o.flags[row] = flags;
     if (o.n_cand) o.n_cand[row] = n_out;

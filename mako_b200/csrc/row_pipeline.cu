@@ -350,8 +350,7 @@ __device__ __noinline__ void wide_id_ordered(Smem& s, RowChain& cs, const uint2*
     }
     const int64_t d = (int64_t)draft_row - o.id_offset;
     const uint32_t draft_idx = (o.mode == kModeVerify && draft_row >= 0 && d >= 0 && d < (int64_t)V) ? (uint32_t)d : 0xffffffffu;
-    draw_long<kThreads>(cs, V, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, [&](uint32_t i) -> float { return qrow[i]; },
-              [](uint32_t i) -> uint32_t { return i; });
+    draw_long<kThreads>(cs, qrow, V, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, [](uint32_t i) -> uint32_t { return i; });
 }
 
 // How a long list names its candidates.
@@ -361,18 +360,15 @@ enum ListOrder : int {
     kByColumn = 2  // keys in order: (column, weight bits)
 };
 
-// Total and walk of a list of more than one warp's worth of candidates. Whole CTA.
+// Total and walk of a list of more than one warp's worth of candidates. `q`: room for n weights, 16-byte aligned. Whole CTA.
 __device__ __noinline__ void draw_list(Smem& s, RowChain& cs, const unsigned long long* keys, const uint16_t* ord, ListOrder order,
-                                       uint32_t n, uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
+                                       float* q, uint32_t n, uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
                                        const RowOut o)
 {
-    const auto q_of = [&](uint32_t i) -> float {
-        if (order == kByWeight)
-            return __uint_as_float(~(uint32_t)(keys[i] >> 32));
-        if (order == kByRank)
-            return __uint_as_float((uint32_t)(keys[ord[i]] >> 32));
-        return __uint_as_float((uint32_t)(keys[i] & 0xffffffffull));
-    };
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads) { // the weights alone, in order
+        const unsigned long long key = keys[order == kByRank ? (uint32_t)ord[i] : i];
+        q[i] = __uint_as_float(order == kByWeight ? ~(uint32_t)(key >> 32) : order == kByRank ? (uint32_t)(key >> 32) : (uint32_t)key);
+    }
     const auto col_of = [&](uint32_t i) -> uint32_t {
         if (order == kByWeight)
             return (uint32_t)(keys[i] & 0xffffffffull);
@@ -394,7 +390,8 @@ __device__ __noinline__ void draw_list(Smem& s, RowChain& cs, const unsigned lon
     }
     if (threadIdx.x == 0)
         s.n_final = n;
-    draw_long<kThreads>(cs, n, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, q_of, col_of);
+    __syncthreads();
+    draw_long<kThreads>(cs, q, n, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, col_of);
 }
 
 // sampler.cpp:44-61 for a list longer than one warp walks: the shortest prefix of the sorted list whose double sum
@@ -1256,7 +1253,9 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         const float c2 = cfg.inv_t * 1.4426950408889634f;
         const float ninf = -__int_as_float(0x7f800000);
         const bool collect = !cfg.greedy || mode == kModeVpLocal;
-        const bool sum_all = mode == kModeVpLocal;
+        // A nucleus that is to be found among the few largest, or a shard record: the streamed sum takes every element.
+        const bool sum_all = mode == kModeVpLocal || cfg.optimistic;
+        const bool hist_bound_alone = !(cfg.minp_eff > 0.0f) && cfg.hist_k <= kVpMaxK + 1u;
         float warp_pub = ninf;
         // The loop over the tiles is compiled four times, with the mask, the top_k histogram and the streamed sum
         // compiled in or out: a row runs a variant that holds little beyond its own work. (One loop with all
@@ -1338,7 +1337,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         if (w[e] == tm)
                             best_col = (int32_t)(base + (e >> 2) * 1024 + rt * 4 + (e & 3));
                 }
-                if (__any_sync(0xffffffffu, tm > warp_pub)) {
+                if (!(kHist && cfg.hist_mode && hist_bound_alone) && __any_sync(0xffffffffu, tm > warp_pub)) {
                     const float wm = warp_max(tm);
                     if (wm > warp_pub) {
                         warp_pub = wm;
@@ -1346,7 +1345,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             atomicMax(&s.m_key, order_key(wm));
                     }
                 }
-                float thr = keep_threshold(cfg, key_to_float(*(volatile uint32_t*)&s.m_key));
+                // Under the histogram bound the distance from the maximum only matters where min_p or a large top_k makes
+                // it the tighter of the two.
+                float thr = (kHist && cfg.hist_mode && hist_bound_alone)
+                                ? -FLT_MAX
+                                : keep_threshold(cfg, key_to_float(*(volatile uint32_t*)&s.m_key));
                 if (kHist && cfg.hist_mode) {
                     // top_k bound. Every thread enters the largest of its 16 elements of the tile, if that is still at
                     // or above the bound in force, into a histogram of the value range: the maxima of different
@@ -1375,10 +1378,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         }
                         __syncwarp();
                     }
-                    // One reader warp per tile rescans the histogram and raises the bound; nobody waits for it. Counts
-                    // only grow and every count is an element at or above its bin's edge, so a bound read from a
+                    // One reader warp rescans the histogram and raises the bound, after every tile while the row is young and
+                    // then after every fourth (the bound of t tiles lets k / t elements of a later tile through; a scan is
+                    // a chain of a dozen dependent shared loads and shuffle rounds); nobody waits for it. Counts only grow and every count is an element at or above its bin's edge, so a bound read from a
                     // histogram that other warps are still adding to has its k elements all the same.
-                    if (t == 0 || rwarp == (t % (kReaders / 32))) {
+                    if (t == 0 || (rwarp == (t % (kReaders / 32)) && (t < 8 || (t & 3u) == 0u))) {
                         uint32_t cum = 0;
                         int found = -1;
                         for (int g = (int)*(volatile uint32_t*)&s.hi_group; g >= 0 && found < 0; --g) {
@@ -1414,15 +1418,22 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     }
                 }
                 if (kSum && cfg.need_sum && best > ninf) {
-                    // Approximate weight of what is NOT collected (`thr` is the bound the collection used; a shard record
-                    // sums everything): the collected
-                    // elements get exact weights in the finish, so only the far tail carries the approximation.
+                    // Approximate weights, relative to the thread's running maximum. Of a row that keeps the few largest (and
+                    // of a shard record) every element; else of what is NOT collected (`thr` is the bound
+                    // the collection used): the collected elements get exact weights in the finish, so only the far tail
+                    // carries the approximation. NaN weighs nothing.
                     if (best > old_best)
                         sum_acc *= (double)exp2f((old_best - best) * c2);
                     float p = 0.0f;
+                    if (kHist && sum_all) { // (the maximum with -inf is what a NaN turns into)
 #pragma unroll
-                    for (int e = 0; e < kEl; ++e)
-                        p += (sum_all || w[e] < thr) ? ex2_approx((w[e] - best) * c2) : 0.0f;
+                        for (int e = 0; e < kEl; ++e)
+                            p += ex2_approx((fmaxf(w[e], ninf) - best) * c2);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < kEl; ++e)
+                            p += w[e] < thr ? ex2_approx((w[e] - best) * c2) : 0.0f;
+                    }
                     sum_acc += (double)p;
                 }
                 if (!(kHist && cfg.hist_mode) && collect) {
@@ -1561,7 +1572,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             const float thr_final = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
             unsigned long long* const fkeys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
             uint32_t n = 0;
-            double sum_kept = 0.0, sum_rest = 0.0; // top_p alone: exact weights at or above the bound, the others
+            double sum_kept = 0.0, sum_again = 0.0; // top_p alone: exact weights at or above the bound; what the streamed sum has too much
             for (uint32_t r0 = 0; r0 < n_raw && n <= kWideCand; r0 += kFastRaw) { // once, for nearly every row
                 uint2 craw[kFastRaw / 32]; // all requested at once: one trip to memory under load, not one per chunk
 #pragma unroll
@@ -1575,11 +1586,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     float q = 0.0f;
                     if (__uint_as_float(c.x) >= thr_final) {
                         q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t));
-                        if (kRowTotal && q == q)
+                    }
+                    if (kRowTotal) {
+                        // as streamed: of a kept element to be taken out again where the sum took every element, of
+                        // one collected while the bound was lower to be added where it took none of the collected
+                        const bool in = __uint_as_float(c.x) >= thr_final;
+                        const double streamed = (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
+                        if (in && q == q)
                             sum_kept += (double)q;
-                    } else if (kRowTotal) {
-                        // collected while the bound was lower: part of the row total, never a candidate
-                        sum_rest += (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
+                        if (in == cfg.optimistic && streamed == streamed)
+                            sum_again += in ? streamed : -streamed;
                     }
                     const bool ok = q >= cfg.minp_eff && q > 0.0f; // false for NaN
                     const uint32_t bal = __ballot_sync(full, ok);
@@ -1593,7 +1609,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             bool done = n <= 32u;
             if (!kRowTotal && n > 32u && n <= kWideCand) {
                 const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                                  a.cand_cap, id_off, a.timing, mode, nullptr};
+                                  a.cand_cap, id_off, a.timing, mode};
                 wide_finish(s, fkeys, n, cfg.top_k, cfg.use_topp, cfg.top_p, cfg.inv_t, m, flags, draft_row, u_row, u2_row, row, o);
                 done = true;
             }
@@ -1644,18 +1660,19 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 }
                 if (cfg.use_topp) { // sampler.cpp:44-61, sequentially
                     double total_d = 0.0, band;
-                    // top_p alone: the total covers every column — exact weights of what was kept, the streamed sum
-                    // and the approximations above for the rest — and carries the margin of the approximate part
+                    // top_p alone: the total covers every column — exact weights of what was kept, and of the streamed
+                    // sum what lies beside them — and carries the margin of the approximate part and, where the kept
+                    // elements' shares had to be taken out of it, of the rounding of the streamed sum's terms
                     const bool row_total = kRowTotal && !(fl & MK_FLAG_NO_CANDIDATE);
                     if (row_total) {
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) {
                             sum_kept += __shfl_xor_sync(full, sum_kept, o);
-                            sum_rest += __shfl_xor_sync(full, sum_rest, o);
+                            sum_again += __shfl_xor_sync(full, sum_again, o);
                         }
-                        const double rest = total_approx + sum_rest;
+                        const double rest = fmax(total_approx - sum_again, 0.0);
                         total_d = sum_kept + rest;
-                        band = 1e-5 * rest + 0x1p-40 * total_d;
+                        band = 1e-5 * rest + (cfg.optimistic ? 2e-6 * sum_kept : 0x1p-40 * total_d);
                     } else {
                         for (uint32_t j = 0; j < n; ++j)
                             total_d += (double)__shfl_sync(full, q, (int)j);
@@ -1772,6 +1789,18 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         __syncthreads(); // n_final is written again below
         if (tid == 0)
             s.n_final = 0;
+    }
+
+    // Top_p alone, and what was kept does not hold the nucleus, or holds too much to tell here: the row is left to the second
+    // launch, with its maximum and total. (Where no weight can exist there is nothing to look for.)
+    if (cfg.optimistic && !s.nan0 && !cfg.force_none && fabsf(m) < __int_as_float(0x7f800000)) {
+        if (tid == 0) {
+            again[0] = 1u;
+            again[1] = __float_as_uint(m);
+            *reinterpret_cast<double*>(again + 2) = total_approx;
+            if (a.token) a.token[row] = -1;
+        }
+        return;
     }
 
     if (mode == kModeVpLocal) {
@@ -1907,10 +1936,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 total_approx += s.warp_sum[i];
             total_need = sum + total_approx;
             band_need = 1e-5 * total_approx + 0x1p-40 * total_need;
-            if (cfg.optimistic && tid == 0) { // for the second pass, should the row ask for it
-                again[1] = __float_as_uint(m);
-                *reinterpret_cast<double*>(again + 2) = total_need;
-            }
         }
     }
     __syncthreads();
@@ -1922,14 +1947,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     }
     if (!overflow && n > (uint32_t)kSortCap && !cfg.use_topp && !(cfg.top_k > 0 && cfg.top_k < n)) {
         const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                          a.cand_cap, id_off, a.timing, mode, nullptr};
+                          a.cand_cap, id_off, a.timing, mode};
         wide_id_ordered(s, *reinterpret_cast<RowChain*>(dyn + kOffChain), scratch, qrow, n_raw, n, V,
                         fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key)), m, cfg.inv_t, cfg.minp_eff, row,
                         flags, u_row, u2_row, draft_row, o);
         return;
     }
     const unsigned long long* ksrc = keys; // the ordered list: shared memory, or the row's scratch for a long one
-    bool pre_sorted = false;
+    bool pre_sorted = false, list_in_front = true; // the half of the scratch that must not be written over
     if (!overflow && n > (uint32_t)kSortCap && mode != kModeDistOnly) {
         // More candidates than the shared-memory sort holds, and a truncation that orders them (the unordered case
         // returned above): a flat row under top_p, or a very large top_k. The candidates are sorted in global
@@ -1940,6 +1965,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                                                 cfg.minp_eff);
         ksrc = P;
         pre_sorted = true;
+        list_in_front = reinterpret_cast<const uint32_t*>(P) == row_scratch;
         // The float total and the walk below are sequential chains that take 32 candidates per step: fed from global
         // memory they run at the pace of its latency, so a list that fits is staged in shared memory first.
         if (n <= kOffChain / 8u) {
@@ -2052,16 +2078,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         n = cfg.top_k;
     }
     const bool short_list = n <= 128u; // one warp does it all, in the reference's own order, without CTA barriers
-    bool retry = false; // first launch, top_p alone: what was kept does not settle the nucleus; the second pass will
     if (cfg.use_topp && !short_list) {
         const uint32_t kk = wide_top_p(s, ksrc, n, cfg.top_p, cfg.need_sum, cfg.need_sum && !(flags & MK_FLAG_NO_CANDIDATE),
                                        total_need, band_need);
-        if (kk & 0x80000000u) {
-            if (cfg.optimistic)
-                retry = true;
-            else
-                flags |= MK_FLAG_GUARD_BAND;
-        }
+        if (kk & 0x80000000u)
+            flags |= MK_FLAG_GUARD_BAND;
         n = max(kk & 0x7fffffffu, 1u);
     }
 
@@ -2069,9 +2090,13 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         a.timing[(size_t)row * 64 + 13] = global_ns();
     if (!short_list) {
         const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
-                          a.cand_cap, id_off, a.timing, mode, retry ? again : nullptr};
+                          a.cand_cap, id_off, a.timing, mode};
+        // the weights in order go behind the keys where there is room, else to the half of the scratch the list is not in
+        float* q_dense = reinterpret_cast<float*>(dyn + kOffKeys + (((size_t)s.nsurv * 8u + 15u) & ~(size_t)15u));
+        if (pre_sorted || (size_t)s.nsurv * 8u + 16u + (size_t)n * 4u > kOffFinBitmap)
+            q_dense = list_in_front ? qrow : reinterpret_cast<float*>(row_scratch);
         draw_list(s, *reinterpret_cast<RowChain*>(dyn + kOffChain), ksrc, ord, sorted ? kByWeight : (by_rank ? kByRank : kByColumn),
-                  n, row, flags, u_row, u2_row, draft_row, o);
+                  q_dense, n, row, flags, u_row, u2_row, draft_row, o);
     } else
     // A short list: float total and the walk, left to right in the reference's order and precision (sampler.cpp:64-73,
     // 80-83, 100-106), by one warp: every lane loads one candidate, the values go round by shuffle and every lane runs
@@ -2113,12 +2138,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 }
             }
             if ((cfg.need_sum && run < want) ||
-                (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))) {
-                if (cfg.optimistic)
-                    retry = true;
-                else
-                    flags |= MK_FLAG_GUARD_BAND;
-            }
+                (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band))))
+                flags |= MK_FLAG_GUARD_BAND;
             n = max(k, 1u);
         }
         float total = 0.0f, q_draft = 0.0f;
@@ -2243,9 +2264,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             }
         }
         if (lane == 0) {
-            if (retry)
-                again[0] = 1u; // every output of this row is written again by the second pass
-            if (a.token) a.token[row] = retry ? -1 : tok;
+            if (a.token) a.token[row] = tok;
             if (a.prob) a.prob[row] = prob;
             if (a.flags) a.flags[row] = flags;
             if (a.n_cand) a.n_cand[row] = n;
