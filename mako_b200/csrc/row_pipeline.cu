@@ -76,6 +76,7 @@ constexpr int kBins = 2048;     // bins of the top_k histogram (see hist_bin)
 struct __align__(128) Smem {
     double warp_sum[kThreads / 32];
     uint64_t full[kMaxStages], ready[kMaxStages], empty[kMaxStages];
+    unsigned long long exp2_table[32]; // for the finish: a copy of expf_host_exact's table
     unsigned long long best_key;    // (order key of the row maximum << 32) | ~column: first argmax wins
     uint32_t m_key;                 // running maximum, as order key
     uint32_t thr_topk_key;          // top_k lower bound, as order key (only ever raised)
@@ -330,7 +331,7 @@ __device__ __noinline__ void wide_id_ordered(Smem& s, RowChain& cs, const uint2*
         const uint2 c = scratch[i];
         if (!(__uint_as_float(c.x) >= thr_final))
             continue;
-        const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t));
+        const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t), s.exp2_table);
         if (q >= minp_eff && q > 0.0f)
             qrow[c.y] = q;
     }
@@ -618,7 +619,7 @@ __device__ __noinline__ const unsigned long long* long_sort(Smem& s, unsigned lo
         for (int k = 0; k < 4; ++k) {
             const uint2 c = cv[k];
             if (__uint_as_float(c.x) >= thr2) {
-                const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t));
+                const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t), s.exp2_table);
                 if (q >= minp_eff && q > 0.0f)
                     KA[atomicAdd(&s.nsurv, 1u)] = pack_by_weight(q, c.y);
             }
@@ -712,7 +713,7 @@ __device__ __noinline__ void wide_finish(Smem& s, const unsigned long long* fkey
         const float qk = q_at(top_k - 1u);
         const uint32_t edge_key = s.thr_topk_key;
         const float below = key_to_float(edge_key - 1u);
-        if (edge_key > order_key(-FLT_MAX) && expf_host_exact(__fmul_rn(__fsub_rn(below, m), inv_t)) >= qk)
+        if (edge_key > order_key(-FLT_MAX) && expf_host_exact(__fmul_rn(__fsub_rn(below, m), inv_t), s.exp2_table) >= qk)
             fl |= MK_FLAG_GUARD_BAND;
         n = top_k;
     }
@@ -1129,9 +1130,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // ---- streaming ----------------------------------------------------------------------------------------------
     if (a.timing && tid == 0)
         a.timing[(size_t)row * 64 + 1] = global_ns();
-    float best = -__int_as_float(0x7f800000);
-    int32_t best_col = -1;
-    double sum_acc = 0.0; // need_sum: sum of exp2((l - best) * c2) over this thread's uncollected elements
+    float seen = -__int_as_float(0x7f800000); // the largest element of the row this warp knows of
+    double sum_acc = 0.0; // need_sum: sum of exp2((l - seen) * c2) over this thread's elements (the uncollected ones)
 
     if (warp == 0) {
         // producer
@@ -1185,6 +1185,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         // fix-up: each of the two warps owns every other tile of those that follow the ones edited above (a long
         // history: warp 0 owns them all, because its per-tile counters are shared), so two tiles are edited at a time
         // and nothing synchronises across warps
+        if (warp == kFixers / 32)
+            s.exp2_table[lane] = kExp2Tab[lane]; // before the row's readers need anything of these warps
         if (has_special) {
             const uint32_t fw = warp - 1;
             if (fw == 0 && lane == 0)
@@ -1256,7 +1258,20 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         // A nucleus that is to be found among the few largest, or a shard record: the streamed sum takes every element.
         const bool sum_all = mode == kModeVpLocal || cfg.optimistic;
         const bool hist_bound_alone = !(cfg.minp_eff > 0.0f) && cfg.hist_k <= kVpMaxK + 1u;
-        float warp_pub = ninf;
+        // What a thread keeps of its elements, four at a time: it is rarely more than one.
+        auto keep_fours = [&](const float (&tq)[kVec], const float (&w)[kEl], float thr, uint32_t base) {
+#pragma unroll
+            for (int j = 0; j < kVec; ++j)
+                if (tq[j] >= thr) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (w[4 * j + c] >= thr) {
+                            const uint32_t slot = atomicAdd(&s.ncand, 1u);
+                            if (slot < scratch_cap)
+                                scratch[slot] = make_uint2(__float_as_uint(w[4 * j + c]), base + j * 1024 + rt * 4 + c);
+                        }
+                }
+        };
         // The loop over the tiles is compiled four times, with the mask, the top_k histogram and the streamed sum
         // compiled in or out: a row runs a variant that holds little beyond its own work. (One loop with all
         // three as run-time branches costs the common penalised row 12 % of its launch time, and all eight
@@ -1325,25 +1340,33 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 if (t == 0 && rt == 0 && w[0] != w[0])
                     s.nan0 = 1;
 
-                float tm = ninf;
+                float tq[kVec], tm = ninf; // the largest of each four, and of all (NaN is never the larger)
 #pragma unroll
-                for (int e = 0; e < kEl; ++e)
-                    tm = fmaxf(tm, w[e]);
-                const float old_best = best;
-                if (tm > best) {
-                    best = tm;
-#pragma unroll
-                    for (int e = kEl - 1; e >= 0; --e)
-                        if (w[e] == tm)
-                            best_col = (int32_t)(base + (e >> 2) * 1024 + rt * 4 + (e & 3));
+                for (int j = 0; j < kVec; ++j) {
+                    tq[j] = fmaxf(fmaxf(fmaxf(w[4 * j], ninf), w[4 * j + 1]), fmaxf(w[4 * j + 2], w[4 * j + 3]));
+                    tm = fmaxf(tm, tq[j]);
                 }
-                if (!(kHist && cfg.hist_mode && hist_bound_alone) && __any_sync(0xffffffffu, tm > warp_pub)) {
-                    const float wm = warp_max(tm);
-                    if (wm > warp_pub) {
-                        warp_pub = wm;
-                        if (lane == 0)
+                // An element that is the row's maximum is at or above all its warp knows of. Only a warp that may hold
+                // one — a dozen tiles of a row, not most of them, as it would be for every thread's own maximum —
+                // looks for its column, the first of equals.
+                if (__any_sync(0xffffffffu, tm >= seen)) {
+                    const float wm = warp_max(tm), before = seen;
+                    const float m_run = key_to_float(__shfl_sync(0xffffffffu, *(volatile uint32_t*)&s.m_key, 0));
+                    if (wm >= m_run && wm > ninf) {
+                        uint32_t col = 0xffffffffu;
+#pragma unroll
+                        for (int e = kEl - 1; e >= 0; --e)
+                            if (w[e] == wm)
+                                col = base + (e >> 2) * 1024 + rt * 4 + (e & 3);
+                        col = __reduce_min_sync(0xffffffffu, col);
+                        if (lane == 0) {
                             atomicMax(&s.m_key, order_key(wm));
+                            atomicMax(&s.best_key, ((unsigned long long)order_key(wm) << 32) | (unsigned long long)(0xffffffffu - col));
+                        }
                     }
+                    seen = fmaxf(wm, m_run);
+                    if (kSum && cfg.need_sum && seen > before)
+                        sum_acc *= (double)exp2f((before - seen) * c2);
                 }
                 // Under the histogram bound the distance from the maximum only matters where min_p or a large top_k makes
                 // it the tighter of the two.
@@ -1407,32 +1430,23 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             thr = fmaxf(thr, key_to_float(*(volatile uint32_t*)&s.thr_topk_key));
                         }
                     }
-                    if (collect && tm >= thr) {
-#pragma unroll
-                        for (int e = 0; e < kEl; ++e)
-                            if (w[e] >= thr) {
-                                const uint32_t slot = atomicAdd(&s.ncand, 1u);
-                                if (slot < scratch_cap)
-                                    scratch[slot] = make_uint2(__float_as_uint(w[e]), base + (e >> 2) * 1024 + rt * 4 + (e & 3));
-                            }
-                    }
+                    if (collect && tm >= thr)
+                        keep_fours(tq, w, thr, base);
                 }
-                if (kSum && cfg.need_sum && best > ninf) {
-                    // Approximate weights, relative to the thread's running maximum. Of a row that keeps the few largest (and
+                if (kSum && cfg.need_sum && seen > ninf) {
+                    // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest (and
                     // of a shard record) every element; else of what is NOT collected (`thr` is the bound
                     // the collection used): the collected elements get exact weights in the finish, so only the far tail
                     // carries the approximation. NaN weighs nothing.
-                    if (best > old_best)
-                        sum_acc *= (double)exp2f((old_best - best) * c2);
                     float p = 0.0f;
                     if (kHist && sum_all) { // (the maximum with -inf is what a NaN turns into)
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
-                            p += ex2_approx((fmaxf(w[e], ninf) - best) * c2);
+                            p += ex2_approx((fmaxf(w[e], ninf) - seen) * c2);
                     } else {
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
-                            p += w[e] < thr ? ex2_approx((w[e] - best) * c2) : 0.0f;
+                            p += w[e] < thr ? ex2_approx((w[e] - seen) * c2) : 0.0f;
                     }
                     sum_acc += (double)p;
                 }
@@ -1469,14 +1483,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                                 }
                         }
                     } else if (some) {
-#pragma unroll
-                        for (int e = 0; e < kEl; ++e)
-                            if (w[e] >= thr) {
-                                const uint32_t slot = atomicAdd(&s.ncand, 1u);
-                                const uint2 c = make_uint2(__float_as_uint(w[e]), base + (e >> 2) * 1024 + rt * 4 + (e & 3));
-                                if (slot < scratch_cap)
-                                    scratch[slot] = c;
-                            }
+                        keep_fours(tq, w, thr, base);
                     }
                 }
             }
@@ -1493,9 +1500,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             read_tiles(F{}, T{}, T{}, F{}); // top_p alone (with its first-launch histogram), shard records
         else
             read_tiles(T{}, T{}, T{}, F{}); // masked rows: everything, chosen at run time
-        if (best_col >= 0)
-            atomicMax(&s.best_key,
-                      ((unsigned long long)order_key(best) << 32) | (unsigned long long)(0xffffffffu - (uint32_t)best_col));
     }
     __syncthreads();
 
@@ -1534,8 +1538,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         double part = 0.0;
         if (warp > kFixers / 32) {
             const float c2 = cfg.inv_t * 1.4426950408889634f;
-            if (best > -__int_as_float(0x7f800000) && sum_acc > 0.0)
-                part += sum_acc * exp2((double)(best - m) * (double)c2);
+            if (seen > -__int_as_float(0x7f800000) && sum_acc > 0.0)
+                part += sum_acc * exp2((double)(seen - m) * (double)c2);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -1585,7 +1589,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     const uint2 c = craw[i];
                     float q = 0.0f;
                     if (__uint_as_float(c.x) >= thr_final) {
-                        q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t));
+                        q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table);
                     }
                     if (kRowTotal) {
                         // as streamed: of a kept element to be taken out again where the sum took every element, of
@@ -1654,7 +1658,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     const uint32_t edge_key = s.thr_topk_key;
                     const float below = key_to_float(edge_key - 1u);
                     if (edge_key > order_key(-FLT_MAX) &&
-                        expf_host_exact(__fmul_rn(__fsub_rn(below, m), cfg.inv_t)) >= qk)
+                        expf_host_exact(__fmul_rn(__fsub_rn(below, m), cfg.inv_t), s.exp2_table) >= qk)
                         fl |= MK_FLAG_GUARD_BAND;
                     n = cfg.top_k;
                 }
@@ -1902,7 +1906,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     continue;
                 }
                 const float x = __fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t);
-                const float q = expf_host_exact(x);
+                const float q = expf_host_exact(x, s.exp2_table);
                 if (q == q)
                     exact += (double)q;
                 if (in && q >= cfg.minp_eff && q > 0.0f) {
@@ -2073,7 +2077,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         const float qk = q_of(cfg.top_k - 1);
         const uint32_t edge_key = s.thr_topk_key;
         const float below = key_to_float(edge_key - 1u);
-        if (edge_key > order_key(-FLT_MAX) && expf_host_exact(__fmul_rn(__fsub_rn(below, m), cfg.inv_t)) >= qk)
+        if (edge_key > order_key(-FLT_MAX) && expf_host_exact(__fmul_rn(__fsub_rn(below, m), cfg.inv_t), s.exp2_table) >= qk)
             flags |= MK_FLAG_GUARD_BAND;
         n = cfg.top_k;
     }
