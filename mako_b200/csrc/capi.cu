@@ -142,7 +142,6 @@ void fill_common(mk::RowKernelArgs& a, const mk_sampler* s, const mk_rows* r)
     a.overlap = s->overlap;
     a.debug_skip_tile = s->skip_tile;
     a.debug_wait_probes = s->wait_probes;
-    a.use_bulk_copy = ((reinterpret_cast<uintptr_t>(r->logits) & 15u) == 0 && (r->ld % 4u) == 0) ? 1 : 0;
 }
 
 void fill_out(mk::RowKernelArgs& a, const mk_sample_out* o)
@@ -168,7 +167,7 @@ bool all_greedy(const mk_rows* r)
 // run again as one CTA by a follow-up launch that skips every other row, so the results are those of the plain path.
 bool split_eligible(const mk_sampler* s, const mk_rows* r, const mk::RowKernelArgs& a)
 {
-    if (!s->split || r->batch == 0 || r->batch > kSplitMaxBatch || r->params_dev || !a.use_bulk_copy)
+    if (!s->split || r->batch == 0 || r->batch > kSplitMaxBatch || r->params_dev)
         return false;
     const mk_sampling_params& p = r->params;
     if (!(p.temperature > 0.0f) || p.top_k == 0 || p.top_k > mk::kVpMaxK)

@@ -835,11 +835,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     const uint32_t warp = tid >> 5, lane = tid & 31;
     // a split launch: CTA (row, g) takes columns [g * split_w, ...) of the row, and that share of the row's scratch
     const uint32_t col0 = kSplit ? blockIdx.y * a.split_w : 0u;
-    const uint32_t V = kSplit ? min(a.split_w, a.n_vocab - col0) : a.n_vocab;
-    const int32_t id_off = kSplit ? a.id_offset + (int32_t)col0 : a.id_offset;
+    const uint32_t n_cols = kSplit ? min(a.split_w, a.n_vocab - col0) : a.n_vocab;
+    // The bulk copies start at 16-byte boundaries. A row that does not is taken from the boundary before it: the places of
+    // the row below are its columns moved up by `shift`, and the up to three places in front, which lie in the same 16 bytes
+    // as the row's first column, read as -inf. 256 x 50257 packed rows: 210 us by plain loads of one warp, 37 us so.
+    const uint32_t shift = (uint32_t)((reinterpret_cast<uintptr_t>(a.logits + (size_t)row * a.ld + col0) >> 2) & 3u);
+    const uint32_t V = n_cols + shift;
+    const int32_t id_off = (kSplit ? a.id_offset + (int32_t)col0 : a.id_offset) - (int32_t)shift;
     const uint32_t scratch_cap = kSplit ? min(a.split_w, a.scratch_cap - col0) : a.scratch_cap;
     const uint32_t n_tiles = (V + kTile - 1) / kTile;
-    const float* __restrict__ lrow = a.logits + (size_t)row * a.ld + col0;
+    const float* __restrict__ lrow = a.logits + (size_t)row * a.ld + col0 - shift;
     // A speculative round (src/gen/session.cpp:451-506): row = sequence * n_pos + position. Position j < n_pos - 1
     // verifies draft j, the last one is the bonus row and is sampled; the penalties of position j count the sequence's
     // history plus drafts 0..j-1 (each accepted draft is emit()ted before the next row is looked at, :491); a forced
@@ -902,7 +907,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             hc[i] = (j < hlen) ? (uint32_t)hist_at(j) - (uint32_t)id_off : 0xffffffffu;
         }
     }
-    const RowCfg cfg = make_cfg(prm, V, mode, a.vp_k, a.pass);
+    const RowCfg cfg = make_cfg(prm, n_cols, mode, a.vp_k, a.pass);
     const uint32_t* __restrict__ mrow = a.mask ? a.mask + (size_t)row * a.mask_ld + (col0 >> 5) : nullptr;
     // Per-row scratch, 16 bytes per column: scratch_cap raw candidates (logit bits, column) — sorted in place as
     // 64-bit keys by the large sorted-list path — then as much again: the merge sort's second buffer, or (large
@@ -990,8 +995,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // The producer fills the ring before anything else, so that the copies fly during the set-up (unless the set-up
     // runs ahead of the previous kernel: then the logits come after the wait below). With a history the last stage
     // first serves the set-up as a list (see below) and is requested once that list has been used.
-    const uint32_t tiles_issued = a.use_bulk_copy ? min(n_stages, n_tiles) : 0u;
-    const bool list_owners = use_table && has_hist && tiles_issued > 0;
+    const uint32_t tiles_issued = min(n_stages, n_tiles);
+    const bool list_owners = use_table && has_hist;
     const uint32_t tiles_early = (list_owners && tiles_issued == n_stages) ? n_stages - 1u : tiles_issued;
     auto fill_ring = [&](uint32_t t0, uint32_t t1) {
         for (uint32_t t = t0; t < t1; ++t) {
@@ -1160,25 +1165,17 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 break;
             if (t == a.debug_skip_tile)
                 continue;
-            if (a.use_bulk_copy) {
-                if (lane == 0) {
-                    fence_proxy_async();
-                    const uint32_t bytes = (n_t * 4u) & ~15u;
-                    for (uint32_t e = bytes / 4; e < n_t; ++e)
-                        dst[e] = src[e];
-                    if (bytes > 0) {
-                        mbar_arrive_expect_tx(&s.full[st], bytes);
-                        bulk_load(dst, src, bytes, &s.full[st]);
-                    } else {
-                        mbar_arrive(&s.full[st]);
-                    }
-                }
-            } else {
-                for (uint32_t e = lane; e < n_t; e += 32)
+            if (lane == 0) {
+                fence_proxy_async();
+                const uint32_t bytes = (n_t * 4u) & ~15u;
+                for (uint32_t e = bytes / 4; e < n_t; ++e)
                     dst[e] = src[e];
-                __syncwarp();
-                if (lane == 0)
+                if (bytes > 0) {
+                    mbar_arrive_expect_tx(&s.full[st], bytes);
+                    bulk_load(dst, src, bytes, &s.full[st]);
+                } else {
                     mbar_arrive(&s.full[st]);
+                }
             }
         }
     } else if (warp <= kFixers / 32) {
@@ -1283,7 +1280,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 #pragma unroll
             for (int j = 0; j < kVec; ++j) {
                 const uint32_t i0 = j * 1024 + rt * 4;
-                mw_next[j] = (kMask && mrow) ? ((i0 < V) ? __ldg(mrow + (i0 >> 5)) : 0u) : 0xffffffffu;
+                mw_next[j] = (kMask && mrow) ? ((i0 < n_cols) ? __ldg(mrow + (i0 >> 5)) : 0u) : 0xffffffffu;
             }
             uint32_t st = 0, k = 0;
             for (uint32_t t = 0; t < n_tiles; ++t, ++st) {
@@ -1300,7 +1297,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 #pragma unroll
                     for (int j = 0; j < kVec; ++j) {
                         const uint32_t i0 = base + kTile + j * 1024 + rt * 4;
-                        mw_next[j] = (i0 < V) ? __ldg(mrow + (i0 >> 5)) : 0u;
+                        mw_next[j] = (i0 < n_cols) ? __ldg(mrow + (i0 >> 5)) : 0u;
                     }
                 }
                 if (!mbar_wait(&avail[st], k & 1, (*(volatile uint32_t*)&s.abort_flag) ? 1u : wait_probes))
@@ -1322,7 +1319,13 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 if (kMask && mrow) {
 #pragma unroll
                     for (int j = 0; j < kVec; ++j) {
-                        const uint32_t bits = mw[j] >> ((rt * 4) & 31);
+                        uint32_t bits = mw[j] >> ((rt * 4) & 31);
+                        if (shift) { // four columns that may lie in two words, neither of them the one that was requested
+                            const int32_t c = (int32_t)(base + j * 1024 + rt * 4) - (int32_t)shift, wd = c >> 5;
+                            const uint32_t lo = (wd >= 0 && wd * 32 < (int32_t)n_cols) ? __ldg(mrow + wd) : 0u;
+                            const uint32_t hi = ((wd + 1) * 32 < (int32_t)n_cols) ? __ldg(mrow + wd + 1) : 0u;
+                            bits = __funnelshift_r(lo, hi, (uint32_t)c & 31u);
+                        }
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
                             if (!((bits >> c) & 1u))
@@ -1337,8 +1340,17 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             if (base + j * 1024 + rt * 4 + c >= V)
                                 w[4 * j + c] = ninf;
                 }
-                if (t == 0 && rt == 0 && w[0] != w[0])
-                    s.nan0 = 1;
+                if (t == 0 && rt == 0) {
+                    float first = w[0];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        if ((uint32_t)c < shift) {
+                            first = w[c + 1];
+                            w[c] = ninf;
+                        }
+                    if (first != first)
+                        s.nan0 = 1;
+                }
 
                 float tq[kVec], tm = ninf; // the largest of each four, and of all (NaN is never the larger)
 #pragma unroll
@@ -1522,10 +1534,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 
     const bool any_finite = s.best_key != 0ull;
     float m = any_finite ? key_to_float((uint32_t)(s.best_key >> 32)) : -__int_as_float(0x7f800000);
-    uint32_t arg_col = any_finite ? (0xffffffffu - (uint32_t)(s.best_key & 0xffffffffull)) : 0u;
+    uint32_t arg_col = any_finite ? (0xffffffffu - (uint32_t)(s.best_key & 0xffffffffull)) : shift;
     if (s.nan0) { // max_element keeps a NaN in front: every weight is NaN, the first column is returned
         m = __int_as_float(0x7fc00000);
-        arg_col = 0;
+        arg_col = shift;
     }
     uint32_t flags = hlen_clamped ? MK_FLAG_HISTORY_FULL : 0u;
     if (mrow && !any_finite && !s.nan0)
@@ -1837,7 +1849,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             float* hf = reinterpret_cast<float*>(rec);
             uint32_t* hu = reinterpret_cast<uint32_t*>(rec);
             hf[0] = m;
-            hu[1] = n_out | (over ? 0x80000000u : 0u) | ((V > a.vp_k) ? 0x40000000u : 0u);
+            hu[1] = n_out | (over ? 0x80000000u : 0u) | ((n_cols > a.vp_k) ? 0x40000000u : 0u);
             *reinterpret_cast<double*>(rec + 8) = total_approx;
         }
         for (uint32_t i = tid; i < a.vp_k; i += kThreads) {

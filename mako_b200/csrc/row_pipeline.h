@@ -53,7 +53,6 @@ struct RowKernelArgs {
     unsigned long long* timing; // optional [batch][64] ns timestamps (slots: see mk_debug_set_timing)
     int mode;
     int pass;              // 0: first launch; 1: second pass, only the rows that asked for it (set by launch_row_kernel)
-    int use_bulk_copy;     // 1: TMA bulk staging (aligned rows); 0: plain loads
     int overlap;           // MK_OVERLAP_*: launch behind the previous kernel of the stream programmatically
     // a speculative round: row = sequence * spec_n_pos + position (0: off); history and history_len are per sequence
     uint32_t spec_n_pos;
