@@ -490,7 +490,7 @@ def run_other(args, cfg_id: int, dev, timer: Timer, peak: float, peak_kind: str)
         d = to_device(make_inputs(cfg, 0, 1), dev)[0]
         s = BatchSampler(v, 1, dev.index)
         s.set_overlap(args.overlap)
-        for split, tag, launches in ((True, ", one row per step split over 37 CTAs", 3),
+        for split, tag, launches in ((True, ", one row per step split over 37 CTAs", 1),
                                      (False, ", one row per step as one CTA", 1)):
             s.set_split(split)
             g = capture(dev, lambda k: s.sample(d["logits"][k % pool:k % pool + 1], params,

@@ -41,8 +41,8 @@ int cuda_fail(cudaError_t e, const char* what)
 inline uint32_t scratch_cap(uint32_t n_vocab) { return (n_vocab + 3u) & ~3u; }
 
 constexpr uint32_t kPqCap = 4096;      // candidates per list in p/q verification
-constexpr uint32_t kSplitMaxBatch = 8, kSplitMaxShards = 64, kSplitKeys = 1024;
 constexpr uint32_t kMaxTiles = 512, kTile = 4096;
+constexpr uint32_t kPlaces = 296; // CTAs of the row kernel that are resident at once: two on each of 148 SMs
 
 } // namespace
 
@@ -65,9 +65,9 @@ struct mk_sampler {
     unsigned long long* pick_best = nullptr; // mk_draft_pick: one packed (score, id) maximum per sequence
     unsigned char* stage = nullptr;
     size_t stage_bytes = 0;
-    // small batches under a top_k: every row split over many CTAs (shard records, then the merge)
-    unsigned char* split_records = nullptr; // [kSplitMaxShards][kSplitMaxBatch] records of kVpMaxK entries
-    uint32_t* split_flags = nullptr;        // [kSplitMaxBatch], when the caller asks for no flags
+    // small batches: every row split over many CTAs; twice, for the two row sets of p/q verification
+    mk::SplitPart* split_parts = nullptr; // [2][kSplitMaxRows][kMaxSlices]
+    uint32_t* split_tickets = nullptr;    // [2][kSplitMaxRows], zero between launches
     int split = 1;                          // 0: every batch runs as one CTA per row
 };
 
@@ -160,68 +160,30 @@ bool all_greedy(const mk_rows* r)
     return !r->params_dev && r->params.temperature <= 0.0f;
 }
 
-// A handful of rows under a top_k leaves most of the device idle when each row is one CTA, and the top_k bound costs
-// that CTA a histogram update per element. Such a batch is split instead: every row's columns go to many CTAs, each
-// writing the record a vocabulary shard writes (maximum, partial sum, its best entries); the merge draws from the
-// records. A row the merge cannot prove complete (VP_TRUNCATED: one shard's whole list inside the deciding set) is
-// run again as one CTA by a follow-up launch that skips every other row, so the results are those of the plain path.
-bool split_eligible(const mk_sampler* s, const mk_rows* r, const mk::RowKernelArgs& a)
+// A few rows leave most of the device idle when each is one CTA. Their columns are split instead, into as many slices as fill
+// the device's 296 places once (of at least a tile of 4096 columns), and the last CTA of a row to arrive draws from what all of
+// them kept. Measured (us a call, split / one CTA a row), 151552 columns: one row top_k 18.5 / 35.6, top_p 20.2 / 42.7, min_p
+// 12.3 / 20.7, greedy 7.0 / 16.9; 64 rows 33.3 / 36.7, 93 / 100, 23.3 / 26.9, 14.1 / 17.2; more rows fill the device by
+// themselves. Eight tiles (32000 columns): a row under the histogram bound still gains (top_k 14.1 / 17.3, top_p 17.1 / 19.7),
+// the others lose a microsecond to the meeting of their slices (min_p 9.4 / 8.0, greedy 6.8 / 6.4), so short rows are
+// split only under that bound. `set`: which of the two row sets of p/q verification (0 elsewhere).
+void split_rows(mk::RowKernelArgs& a, const mk_sampler* s, uint32_t batch, uint32_t set)
 {
-    if (!s->split || r->batch == 0 || r->batch > kSplitMaxBatch || r->params_dev)
-        return false;
-    const mk_sampling_params& p = r->params;
-    if (!(p.temperature > 0.0f) || p.top_k == 0 || p.top_k > mk::kVpMaxK)
-        return false;
-    if (r->n_vocab < 4u * kTile || r->id_offset < 0 || (uint64_t)r->id_offset + r->n_vocab > (1u << 26))
-        return false;
-    return s->timing == nullptr && s->skip_tile == 0xffffffffu;
-}
-
-int sample_split(mk_sampler* s, const mk_rows* rows, mk::RowKernelArgs a, const mk_sample_out* out, cudaStream_t stream)
-{
-    (void)out;
-    const uint32_t n_tiles = (rows->n_vocab + kTile - 1) / kTile;
-    const uint32_t per = (n_tiles + kSplitMaxShards - 1) / kSplitMaxShards; // tiles per shard
-    const uint32_t n_shards = (n_tiles + per - 1) / per;
-    uint32_t k = kSplitKeys / n_shards;
-    k = k > mk::kVpMaxK ? mk::kVpMaxK : (k < 8u ? 8u : k);
-    mk::RowKernelArgs first = a;
-    first.mode = mk::kModeVpLocal;
-    first.split_w = per * kTile;
-    first.vp_records = s->split_records;
-    first.vp_k = k;
-    first.token = nullptr;
-    first.prob = nullptr;
-    first.flags = nullptr;
-    first.n_cand = nullptr;
-    first.cand_ids = nullptr;
-    first.cand_q = nullptr;
-    MK_CUDA(mk::launch_row_kernel(first, rows->batch, stream));
-    mk::VpMergeArgs m;
-    std::memset(&m, 0, sizeof m);
-    m.gathered = s->split_records;
-    m.n_shards = n_shards;
-    m.batch = rows->batch;
-    m.k = k;
-    m.n_vocab_total = rows->n_vocab;
-    m.params = rows->params;
-    m.u = a.u;
-    m.token = a.token;
-    m.prob = a.prob;
-    m.flags = a.flags ? a.flags : s->split_flags;
-    m.n_cand = a.n_cand;
-    m.cand_ids = a.cand_ids;
-    m.cand_q = a.cand_q;
-    m.cand_cap = a.cand_cap;
-    MK_CUDA(mk::launch_vp_merge(m, stream));
-    // the rows the merge reported incomplete, as one CTA each; this launch reads the flags the merge wrote, so it is
-    // never started ahead of it
-    a.overlap = MK_OVERLAP_OFF;
-    a.only_flagged = m.flags;
-    a.only_flagged_mask = MK_FLAG_VP_TRUNCATED;
-    a.flags = m.flags;
-    MK_CUDA(mk::launch_row_kernel(a, rows->batch, stream));
-    return MK_OK;
+    if (!s->split || !s->split_parts || batch == 0 || batch > mk::kSplitMaxRows || s->timing || s->skip_tile != 0xffffffffu)
+        return;
+    const uint32_t n_tiles = (a.n_vocab + kTile - 1) / kTile;
+    uint32_t per = (n_tiles * batch + kPlaces - 1) / kPlaces; // tiles per slice
+    const mk_sampling_params& p = a.params;
+    const bool bound = !a.params_dev && p.temperature > 0.0f && ((p.top_k > 0 && p.top_k < a.n_vocab) || (p.top_p < 1.0f && !(p.min_p > 0.0f)));
+    if (n_tiles < (bound ? 4u : 12u))
+        return;
+    const uint32_t least = (n_tiles + mk::kMaxSlices - 1) / mk::kMaxSlices;
+    per = per < least ? least : per;
+    if (per >= n_tiles)
+        return;
+    a.split_w = per * kTile;
+    a.parts = s->split_parts + (size_t)set * mk::kSplitMaxRows * mk::kMaxSlices;
+    a.tickets = s->split_tickets + (size_t)set * mk::kSplitMaxRows;
 }
 
 } // namespace
@@ -313,8 +275,11 @@ int mk_sampler_create(mk_sampler** out, int device, uint32_t n_vocab, uint32_t m
     alloc((void**)&s->q_flags, b * 4);
     alloc((void**)&s->p_tok, b * 4);
     alloc((void**)&s->pick_best, (mk::kDraftPickMaxSeq + 1) * sizeof(unsigned long long)); // maxima + ticket counter
-    alloc((void**)&s->split_records, (size_t)kSplitMaxShards * kSplitMaxBatch * mk::vp_record_bytes(mk::kVpMaxK));
-    alloc((void**)&s->split_flags, kSplitMaxBatch * 4);
+    const size_t split_rows_max = 2u * (size_t)mk::kSplitMaxRows;
+    alloc((void**)&s->split_parts, split_rows_max * mk::kMaxSlices * sizeof(mk::SplitPart));
+    alloc((void**)&s->split_tickets, split_rows_max * 4);
+    if (e == cudaSuccess)
+        e = cudaMemset(s->split_tickets, 0, split_rows_max * 4);
     if (e == cudaSuccess)
         e = cudaMemset(s->pick_best, 0, (mk::kDraftPickMaxSeq + 1) * sizeof(unsigned long long));
     if (e == cudaSuccess)
@@ -338,7 +303,7 @@ void mk_sampler_destroy(mk_sampler* s)
     DeviceGuard g(s->device);
     void* ptrs[] = {s->scratch, s->p_ids, s->q_ids, s->p_q, s->q_q, s->p_total, s->q_total, s->q_prob,
                     s->p_n,     s->q_n,   s->p_flags, s->q_flags, s->p_tok, s->stage, s->pick_best,
-                    s->split_records, s->split_flags, s->scratch_pq};
+                    s->split_parts, s->split_tickets, s->scratch_pq};
     for (void* p : ptrs)
         if (p)
             cudaFree(p);
@@ -365,8 +330,7 @@ int mk_sampler_sample_batch(mk_sampler* s, const mk_rows* rows, const float* u, 
     fill_out(a, out);
     a.u = u;
     a.mode = mk::kModeSample;
-    if (split_eligible(s, rows, a))
-        return sample_split(s, rows, a, out, (cudaStream_t)stream);
+    split_rows(a, s, rows->batch, 0);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, (cudaStream_t)stream));
     return MK_OK;
 }
@@ -437,6 +401,7 @@ int mk_sampler_verify_batch(mk_sampler* s, const mk_rows* rows, const int32_t* d
     a.draft = draft;
     a.accepted = accepted;
     a.mode = mk::kModeVerify;
+    split_rows(a, s, rows->batch, 0);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, (cudaStream_t)stream));
     return MK_OK;
 }
@@ -477,6 +442,7 @@ int mk_sampler_verify_pq_batch(mk_sampler* s, const mk_rows* rows, const float* 
     a.cand_cap = kPqCap;
     a.total_out = s->q_total;
     a.mode = mk::kModeSample;
+    split_rows(a, s, rows->batch, 0);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, st));
     // target rows: p's list
     fill_common(a, s, rows);
@@ -490,6 +456,7 @@ int mk_sampler_verify_pq_batch(mk_sampler* s, const mk_rows* rows, const float* 
     a.mode = mk::kModeDistOnly;
     a.scratch = s->scratch_pq;
     a.overlap = MK_OVERLAP_OFF; // nothing precedes it in that stream but the fork
+    split_rows(a, s, rows->batch, 1);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, s->own_stream));
     MK_CUDA(cudaEventRecord(s->ev_join, s->own_stream));
     MK_CUDA(cudaStreamWaitEvent(st, s->ev_join, 0));

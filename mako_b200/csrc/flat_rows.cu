@@ -167,8 +167,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
         const uint32_t r_mine = chunk + tid;
         bool marked = false;
         if (r_mine < batch)
-            marked = a.scratch[(size_t)r_mine * row_scratch_words(a.scratch_cap) + 4ull * a.scratch_cap] != 0u &&
-                     !(a.only_flagged && !(a.only_flagged[r_mine] & a.only_flagged_mask));
+            marked = a.scratch[(size_t)r_mine * row_scratch_words(a.scratch_cap) + 4ull * a.scratch_cap] != 0u;
         uint32_t n_marked;
         const uint32_t at = seen + block_exclusive(s, marked ? 1u : 0u, n_marked);
         if (n_marked == 0u)

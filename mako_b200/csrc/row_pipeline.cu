@@ -29,8 +29,8 @@
 //                 their own.
 //   second pass   top_p alone: the first launch keeps the 24 largest elements; a row whose nucleus that does not
 //                 settle marks itself, and a second launch of this kernel streams the marked rows again.
-//   split launch  a few rows under a top_k: a second grid dimension over column shards, each CTA writing a shard
-//                 record for the merge kernel (also the local step of vocab-parallel sampling).
+//   split launch  a few rows: a second grid dimension over slices of the columns; every CTA keeps what its slice's bounds
+//                 leave, the last one of a row to arrive narrows that to the row's own bounds and finishes.
 //
 // Numeric contract (what makes ids bit-exact): IEEE division and no FMA contraction in the penalties and in
 // (l - max) * inv_t; q through expf_host_exact; top_p sums in double; total and the walk in float, left to right.
@@ -136,6 +136,28 @@ __device__ __forceinline__ float hist_bin_floor(uint32_t b)
         return -__int_as_float(0x7f800000);
     const uint32_t q = p + 1u;
     return -__uint_as_float((((q >> 5) + 117u) << 23) | ((q & 31u) << 18));
+}
+
+// The highest bin in which the count from the top reaches k, or -1: by one warp, 32 bins at a time from group `hi_group` down.
+__device__ __forceinline__ int hist_scan(const volatile uint32_t* hist, uint32_t hi_group, uint32_t k)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t cum = 0;
+    int found = -1;
+    for (int g = (int)hi_group; g >= 0 && found < 0; --g) {
+        uint32_t suf = hist[g * 32 + lane]; // suffix sum over lanes >= lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_down_sync(0xffffffffu, suf, o);
+            if ((int)lane + o < 32)
+                suf += y;
+        }
+        const uint32_t hit = __ballot_sync(0xffffffffu, cum + suf >= k);
+        if (hit)
+            found = g * 32 + (31 - __clz(hit));
+        cum += __shfl_sync(0xffffffffu, suf, 0);
+    }
+    return found;
 }
 
 __device__ __forceinline__ float warp_max(float v)
@@ -598,13 +620,13 @@ __device__ __noinline__ void mass_cut(Smem& s, unsigned char* dyn, const uint2* 
 // More candidates than the shared-memory sort holds, in an order that matters: the survivors (exact weight, min_p) are
 // compacted into the second half of the row's scratch as sort keys, sorted as kSortCap-key runs in shared memory,
 // then merged pairwise between the two halves. Returns where the sorted list of n keys ends up. Whole CTA.
-__device__ __noinline__ const unsigned long long* long_sort(Smem& s, unsigned long long* keys, uint2* scratch, uint32_t cap,
+__device__ __noinline__ const unsigned long long* long_sort(Smem& s, unsigned long long* keys, uint2* scratch, float* other,
                                                             uint32_t n_raw, uint32_t n, float thr2, float m, float inv_t,
                                                             float minp_eff)
 {
     const uint32_t tid = threadIdx.x;
-    unsigned long long* KA = reinterpret_cast<unsigned long long*>(scratch) + cap; // second half
-    unsigned long long* KB = reinterpret_cast<unsigned long long*>(scratch);                 // over the raw list
+    unsigned long long* KA = reinterpret_cast<unsigned long long*>(other);   // the half the raw list is not in
+    unsigned long long* KB = reinterpret_cast<unsigned long long*>(scratch); // over the raw list
     if (tid == 0)
         s.nsurv = 0;
     __syncthreads();
@@ -822,8 +844,8 @@ __device__ __noinline__ void wide_finish(Smem& s, const unsigned long long* fkey
 
 // kSpec: the rows of a speculative round (row = sequence * n_pos + position); compiled apart, so that the plain
 // kernel carries none of its bookkeeping.
-// kSplit: a launch whose grid has a second dimension over column shards of every row (shard records of a few rows
-// split over many CTAs: the single-row latency path).
+// kSplit: a launch whose grid has a second dimension over slices of every row's columns (a few rows split over many CTAs: the
+// latency path; one row of 151552 columns under top_k 40 / top_p 0.95 41 us as shard records and a merge, 18.5 us so).
 template <bool kSpec, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKernelArgs a)
 {
@@ -833,16 +855,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     const uint32_t row = blockIdx.x;
     const uint32_t tid = threadIdx.x;
     const uint32_t warp = tid >> 5, lane = tid & 31;
-    // a split launch: CTA (row, g) takes columns [g * split_w, ...) of the row, and that share of the row's scratch
+    // a split launch: CTA (row, g) takes columns [g * split_w, ...) of the row, and their share of the row's list
     const uint32_t col0 = kSplit ? blockIdx.y * a.split_w : 0u;
-    const uint32_t n_cols = kSplit ? min(a.split_w, a.n_vocab - col0) : a.n_vocab;
+    uint32_t n_cols = kSplit ? min(a.split_w, a.n_vocab - col0) : a.n_vocab;
     // The bulk copies start at 16-byte boundaries. A row that does not is taken from the boundary before it: the places of
     // the row below are its columns moved up by `shift`, and the up to three places in front, which lie in the same 16 bytes
     // as the row's first column, read as -inf. 256 x 50257 packed rows: 210 us by plain loads of one warp, 37 us so.
     const uint32_t shift = (uint32_t)((reinterpret_cast<uintptr_t>(a.logits + (size_t)row * a.ld + col0) >> 2) & 3u);
-    const uint32_t V = n_cols + shift;
-    const int32_t id_off = (kSplit ? a.id_offset + (int32_t)col0 : a.id_offset) - (int32_t)shift;
-    const uint32_t scratch_cap = kSplit ? min(a.split_w, a.scratch_cap - col0) : a.scratch_cap;
+    uint32_t V = n_cols + shift;
+    int32_t id_off = (kSplit ? a.id_offset + (int32_t)col0 : a.id_offset) - (int32_t)shift;
+    uint32_t scratch_cap = kSplit ? n_cols : a.scratch_cap;
     const uint32_t n_tiles = (V + kTile - 1) / kTile;
     const float* __restrict__ lrow = a.logits + (size_t)row * a.ld + col0 - shift;
     // A speculative round (src/gen/session.cpp:451-506): row = sequence * n_pos + position. Position j < n_pos - 1
@@ -907,15 +929,15 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             hc[i] = (j < hlen) ? (uint32_t)hist_at(j) - (uint32_t)id_off : 0xffffffffu;
         }
     }
-    const RowCfg cfg = make_cfg(prm, n_cols, mode, a.vp_k, a.pass);
+    const RowCfg cfg = make_cfg(prm, a.n_vocab, mode, a.vp_k, a.pass);
     const uint32_t* __restrict__ mrow = a.mask ? a.mask + (size_t)row * a.mask_ld + (col0 >> 5) : nullptr;
     // Per-row scratch, 16 bytes per column: scratch_cap raw candidates (logit bits, column) — sorted in place as
     // 64-bit keys by the large sorted-list path — then as much again: the merge sort's second buffer, or (large
     // unsorted lists) one float per column.
-    uint32_t* const row_scratch = a.scratch + (size_t)row * row_scratch_words(a.scratch_cap) + 4ull * col0;
-    uint2* __restrict__ scratch = reinterpret_cast<uint2*>(row_scratch);
-    float* __restrict__ qrow = reinterpret_cast<float*>(row_scratch + 2u * scratch_cap);
-    uint32_t* const again = row_scratch + 4u * scratch_cap; // set by the first launch: this row wants the second pass
+    uint32_t* const row_scratch = a.scratch + (size_t)row * row_scratch_words(a.scratch_cap);
+    uint2* scratch = reinterpret_cast<uint2*>(row_scratch) + col0; // (a split row: this slice's share of the first half)
+    float* qrow = reinterpret_cast<float*>(row_scratch + 2u * (size_t)a.scratch_cap); // the half the list is not in
+    uint32_t* const again = row_scratch + 4u * (size_t)a.scratch_cap; // set by the first launch: this row wants the second pass
     if (spec && a.spec_forced) {
         const int32_t f = __ldg(a.spec_forced + row);
         if (f >= 0) { // the sampler is bypassed: the token is the forced one, a draft is kept only if it matches
@@ -933,8 +955,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     }
     if (a.pass == 1 && again[0] == 0u)
         return;
-    if (a.only_flagged && !(a.only_flagged[row] & a.only_flagged_mask))
-        return; // a follow-up launch for the rows an earlier step reported: the others are done
     // ---- shared-memory layout of the streaming phase ---------------------------------------------------------------
     const uint32_t bm_words = (V + 31u) / 32u;
     unsigned char* const dyn = smem_raw + kHeadBytes;
@@ -1418,22 +1438,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     // a chain of a dozen dependent shared loads and shuffle rounds); nobody waits for it. Counts only grow and every count is an element at or above its bin's edge, so a bound read from a
                     // histogram that other warps are still adding to has its k elements all the same.
                     if (t == 0 || (rwarp == (t % (kReaders / 32)) && (t < 8 || (t & 3u) == 0u))) {
-                        uint32_t cum = 0;
-                        int found = -1;
-                        for (int g = (int)*(volatile uint32_t*)&s.hi_group; g >= 0 && found < 0; --g) {
-                            const uint32_t cbin = ((volatile uint32_t*)hist)[g * 32 + lane];
-                            uint32_t suf = cbin; // suffix sum over lanes >= lane
-#pragma unroll
-                            for (int o = 1; o < 32; o <<= 1) {
-                                const uint32_t y = __shfl_down_sync(0xffffffffu, suf, o);
-                                if ((int)lane + o < 32)
-                                    suf += y;
-                            }
-                            const uint32_t hit = __ballot_sync(0xffffffffu, cum + suf >= cfg.hist_k);
-                            if (hit)
-                                found = g * 32 + (31 - __clz(hit));
-                            cum += __shfl_sync(0xffffffffu, suf, 0);
-                        }
+                        const int found = hist_scan(hist, *(volatile uint32_t*)&s.hi_group, cfg.hist_k);
                         // the lowest key of a bin is its smallest float; bin 0 (NaN keys) is never a bound
                         if (lane == 0 && found > 0)
                             atomicMax(&s.thr_topk_key, order_key(hist_bin_floor((uint32_t)found)));
@@ -1518,31 +1523,32 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // ---- finish -------------------------------------------------------------------------------------------------
     if (a.timing && tid == 0)
         a.timing[(size_t)row * 64 + 2] = global_ns();
-    if (s.abort_flag) {
-        // A bounded wait ran out. Give copies still in flight time to land before the CTA's shared memory is
-        // released, then report.
-        for (int i = 0; i < 64; ++i)
-            __nanosleep(1000);
+    auto timed_out = [&]() {
         if (tid == 0) {
             if (a.token) a.token[row] = -1;
             if (a.flags) a.flags[row] = MK_FLAG_TIMEOUT;
             if (a.n_cand) a.n_cand[row] = 0;
             if (a.accepted) a.accepted[row] = 0;
         }
-        return;
+    };
+    if (s.abort_flag) {
+        // A bounded wait ran out. Give copies still in flight time to land before the CTA's shared memory is
+        // released, then report.
+        for (int i = 0; i < 64; ++i)
+            __nanosleep(1000);
+        if (!kSplit) {
+            timed_out();
+            return;
+        }
     }
 
-    const bool any_finite = s.best_key != 0ull;
+    bool any_finite = s.best_key != 0ull;
     float m = any_finite ? key_to_float((uint32_t)(s.best_key >> 32)) : -__int_as_float(0x7f800000);
     uint32_t arg_col = any_finite ? (0xffffffffu - (uint32_t)(s.best_key & 0xffffffffull)) : shift;
     if (s.nan0) { // max_element keeps a NaN in front: every weight is NaN, the first column is returned
         m = __int_as_float(0x7fc00000);
         arg_col = shift;
     }
-    uint32_t flags = hlen_clamped ? MK_FLAG_HISTORY_FULL : 0u;
-    if (mrow && !any_finite && !s.nan0)
-        flags |= MK_FLAG_ALL_MASKED;
-
     // need_sum: weight of the uncollected tail (the whole row for a shard record), relative to the row maximum:
     // sum over reader threads of sum_acc * exp2((best - m) * c2), fixed order
     double total_approx = 0.0;
@@ -1569,6 +1575,132 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             total_approx += s.warp_sum[i];
         __syncthreads(); // warp_sum is written again below
     }
+
+    if constexpr (kSplit) {
+        // ---- the slices of the row meet ------------------------------------------------------------------------------
+        // Every CTA leaves its maximum, sum and the place of its list; the last one to arrive goes on with the row. Nobody
+        // waits for anybody.
+        const uint32_t n_slices = gridDim.y;
+        SplitPart* const parts = a.parts + (size_t)row * kMaxSlices;
+        __threadfence(); // this thread's kept elements, before the ticket
+        __syncthreads();
+        if (tid == 0) {
+            SplitPart p;
+            p.best_key = s.best_key ? s.best_key - col0 : 0ull; // places of the row instead of the slice's
+            p.sum = total_approx;
+            p.m = m;
+            p.n = min(s.ncand, scratch_cap);
+            p.bits = (s.nan0 && col0 == 0u ? 1u : 0u) | (s.abort_flag ? 2u : 0u);
+            p.unused = 0u;
+            parts[blockIdx.y] = p;
+            __threadfence();
+            const uint32_t ticket = atomicAdd(&a.tickets[row], 1u);
+            s.n_final = (ticket == n_slices - 1u) ? 1u : 0u;
+            if (s.n_final)
+                a.tickets[row] = 0u; // for the next launch
+        }
+        __syncthreads();
+        if (!s.n_final)
+            return;
+        __threadfence();
+        uint32_t* const n_of = reinterpret_cast<uint32_t*>(dyn + kOffFinOrd);
+        uint32_t* const hist2 = reinterpret_cast<uint32_t*>(dyn + kOffFinBitmap);
+        if (cfg.hist_mode)
+            for (uint32_t i = tid; i < (uint32_t)kBins; i += kThreads)
+                hist2[i] = 0u;
+        if (warp == 0) {
+            unsigned long long best_key = 0ull;
+            uint32_t bits = 0u;
+            for (uint32_t g = lane; g < n_slices; g += 32u) {
+                best_key = max(best_key, __ldcg(&parts[g].best_key));
+                bits |= __ldcg(&parts[g].bits);
+                n_of[g] = __ldcg(&parts[g].n);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                best_key = max(best_key, __shfl_xor_sync(0xffffffffu, best_key, o));
+            bits = __reduce_or_sync(0xffffffffu, bits);
+            const float mm = best_key ? key_to_float((uint32_t)(best_key >> 32)) : -__int_as_float(0x7f800000);
+            double sum = 0.0;
+            if (cfg.need_sum)
+                for (uint32_t g = lane; g < n_slices; g += 32u) {
+                    const double sg = __ldcg(&parts[g].sum);
+                    if (sg > 0.0)
+                        sum += sg * exp2((double)(__ldcg(&parts[g].m) - mm) * ((double)cfg.inv_t * 1.4426950408889634));
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0) {
+                s.best_key = best_key;
+                s.nan0 = bits & 1u;
+                s.abort_flag = bits & 2u;
+                s.warp_sum[0] = sum;
+                s.ncand = 0u;
+                s.hi_group = 0u;
+                s.thr_topk_key = order_key(-FLT_MAX);
+                s.n_final = 0u;
+                again[0] = 0u;
+            }
+        }
+        __syncthreads();
+        if (s.abort_flag) {
+            timed_out();
+            return;
+        }
+        n_cols = a.n_vocab;
+        V = n_cols + shift;
+        id_off = a.id_offset - (int32_t)shift;
+        scratch_cap = a.scratch_cap;
+        total_approx = s.warp_sum[0];
+        any_finite = s.best_key != 0ull;
+        m = any_finite ? key_to_float((uint32_t)(s.best_key >> 32)) : -__int_as_float(0x7f800000);
+        arg_col = any_finite ? (0xffffffffu - (uint32_t)(s.best_key & 0xffffffffull)) : shift;
+        if (s.nan0) {
+            m = __int_as_float(0x7fc00000);
+            arg_col = shift;
+        }
+        // One list of what the row's own bounds leave: the lists are sparse in the first half of the scratch, it goes to the
+        // second.
+        const uint2* const lists = reinterpret_cast<const uint2*>(row_scratch);
+        uint2* const merged = reinterpret_cast<uint2*>(row_scratch + 2u * (size_t)a.scratch_cap);
+        if (cfg.hist_mode) {
+            for (uint32_t g = warp; g < n_slices; g += kThreads / 32)
+                for (uint32_t i = lane; i < n_of[g]; i += 32u) {
+                    const uint32_t bin = hist_bin(__uint_as_float(__ldcg(&lists[g * a.split_w + i]).x));
+                    atomicAdd(&hist2[bin], 1u);
+                    atomicMax(&s.hi_group, bin >> 5);
+                }
+            __syncthreads();
+            if (warp == 0) {
+                const int found = hist_scan(hist2, s.hi_group, cfg.hist_k);
+                if (lane == 0 && found > 0)
+                    s.thr_topk_key = order_key(hist_bin_floor((uint32_t)found));
+            }
+            __syncthreads();
+        }
+        const float thr = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
+        for (uint32_t g = warp; g < n_slices; g += kThreads / 32)
+            for (uint32_t i0 = 0; i0 < n_of[g]; i0 += 32u) {
+                uint2 c = make_uint2(0xff800000u, 0u);
+                if (i0 + lane < n_of[g])
+                    c = __ldcg(&lists[g * a.split_w + i0 + lane]);
+                const bool in = __uint_as_float(c.x) >= thr;
+                const uint32_t bal = __ballot_sync(0xffffffffu, in);
+                uint32_t at = 0;
+                if (lane == 0 && bal)
+                    at = atomicAdd(&s.ncand, (uint32_t)__popc(bal));
+                at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+                if (in)
+                    merged[at] = make_uint2(c.x, c.y + g * a.split_w);
+            }
+        __syncthreads();
+        scratch = merged;
+        qrow = reinterpret_cast<float*>(row_scratch);
+    }
+    uint32_t flags = hlen_clamped ? MK_FLAG_HISTORY_FULL : 0u;
+    if (mrow && !any_finite && !s.nan0)
+        flags |= MK_FLAG_ALL_MASKED;
 
     // ---- the short finish: what nearly every row takes ---------------------------------------------------------
     // Few collected elements, at most 32 of them candidates, no row total beyond their own: one warp does it all in
@@ -1843,7 +1975,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         __syncthreads();
         block_sort(keys, n2);
         unsigned char* rec = reinterpret_cast<unsigned char*>(a.vp_records) +
-                             ((size_t)(kSplit ? blockIdx.y * gridDim.x : 0u) + row) * vp_record_bytes(a.vp_k);
+                             (size_t)row * vp_record_bytes(a.vp_k);
         const uint32_t n_out = min(n_raw, a.vp_k);
         if (tid == 0) {
             float* hf = reinterpret_cast<float*>(rec);
@@ -1970,18 +2102,18 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         return;
     }
     const unsigned long long* ksrc = keys; // the ordered list: shared memory, or the row's scratch for a long one
-    bool pre_sorted = false, list_in_front = true; // the half of the scratch that must not be written over
+    bool pre_sorted = false, over_raw = true; // which half of the scratch must not be written over
     if (!overflow && n > (uint32_t)kSortCap && mode != kModeDistOnly) {
         // More candidates than the shared-memory sort holds, and a truncation that orders them (the unordered case
         // returned above): a flat row under top_p, or a very large top_k. The candidates are sorted in global
         // memory — 8192-key runs in shared memory, then merge passes between the two halves of the row's scratch —
         // and the steps below read the list from there.
-        const unsigned long long* P = long_sort(s, keys, scratch, scratch_cap, n_raw, n,
+        const unsigned long long* P = long_sort(s, keys, scratch, qrow, n_raw, n,
                                                 fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key)), m, cfg.inv_t,
                                                 cfg.minp_eff);
         ksrc = P;
         pre_sorted = true;
-        list_in_front = reinterpret_cast<const uint32_t*>(P) == row_scratch;
+        over_raw = reinterpret_cast<const void*>(P) == reinterpret_cast<const void*>(scratch);
         // The float total and the walk below are sequential chains that take 32 candidates per step: fed from global
         // memory they run at the pace of its latency, so a list that fits is staged in shared memory first.
         if (n <= kOffChain / 8u) {
@@ -2110,7 +2242,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         // the weights in order go behind the keys where there is room, else to the half of the scratch the list is not in
         float* q_dense = reinterpret_cast<float*>(dyn + kOffKeys + (((size_t)s.nsurv * 8u + 15u) & ~(size_t)15u));
         if (pre_sorted || (size_t)s.nsurv * 8u + 16u + (size_t)n * 4u > kOffFinBitmap)
-            q_dense = list_in_front ? qrow : reinterpret_cast<float*>(row_scratch);
+            q_dense = over_raw ? qrow : reinterpret_cast<float*>(scratch);
         draw_list(s, *reinterpret_cast<RowChain*>(dyn + kOffChain), ksrc, ord, sorted ? kByWeight : (by_rank ? kByRank : kByColumn),
                   q_dense, n, row, flags, u_row, u2_row, draft_row, o);
     } else
@@ -2345,11 +2477,12 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     RowKernelArgs first = a;
     first.pass = 0;
     const bool spec = a.spec_n_pos != 0u;
-    if (a.split_w != 0u) { // shard records of every row, one CTA per (row, column shard)
+    if (a.split_w != 0u) { // one CTA per (row, slice)
         lc.gridDim = dim3(batch, (a.n_vocab + a.split_w - 1u) / a.split_w);
-        return cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, true>, first);
-    }
-    e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, first)
+        e = cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, true>, first);
+        lc.gridDim = dim3(batch);
+    } else
+        e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, first)
              : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false>, first);
     if (e != cudaSuccess)
         return e;
@@ -2368,6 +2501,7 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
         }
         RowKernelArgs second = a; // what is left
         second.pass = 1;
+        second.split_w = 0;
         e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, second)
                  : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false>, second);
     }

@@ -15,6 +15,17 @@ enum RowMode : int {
     kModeVpLocal = 3   // vocab-parallel shard record
 };
 
+// What one CTA of a split row leaves for the last of them.
+struct SplitPart {
+    unsigned long long best_key; // (order key of the slice's maximum << 32) | ~place; 0: nothing finite
+    double sum;                  // top_p alone: streamed weights relative to the slice's maximum
+    float m;
+    uint32_t n;                  // elements kept, in the slice's share of the row's list
+    uint32_t bits;               // 1: the row's first column is NaN, 2: a wait ran out
+    uint32_t unused;
+};
+constexpr uint32_t kMaxSlices = 64, kSplitMaxRows = 64;
+
 struct RowKernelArgs {
     // inputs
     const float* logits;
@@ -58,12 +69,11 @@ struct RowKernelArgs {
     uint32_t spec_n_pos;
     const int32_t* spec_drafts; // [n_seq][spec_n_pos - 1]
     const int32_t* spec_forced; // [n_seq][spec_n_pos] forced token or -1, or NULL
-    // split launch (shard records only): every row's columns in shards of split_w columns, one CTA per (row, shard);
-    // records laid out [n_shards][batch]. 0: off
+    // split launch: every row's columns in slices of split_w columns, one CTA per (row, slice); the last CTA of a row to arrive
+    // (tickets: zero between launches) draws from what all of them kept. 0: off
     uint32_t split_w;
-    // follow-up launch: only rows whose flags (written by an earlier step) have one of these bits set are processed
-    const uint32_t* only_flagged;
-    uint32_t only_flagged_mask;
+    SplitPart* parts;  // [batch][kMaxSlices]
+    uint32_t* tickets; // [batch]
     uint32_t debug_skip_tile;   // test hook: the copy of this tile is never requested (0xffffffff: none)
     uint32_t debug_wait_probes; // test hook: probes a wait for a tile makes before it gives up (0: the default)
 };
