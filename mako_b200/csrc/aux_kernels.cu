@@ -11,29 +11,32 @@ namespace mk {
 
 namespace {
 
-constexpr int kMergeThreads = 128;    // a CTA per row of a large batch
-constexpr int kMergeThreadsFew = 512; // a handful of rows: the sort is what takes the time, so more threads on it
+constexpr int kMergeThreads = 256;    // a CTA per row of a large batch: eight on an SM, more than 1024 rows at once
+constexpr int kMergeThreadsFew = 512; // a handful of rows
 constexpr int kMergeCap = 2048; // n_shards * k
 constexpr uint32_t kShardShift = 26, kIdMask = (1u << kShardShift) - 1u; // sort keys: shard above the token id
 
+// Bitonic sort of n2 (power of two) keys in shared memory by n_threads threads, a pair of keys a thread and trip. Pairs less than
+// 64 keys apart stay within a warp's own 64 keys, so those steps need no barrier of the CTA (512 keys: 6 of 45 do).
 __device__ void sort_keys(unsigned long long* keys, uint32_t n2, uint32_t n_threads)
 {
     for (uint32_t k = 2; k <= n2; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < n2; i += n_threads) {
-                const uint32_t l = i ^ j;
-                if (l > i) {
-                    const unsigned long long a = keys[i], b = keys[l];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        keys[i] = b;
-                        keys[l] = a;
-                    }
+            for (uint32_t c = threadIdx.x; c < (n2 >> 1); c += n_threads) {
+                const uint32_t i = ((c & ~(j - 1u)) << 1) | (c & (j - 1u)), l = i | j;
+                const unsigned long long a = keys[i], b = keys[l];
+                if ((a > b) == ((i & k) == 0)) {
+                    keys[i] = b;
+                    keys[l] = a;
                 }
             }
-            __syncthreads();
+            if (j > 32u || (j == 1u && k >= 64u))
+                __syncthreads();
+            else
+                __syncwarp();
         }
     }
+    __syncthreads();
 }
 
 } // namespace
@@ -95,6 +98,9 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
         arg_id = 0;
         arg_shard = 0;
     }
+    __shared__ unsigned long long s_exp2[32]; // expf_host_exact's table: constant memory serves a lane at a time
+    if (tid < 32)
+        s_exp2[tid] = kExp2Tab[tid];
     if (tid == 0) {
         s_n = 0;
         s_nfinal = 0;
@@ -127,7 +133,7 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
                 continue;
             const uint2 c = reinterpret_cast<const uint2*>(rec(g) + kVpHeaderBytes)[i];
             const float x = __fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t);
-            const float q = expf_host_exact(x);
+            const float q = expf_host_exact(x, s_exp2);
             if (q >= minp_eff && q > 0.0f) {
                 const uint32_t slot = atomicAdd(&s_n, 1u);
                 keys[slot] = ((unsigned long long)__float_as_uint(q) << 32) | (g << kShardShift) | c.y;
@@ -181,7 +187,7 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
         if (cut_k)
             n = prm.top_k;
         if (use_topp) {
-            double total = 0.0, band;
+            double total = 0.0, band = 0.0;
             if (need_sum && !(flags & MK_FLAG_NO_CANDIDATE)) {
                 const double c2 = (double)inv_t * 1.4426950408889634;
                 for (uint32_t g0 = 0; g0 < a.n_shards; g0 += 32u) { // the shards' rescaled sums, added in shard order
@@ -194,31 +200,45 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
                         total += __shfl_sync(full, term, j);
                 }
                 band = 1e-5 * total;
-            } else {
-                for (uint32_t base = 0; base < n; base += 32u) {
-                    const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-                    const int cnt = (int)min(32u, n - base);
-                    for (int j = 0; j < cnt; ++j)
-                        total += (double)__shfl_sync(full, q, j);
-                }
+            }
+            // prefix sums in double, a run of candidates a lane (their rounding is far inside `band`)
+            const uint32_t len = (n + 31u) / 32u, r0 = min(lane * len, n), r1 = min(r0 + len, n);
+            double mine = 0.0;
+            for (uint32_t i = r0; i < r1; ++i)
+                mine += (double)q_at(i);
+            double inc = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double y = __shfl_up_sync(full, inc, o);
+                if ((int)lane >= o)
+                    inc += y;
+            }
+            const double list_total = __shfl_sync(full, inc, 31);
+            if (!(need_sum && !(flags & MK_FLAG_NO_CANDIDATE))) {
+                total = list_total;
                 band = 0x1p-40 * total;
             }
             const double want = (double)prm.top_p * total;
-            double run = 0.0, prev = 0.0;
-            uint32_t k = 0;
-            bool open = true;
-            for (uint32_t base = 0; base < n && open; base += 32u) {
-                const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-                const int cnt = (int)min(32u, n - base);
-                for (int j = 0; j < cnt; ++j) {
-                    const double qj = (double)__shfl_sync(full, q, j);
-                    open = open && run < want;
-                    if (open) {
-                        prev = run;
-                        run += qj;
-                        k = base + (uint32_t)j + 1u;
-                    }
+            double run = inc - mine, prev = run;
+            uint32_t k = 0xffffffffu; // candidates taken: the first count whose sum is not below `want`
+            for (uint32_t i = r0; i < r1; ++i) {
+                prev = run;
+                run += (double)q_at(i);
+                if (!(run < want)) {
+                    k = i + 1u;
+                    break;
                 }
+            }
+            const uint32_t k_all = __reduce_min_sync(full, k);
+            if (k_all != 0xffffffffu) {
+                const int owner = __ffs((int)__ballot_sync(full, k == k_all)) - 1;
+                run = __shfl_sync(full, run, owner);
+                prev = __shfl_sync(full, prev, owner);
+                k = k_all;
+            } else { // the list ends first
+                run = list_total;
+                prev = list_total - (double)q_at(n - 1u);
+                k = n;
             }
             if (need_sum && run < want)
                 flags |= MK_FLAG_VP_TRUNCATED;
@@ -245,34 +265,40 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
         }
         if (__any_sync(full, cut_short))
             flags |= MK_FLAG_VP_TRUNCATED;
+        // 32 candidates a step, lanes past the end of the list holding zeros (which change nothing and never win): the
+        // shuffles do not depend on the chains, which then run at the adder's latency
         float total = 0.0f;
         for (uint32_t base = 0; base < n; base += 32u) {
             const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-            const int cnt = (int)min(32u, n - base);
-            for (int j = 0; j < cnt; ++j)
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
                 total = __fadd_rn(total, __shfl_sync(full, q, j));
         }
         float r = __fmul_rn(a.u[row], total);
         const float eps = 1e-6f * total;
         uint32_t hit = n - 1u;
         float q_hit = q_at(n - 1u);
-        bool found = false;
-        for (uint32_t base = 0; base < n && !found; base += 32u) {
+        for (uint32_t base = 0; base < n; base += 32u) {
             const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-            const int cnt = (int)min(32u, n - base);
-            for (int j = 0; j < cnt && !found; ++j) {
+            uint32_t short_of = 0u;
+            float rr = r;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
                 const float qj = __shfl_sync(full, q, j);
-                const uint32_t i = base + (uint32_t)j;
-                if (r < qj) {
-                    found = true;
-                    hit = i;
-                    q_hit = qj;
-                    if ((i > 0 && r < eps) || (i + 1 < n && __fsub_rn(qj, r) < eps))
-                        flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
-                } else {
-                    r = __fsub_rn(r, qj);
-                }
+                short_of |= (rr < qj) ? (1u << j) : 0u;
+                rr = __fsub_rn(rr, qj);
             }
+            if (short_of) { // the first candidate the draw falls short of; the remainder in front of it, once more
+                const int jh = __ffs((int)short_of) - 1;
+                for (int j = 0; j < jh; ++j)
+                    r = __fsub_rn(r, __shfl_sync(full, q, j));
+                hit = base + (uint32_t)jh;
+                q_hit = __shfl_sync(full, q, jh);
+                if ((hit > 0 && r < eps) || (hit + 1 < n && __fsub_rn(q_hit, r) < eps))
+                    flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
+                break;
+            }
+            r = rr;
         }
         if (lane == 0) {
             if (a.token) a.token[row] = (int32_t)(tag_at(hit) & kIdMask);
