@@ -1807,7 +1807,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         fl |= MK_FLAG_GUARD_BAND;
                     n = cfg.top_k;
                 }
-                if (cfg.use_topp) { // sampler.cpp:44-61, sequentially
+                if (cfg.use_topp) { // sampler.cpp:44-61, the sums as a scan: it rounds far inside `band`
+                    double inc = (double)q;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const double y = __shfl_up_sync(full, inc, o);
+                        if ((int)lane >= o)
+                            inc += y;
+                    }
                     double total_d = 0.0, band;
                     // top_p alone: the total covers every column — exact weights of what was kept, and of the streamed
                     // sum what lies beside them — and carries the margin of the approximate part and, where the kept
@@ -1823,20 +1830,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         total_d = sum_kept + rest;
                         band = 1e-5 * rest + (cfg.optimistic ? 2e-6 * sum_kept : 0x1p-40 * total_d);
                     } else {
-                        for (uint32_t j = 0; j < n; ++j)
-                            total_d += (double)__shfl_sync(full, q, (int)j);
+                        total_d = __shfl_sync(full, inc, (int)n - 1);
                         band = 0x1p-40 * total_d;
                     }
                     const double want = (double)cfg.top_p * total_d;
-                    double run = 0.0, prev = 0.0;
-                    uint32_t k = 0;
-                    for (uint32_t j = 0; j < n && run < want; ++j) {
-                        prev = run;
-                        run += (double)__shfl_sync(full, q, (int)j);
-                        k = j + 1u;
-                    }
-                    if ((row_total && run < want) ||
-                        (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))) {
+                    const uint32_t reached = __ballot_sync(full, lane < n && !(inc < want));
+                    const uint32_t k = reached ? (uint32_t)__ffs((int)reached) : n; // candidates taken
+                    const double run = __shfl_sync(full, inc, (int)k - 1), prev = __shfl_sync(full, inc, max((int)k - 2, 0));
+                    if ((row_total && run < want) || fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)) {
                         if (cfg.optimistic) {
                             retry = true; // what was kept does not settle the nucleus: the second pass will
                             if (lane == 0) {
@@ -1847,13 +1848,15 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             fl |= MK_FLAG_GUARD_BAND;
                         }
                     }
-                    n = max(k, 1u);
+                    n = k;
                 }
                 if (lane >= n)
                     q = 0.0f;
-                float total = 0.0f;
-                for (uint32_t j = 0; j < n; ++j)
-                    total = __fadd_rn(total, __shfl_sync(full, q, (int)j));
+                float total = 0.0f; // eight at a time: the shuffles do not wait for the sum, zeros change nothing
+                for (uint32_t base = 0; base < n; base += 8u)
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; ++j)
+                        total = __fadd_rn(total, __shfl_sync(full, q, (int)(base + j)));
                 const int32_t draft = (mode == kModeVerify) ? draft_row : -1;
                 const uint32_t dm = __ballot_sync(full, draft >= 0 && lane < n && (int32_t)col + id_off == draft);
                 const uint32_t draft_idx = dm ? (uint32_t)__ffs((int)dm) - 1u : 0xffffffffu;
@@ -1888,19 +1891,26 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         const float qw = (lane == skip_idx) ? 0.0f : q; // the skipped draft never wins
                         uint32_t hit = last_valid; // rounding: the last candidate (sampler.cpp:72)
                         float q_hit = __shfl_sync(full, qw, (int)last_valid);
-                        bool found = false;
-                        for (uint32_t j = 0; j < n && !found; ++j) {
-                            const float qj = __shfl_sync(full, qw, (int)j);
-                            if (r < qj) {
-                                found = true;
-                                hit = j;
-                                q_hit = qj;
-                                // boundary below (not for the first candidate) or above (not for the last)
-                                if ((j != first_valid && r < eps) || (j < last_valid && __fsub_rn(qj, r) < eps))
-                                    fl |= MK_FLAG_NEAR_CDF_BOUNDARY;
-                            } else {
-                                r = __fsub_rn(r, qj);
+                        for (uint32_t base = 0; base < n; base += 8u) {
+                            uint32_t short_of = 0u; // the candidates the draw falls short of, if all before are passed
+                            float rr = r;
+#pragma unroll
+                            for (uint32_t j = 0; j < 8u; ++j) {
+                                const float qj = __shfl_sync(full, qw, (int)(base + j));
+                                short_of |= (rr < qj) ? 1u << j : 0u;
+                                rr = __fsub_rn(rr, qj);
                             }
+                            if (short_of) {
+                                hit = base + (uint32_t)__ffs((int)short_of) - 1u;
+                                for (uint32_t j = base; j < hit; ++j)
+                                    r = __fsub_rn(r, __shfl_sync(full, qw, (int)j));
+                                q_hit = __shfl_sync(full, qw, (int)hit);
+                                // boundary below (not for the first candidate) or above (not for the last)
+                                if ((hit != first_valid && r < eps) || (hit < last_valid && __fsub_rn(q_hit, r) < eps))
+                                    fl |= MK_FLAG_NEAR_CDF_BOUNDARY;
+                                break;
+                            }
+                            r = rr;
                         }
                         tok = (int32_t)__shfl_sync(full, col, (int)hit) + id_off;
                         prob = __fdiv_rn(q_hit, walk_total);
@@ -2010,6 +2020,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 o.y = (uint32_t)((int32_t)(uint32_t)(key & 0xffffffffull) + id_off);
             }
             reinterpret_cast<uint2*>(rec + kVpHeaderBytes)[i] = o;
+        }
+        if (a.timing && tid == 0) {
+            a.timing[(size_t)row * 64 + 9] = n_all;
+            a.timing[(size_t)row * 64 + 10] = n_raw;
+            a.timing[(size_t)row * 64 + 3] = global_ns();
         }
         return;
     }
