@@ -49,6 +49,7 @@ constexpr uint32_t kPlaces = 296; // CTAs of the row kernel that are resident at
 struct mk_sampler {
     int device = 0;
     uint32_t n_vocab = 0, max_batch = 0;
+    unsigned char* block = nullptr; // the one allocation the arrays below lie in (all but the host-buffer staging)
     uint32_t* scratch = nullptr; // [max_batch][4*n_vocab] words: raw candidates (a row can never overflow it) + sort buffer / a float per column
     uint32_t* scratch_pq = nullptr; // the same again: p/q verification runs its two row sets side by side
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -80,7 +81,9 @@ struct DeviceGuard {
     {
         if (cudaGetDevice(&prev) != cudaSuccess)
             ok = false;
-        else if (prev != dev && cudaSetDevice(dev) != cudaSuccess)
+        else if (prev == dev)
+            prev = -1; // nothing to go back to
+        else if (cudaSetDevice(dev) != cudaSuccess)
             ok = false;
     }
     ~DeviceGuard()
@@ -243,45 +246,56 @@ int mk_sampler_create(mk_sampler** out, int device, uint32_t n_vocab, uint32_t m
     DeviceGuard g(device);
     if (!g.ok)
         return fail(MK_ERR_CUDA, "cannot select device %d", device);
-    cudaDeviceProp prop;
-    MK_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major < 10)
-        return fail(MK_ERR_UNSUPPORTED, "device %d is sm_%d%d; the kernels are built for sm_100a only", device,
-                    prop.major, prop.minor);
+    int major = 0, minor = 0; // (not cudaGetDeviceProperties: it takes longer than everything else here)
+    MK_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    MK_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major < 10)
+        return fail(MK_ERR_UNSUPPORTED, "device %d is sm_%d%d; the kernels are built for sm_100a only", device, major, minor);
     mk_sampler* s = new (std::nothrow) mk_sampler();
     if (!s)
         return fail(MK_ERR_INVALID_ARGUMENT, "out of host memory");
     s->device = device;
     s->n_vocab = n_vocab;
     s->max_batch = max_batch;
-    const size_t b = max_batch;
-    cudaError_t e = cudaSuccess;
-    auto alloc = [&](void** p, size_t bytes) {
-        if (e == cudaSuccess)
-            e = cudaMalloc(p, bytes);
-    };
-    alloc((void**)&s->scratch, b * mk::row_scratch_words(scratch_cap(n_vocab)) * 4);
-    alloc((void**)&s->scratch_pq, b * mk::row_scratch_words(scratch_cap(n_vocab)) * 4);
-    alloc((void**)&s->p_ids, b * kPqCap * 4);
-    alloc((void**)&s->q_ids, b * kPqCap * 4);
-    alloc((void**)&s->p_q, b * kPqCap * 4);
-    alloc((void**)&s->q_q, b * kPqCap * 4);
-    alloc((void**)&s->p_total, b * 4);
-    alloc((void**)&s->q_total, b * 4);
-    alloc((void**)&s->q_prob, b * 4);
-    alloc((void**)&s->p_n, b * 4);
-    alloc((void**)&s->q_n, b * 4);
-    alloc((void**)&s->p_flags, b * 4);
-    alloc((void**)&s->q_flags, b * 4);
-    alloc((void**)&s->p_tok, b * 4);
-    alloc((void**)&s->pick_best, (mk::kDraftPickMaxSeq + 1) * sizeof(unsigned long long)); // maxima + ticket counter
+    // One allocation, shared out: as one for each array they were most of what creating a handle takes.
+    const size_t b = max_batch, row_bytes = mk::row_scratch_words(scratch_cap(n_vocab)) * 4;
     const size_t split_rows_max = 2u * (size_t)mk::kSplitMaxRows;
-    alloc((void**)&s->split_parts, split_rows_max * mk::kMaxSlices * sizeof(mk::SplitPart));
-    alloc((void**)&s->split_tickets, split_rows_max * 4);
-    if (e == cudaSuccess)
-        e = cudaMemset(s->split_tickets, 0, split_rows_max * 4);
-    if (e == cudaSuccess)
-        e = cudaMemset(s->pick_best, 0, (mk::kDraftPickMaxSeq + 1) * sizeof(unsigned long long));
+    const size_t zero_bytes = (mk::kDraftPickMaxSeq + 1) * sizeof(unsigned long long) + split_rows_max * 4;
+    struct Share {
+        void** to;
+        size_t bytes;
+    } const shares[] = {
+        {(void**)&s->pick_best, zero_bytes}, // maxima and ticket counter of the drafter picks, then the split rows' tickets
+        {(void**)&s->split_parts, split_rows_max * mk::kMaxSlices * sizeof(mk::SplitPart)},
+        {(void**)&s->scratch, b * row_bytes},
+        {(void**)&s->scratch_pq, b * row_bytes},
+        {(void**)&s->p_ids, b * kPqCap * 4},
+        {(void**)&s->q_ids, b * kPqCap * 4},
+        {(void**)&s->p_q, b * kPqCap * 4},
+        {(void**)&s->q_q, b * kPqCap * 4},
+        {(void**)&s->p_total, b * 4},
+        {(void**)&s->q_total, b * 4},
+        {(void**)&s->q_prob, b * 4},
+        {(void**)&s->p_n, b * 4},
+        {(void**)&s->q_n, b * 4},
+        {(void**)&s->p_flags, b * 4},
+        {(void**)&s->q_flags, b * 4},
+        {(void**)&s->p_tok, b * 4},
+    };
+    auto up = [](size_t x) { return (x + 255u) & ~(size_t)255u; };
+    size_t bytes = 0;
+    for (const Share& x : shares)
+        bytes += up(x.bytes);
+    cudaError_t e = cudaMalloc((void**)&s->block, bytes);
+    if (e == cudaSuccess) {
+        unsigned char* at = s->block;
+        for (const Share& x : shares) {
+            *x.to = at;
+            at += up(x.bytes);
+        }
+        s->split_tickets = reinterpret_cast<uint32_t*>(s->pick_best + mk::kDraftPickMaxSeq + 1);
+        e = cudaMemset(s->pick_best, 0, zero_bytes);
+    }
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess)
@@ -301,12 +315,10 @@ void mk_sampler_destroy(mk_sampler* s)
     if (!s)
         return;
     DeviceGuard g(s->device);
-    void* ptrs[] = {s->scratch, s->p_ids, s->q_ids, s->p_q, s->q_q, s->p_total, s->q_total, s->q_prob,
-                    s->p_n,     s->q_n,   s->p_flags, s->q_flags, s->p_tok, s->stage, s->pick_best,
-                    s->split_parts, s->split_tickets, s->scratch_pq};
-    for (void* p : ptrs)
-        if (p)
-            cudaFree(p);
+    if (s->block)
+        cudaFree(s->block);
+    if (s->stage)
+        cudaFree(s->stage);
     if (s->ev_fork)
         cudaEventDestroy(s->ev_fork);
     if (s->ev_join)

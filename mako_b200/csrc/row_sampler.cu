@@ -6,6 +6,7 @@
 #include "row_pipeline.h"
 
 #include <limits>
+#include <mutex>
 #include <new>
 #include <random>
 #include <vector>
@@ -22,12 +23,75 @@ struct mk_row_sampler {
     int32_t* d_history = nullptr;
     size_t d_history_cap = 0;
     float* d_row = nullptr;     // staging for a host logits row
-    float* d_u = nullptr;       // [2]
-    int32_t* d_io = nullptr;    // [0] token, [1] accepted, [2] draft
+    // What a call hands the kernel and gets back, in pinned host memory the device reads and writes in place: the uniforms and the
+    // draft are read while the row streams, the result is there when the stream is. (As copies of their own around the
+    // launch they were most of a call: sample() of one row of 151552 columns 44 us, 37 us so.)
+    struct alignas(64) Io {
+        float u[2];
+        int32_t token, accepted, draft;
+    };
+    Io* io = nullptr;
     cudaStream_t stream = nullptr;
 };
 
 namespace {
+
+// The handle's device for the length of a call; nothing is set where it is current already.
+struct OnDevice {
+    int prev = -1;
+    explicit OnDevice(int device)
+    {
+        int now = -1;
+        if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess)
+            prev = now;
+    }
+    ~OnDevice()
+    {
+        if (prev >= 0)
+            cudaSetDevice(prev);
+    }
+};
+
+// Pinned memory is slow to get (2 ms and more, as long as the rest of a sampler takes), so the handles of a process share one
+// page of it: 64 places, taken and given back under a lock, allocated by the first handle and freed with the last. More handles
+// than places get one of their own.
+constexpr int kIoPlaces = 64;
+std::mutex g_io_lock;
+mk_row_sampler::Io* g_io_page = nullptr;
+uint64_t g_io_taken = 0;
+
+mk_row_sampler::Io* io_alloc(size_t n)
+{
+    void* p = nullptr;
+    return cudaHostAlloc(&p, n * sizeof(mk_row_sampler::Io), cudaHostAllocPortable) == cudaSuccess ? static_cast<mk_row_sampler::Io*>(p)
+                                                                                                  : nullptr;
+}
+
+mk_row_sampler::Io* io_take()
+{
+    std::lock_guard<std::mutex> hold(g_io_lock);
+    if (!g_io_page)
+        g_io_page = io_alloc(kIoPlaces);
+    if (!g_io_page || g_io_taken == ~0ull)
+        return io_alloc(1);
+    const int i = __builtin_ctzll(~g_io_taken);
+    g_io_taken |= 1ull << i;
+    return g_io_page + i;
+}
+
+void io_give(mk_row_sampler::Io* io)
+{
+    std::lock_guard<std::mutex> hold(g_io_lock);
+    if (!g_io_page || io < g_io_page || io >= g_io_page + kIoPlaces) {
+        cudaFreeHost(io);
+        return;
+    }
+    g_io_taken &= ~(1ull << (io - g_io_page));
+    if (g_io_taken == 0) {
+        cudaFreeHost(g_io_page);
+        g_io_page = nullptr;
+    }
+}
 
 float next_uniform(std::mt19937_64& g)
 {
@@ -107,7 +171,7 @@ int mk_row_sampler_create(mk_row_sampler** out, const mk_sampling_params* p, uin
     cudaGetDevice(&prev);
     cudaSetDevice(device);
     bool ok = cudaMalloc((void**)&r->d_row, (size_t)n_vocab * 4) == cudaSuccess &&
-              cudaMalloc((void**)&r->d_u, 8) == cudaSuccess && cudaMalloc((void**)&r->d_io, 12) == cudaSuccess &&
+              (r->io = io_take()) != nullptr &&
               cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking) == cudaSuccess;
     cudaSetDevice(prev);
     if (!ok) {
@@ -127,8 +191,7 @@ void mk_row_sampler_destroy(mk_row_sampler* r)
     cudaSetDevice(r->device);
     if (r->d_history) cudaFree(r->d_history);
     if (r->d_row) cudaFree(r->d_row);
-    if (r->d_u) cudaFree(r->d_u);
-    if (r->d_io) cudaFree(r->d_io);
+    if (r->io) io_give(r->io);
     if (r->stream) cudaStreamDestroy(r->stream);
     cudaSetDevice(prev);
     mk_sampler_destroy(r->core);
@@ -165,26 +228,18 @@ int mk_row_sampler_sample(mk_row_sampler* r, const float* logits, int32_t* token
 {
     if (!r || !logits || !token)
         return MK_ERR_INVALID_ARGUMENT;
-    int prev = 0;
-    cudaGetDevice(&prev);
-    cudaSetDevice(r->device);
-    const bool greedy = mk_row_sampler_greedy(r);
-    float u[2] = {0.0f, 0.0f};
-    if (!greedy) { // greedy draws nothing from the generator
-        u[0] = next_uniform(r->rng);
-        cudaMemcpyAsync(r->d_u, u, 4, cudaMemcpyHostToDevice, r->stream);
-    }
+    OnDevice here(r->device);
+    if (!mk_row_sampler_greedy(r)) // greedy draws nothing from the generator
+        r->io->u[0] = next_uniform(r->rng);
     mk_rows rows;
     fill_rows(r, device_row(r, logits), rows);
     mk_sample_out out{};
-    out.token = r->d_io;
-    int rc = mk_sampler_sample_batch(r->core, &rows, r->d_u, &out, r->stream);
-    if (rc == MK_OK) {
-        if (cudaMemcpyAsync(token, r->d_io, 4, cudaMemcpyDeviceToHost, r->stream) != cudaSuccess ||
-            cudaStreamSynchronize(r->stream) != cudaSuccess)
-            rc = MK_ERR_CUDA;
-    }
-    cudaSetDevice(prev);
+    out.token = &r->io->token;
+    int rc = mk_sampler_sample_batch(r->core, &rows, r->io->u, &out, r->stream);
+    if (rc == MK_OK && cudaStreamSynchronize(r->stream) != cudaSuccess)
+        rc = MK_ERR_CUDA;
+    if (rc == MK_OK)
+        *token = *(volatile int32_t*)&r->io->token;
     return rc;
 }
 
@@ -193,37 +248,28 @@ int mk_row_sampler_verify(mk_row_sampler* r, const float* logits, int32_t draft,
 {
     if (!r || !logits || !token || !accepted)
         return MK_ERR_INVALID_ARGUMENT;
-    int prev = 0;
-    cudaGetDevice(&prev);
-    cudaSetDevice(r->device);
+    OnDevice here(r->device);
     const bool greedy = mk_row_sampler_greedy(r);
-    float u[2] = {0.0f, 0.0f};
     std::mt19937_64 after_first = r->rng;
     if (!greedy) {
-        u[0] = next_uniform(r->rng);
+        r->io->u[0] = next_uniform(r->rng);
         after_first = r->rng;
-        u[1] = next_uniform(r->rng);
-        cudaMemcpyAsync(r->d_u, u, 8, cudaMemcpyHostToDevice, r->stream);
+        r->io->u[1] = next_uniform(r->rng);
     }
-    int32_t io[3] = {0, 0, draft};
-    cudaMemcpyAsync(r->d_io + 2, &io[2], 4, cudaMemcpyHostToDevice, r->stream);
+    r->io->draft = draft;
     mk_rows rows;
     fill_rows(r, device_row(r, logits), rows);
     mk_sample_out out{};
-    out.token = r->d_io;
-    int rc = mk_sampler_verify_batch(r->core, &rows, r->d_io + 2, r->d_u, r->d_u + 1, &out, r->d_io + 1, r->stream);
+    out.token = &r->io->token;
+    int rc = mk_sampler_verify_batch(r->core, &rows, &r->io->draft, r->io->u, r->io->u + 1, &out, &r->io->accepted, r->stream);
+    if (rc == MK_OK && cudaStreamSynchronize(r->stream) != cudaSuccess)
+        rc = MK_ERR_CUDA;
     if (rc == MK_OK) {
-        if (cudaMemcpyAsync(io, r->d_io, 8, cudaMemcpyDeviceToHost, r->stream) != cudaSuccess ||
-            cudaStreamSynchronize(r->stream) != cudaSuccess)
-            rc = MK_ERR_CUDA;
-    }
-    if (rc == MK_OK) {
-        *token = io[0];
-        *accepted = io[1];
-        if (!greedy && io[1])
+        *token = *(volatile int32_t*)&r->io->token;
+        *accepted = *(volatile int32_t*)&r->io->accepted;
+        if (!greedy && *accepted)
             r->rng = after_first; // the second draw was not consumed
     }
-    cudaSetDevice(prev);
     return rc;
 }
 

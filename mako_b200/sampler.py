@@ -31,7 +31,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 class Sampler:
@@ -106,6 +106,7 @@ class BatchSampler:
         check(lib.mk_sampler_create(C.byref(self._h), device, n_vocab, max_batch))
         self.n_vocab, self.max_batch, self.cand_cap = n_vocab, max_batch, cand_cap
         d = self.device
+        self._views = (-1, ())
         self.token = torch.empty(max_batch, dtype=torch.int32, device=d)
         self.prob = torch.empty(max_batch, dtype=torch.float32, device=d)
         self.flags = torch.zeros(max_batch, dtype=torch.int32, device=d)
@@ -180,9 +181,10 @@ class BatchSampler:
         return o
 
     def _result(self, b: int, **kw) -> SampleResult:
-        return SampleResult(self.token[:b], self.prob[:b], self.flags[:b], self.n_cand[:b],
-                            self.cand_ids[:b] if self.cand_cap else None,
-                            self.cand_q[:b] if self.cand_cap else None, **kw)
+        if self._views[0] != b:  # the outputs' first rows: slicing them anew was a quarter of a call's host time
+            self._views = (b, (self.token[:b], self.prob[:b], self.flags[:b], self.n_cand[:b],
+                               self.cand_ids[:b] if self.cand_cap else None, self.cand_q[:b] if self.cand_cap else None))
+        return SampleResult(*self._views[1], **kw)
 
     # -- the operations -----------------------------------------------------------------------------------------
     def sample(self, logits, params, u=None, *, history=None, history_len=None, mask=None, bias=None) -> SampleResult:
