@@ -128,7 +128,7 @@ int mk_check_sampling(const mk_sampling_params* p);
 #define MK_OVERLAP_STABLE_SIDE_INPUTS 2
 int mk_sampler_set_overlap(mk_sampler* s, int mode);
 
-/* No counterpart in the reference. A sample, verify or p/q verify call of at most 64 rows leaves the device idle as one CTA
+/* No counterpart in the reference. A sample, verify or p/q verify call of at most 148 rows leaves the device idle as one CTA
  * per row, so by default every row's columns are split over up to 64 CTAs where that is faster (long rows, or a top_k or
  * top_p bound); the last of a row's CTAs to arrive draws from what all of them kept. Same tokens, probabilities and
  * candidate lists as the plain path. on = 0 makes every batch run as one CTA per row. */

@@ -21,6 +21,8 @@ namespace mk {
 
 constexpr uint32_t kRun = 8;            // candidates a thread and round
 constexpr uint32_t kUnitCap = 1u << 25; // increments are clamped here: past the binade's end whatever they are
+constexpr uint32_t kHead = 64;          // the first candidates of a total
+constexpr uint32_t kBeside = 32;        // candidates taken element by element at a crossing
 constexpr uint32_t kCleanRounds = 4;    // rounds of one warp without a crossing before the CTA takes over
 constexpr float kChainFloor = 0x1p-100f; // smaller running values are taken element by element: their unit would be a denormal
 
@@ -58,6 +60,19 @@ __device__ __forceinline__ void warp_compose(uint32_t& f0, uint32_t& f1)
     }
 }
 
+// The eight weights from place i on; zeros past the end, which change nothing and never win. i is a multiple of eight.
+__device__ __forceinline__ void load_run(const float* q, uint32_t i, uint32_t n, float (&w)[kRun])
+{
+    if (i + kRun <= n) {
+        const float4 x = *reinterpret_cast<const float4*>(q + i), y = *reinterpret_cast<const float4*>(q + i + 4);
+        w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w, w[4] = y.x, w[5] = y.y, w[6] = y.z, w[7] = y.w;
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < kRun; ++j)
+            w[j] = i + j < n ? q[i + j] : 0.0f;
+    }
+}
+
 // The units of a binade, and what a run of candidates from i0 on adds to (kDown: takes from) a value in it.
 template <bool kDown>
 struct Binade {
@@ -75,14 +90,7 @@ struct Binade {
     __device__ __forceinline__ void run(const float* q, uint32_t i0, uint32_t n, uint32_t& u0, uint32_t& u1, float& top) const
     {
         float w[kRun];
-        if (i0 + kRun <= n) {
-            const float4 x = *reinterpret_cast<const float4*>(q + i0), y = *reinterpret_cast<const float4*>(q + i0 + 4);
-            w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w, w[4] = y.x, w[5] = y.y, w[6] = y.z, w[7] = y.w;
-        } else {
-#pragma unroll
-            for (uint32_t j = 0; j < kRun; ++j)
-                w[j] = i0 + j < n ? q[i0 + j] : 0.0f;
-        }
+        load_run(q, i0, n, w);
         float a0 = base0, a1 = base1;
         top = 0.0f;
 #pragma unroll
@@ -106,18 +114,33 @@ struct Binade {
     }
 };
 
-// One step of a chain: true when the walk ends at q.
+// Eight steps of a chain, one after the other; true when the walk ends in them (`hit` of them are passed, v is what is left).
 template <bool kDown>
-__device__ __forceinline__ bool chain_step(float& v, float q)
+__device__ __forceinline__ bool chain_steps(float& v, const float (&w)[kRun], uint32_t& hit)
 {
-    if (kDown) {
-        if (v < q)
-            return true;
-        v = __fsub_rn(v, q);
+    if (!kDown) {
+#pragma unroll
+        for (uint32_t j = 0; j < kRun; ++j)
+            v = __fadd_rn(v, w[j]);
         return false;
     }
-    v = __fadd_rn(v, q);
-    return false;
+    uint32_t short_of = 0u;
+    float r = v;
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j) {
+        short_of |= (r < w[j]) ? 1u << j : 0u;
+        r = __fsub_rn(r, w[j]);
+    }
+    if (!short_of) {
+        v = r;
+        return false;
+    }
+    hit = (uint32_t)__ffs((int)short_of) - 1u;
+#pragma unroll
+    for (uint32_t j = 0; j < kRun; ++j)
+        if (j < hit)
+            v = __fsub_rn(v, w[j]);
+    return true;
 }
 
 // The chain over q[0 .. n) from `value` on (q 16-byte aligned, no weight negative; zeros change nothing and never win). The
@@ -140,11 +163,10 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
             uint32_t clean = 0, hit = none;
             float r_hit = 0.0f;
             while (pos < n && clean < kCleanRounds && hit == none) {
-                uint32_t stop = pos; // [pos, stop) is taken element by element
+                // Taken element by element: the start of a total, where the value doubles every few candidates; where a run
+                // leaves the binade, with the runs behind it (it often leaves the next one soon); and small values.
                 const bool small = !(value >= kChainFloor && value < __int_as_float(0x7f800000)); // a NaN too
-                if (small) {
-                    stop = min(n, pos + 32u);
-                } else {
+                if (!small && (kDown || pos >= kHead)) {
                     const Binade<kDown> b(value);
                     uint32_t u0, u1;
                     float top;
@@ -165,15 +187,18 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
                     const uint32_t f = (uint32_t)__ffs((int)bad) - 1u;
                     value = (float)__shfl_sync(full, start, (int)f) * b.unit;
                     pos += f * kRun;
-                    stop = min(n, pos + kRun);
                     clean = 0;
                 }
-                for (; pos < stop; ++pos)
-                    if (chain_step<kDown>(value, q[pos])) {
-                        hit = pos;
+                const uint32_t stop = min(n, pos + kBeside);
+                for (; pos < stop && hit == none; pos += kRun) {
+                    float w[kRun];
+                    load_run(q, pos, n, w);
+                    uint32_t passed;
+                    if (chain_steps<kDown>(value, w, passed)) {
+                        hit = pos + passed;
                         r_hit = value;
-                        break;
                     }
+                }
             }
             if (lane == 0u) {
                 cs.value = value;

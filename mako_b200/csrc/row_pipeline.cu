@@ -847,7 +847,8 @@ __device__ __noinline__ void wide_finish(Smem& s, const unsigned long long* fkey
 // kernel carries none of its bookkeeping.
 // kSplit: a launch whose grid has a second dimension over slices of every row's columns (a few rows split over many CTAs: the
 // latency path; one row of 151552 columns under top_k 40 / top_p 0.95 41 us as shard records and a merge, 18.5 us so).
-template <bool kSpec, bool kSplit>
+// kMasked: rows with an allowed-token mask; apart, because the tile loop's code is what a row pays for, executed or not.
+template <bool kSpec, bool kSplit, bool kMasked>
 __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKernelArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -931,7 +932,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         }
     }
     const RowCfg cfg = make_cfg(prm, a.n_vocab, mode, a.vp_k, a.pass);
-    const uint32_t* __restrict__ mrow = a.mask ? a.mask + (size_t)row * a.mask_ld + (col0 >> 5) : nullptr;
+    const uint32_t* __restrict__ mrow = (kMasked && a.mask) ? a.mask + (size_t)row * a.mask_ld + (col0 >> 5) : nullptr;
     // Per-row scratch, 16 bytes per column: scratch_cap raw candidates (logit bits, column) — sorted in place as
     // 64-bit keys by the large sorted-list path — then as much again: the merge sort's second buffer, or (large
     // unsorted lists) one float per column.
@@ -1215,6 +1216,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             if (!long_history)
                 t_first += (fw + (kFixers / 32) - (prefixed % (kFixers / 32))) % (kFixers / 32); // t % 2 == fw
             const bool idle = long_history && fw != 0;
+            // the bias entries, four a lane, are kept at hand; what there is beyond 128 of them is read again for every tile
+            mk_bias held[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i)
+                held[i] = (lane + i * 32u < nb) ? brow[lane + i * 32u] : mk_bias{-1, 0.0f};
             uint32_t st = t_first % n_stages, k = t_first / n_stages;
             for (uint32_t t = t_first; t < n_tiles && !idle; t += t_step, st += t_step) {
                 if (st >= n_stages) {
@@ -1227,10 +1233,17 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 if (!mbar_wait(&s.full[st], k & 1, (*(volatile uint32_t*)&s.abort_flag) ? 1u : wait_probes))
                     atomicExch(&s.abort_flag, 1u);
                 if (nb > 0) {
-                    for (uint32_t j = lane; j < nb; j += 32) {
+                    const uint32_t first_id = base + (uint32_t)id_off; // ids of the tile: unsigned, those below it wrap past n_t
+#pragma unroll
+                    for (uint32_t i = 0; i < 4u; ++i) {
+                        const uint32_t loc = (uint32_t)held[i].id - first_id;
+                        if (held[i].id >= 0 && loc < n_t)
+                            tp[loc] = __fadd_rn(tp[loc], held[i].value);
+                    }
+                    for (uint32_t j = 128u + lane; j < nb; j += 32u) {
                         const mk_bias be = brow[j];
-                        const int64_t loc = (int64_t)be.id - id_off - (int64_t)base;
-                        if (be.id >= 0 && loc >= 0 && loc < (int64_t)n_t)
+                        const uint32_t loc = (uint32_t)be.id - first_id;
+                        if (be.id >= 0 && loc < n_t)
                             tp[loc] = __fadd_rn(tp[loc], be.value);
                     }
                     __syncwarp();
@@ -1290,7 +1303,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         }
                 }
         };
-        // The loop over the tiles is compiled four times, with the mask, the top_k histogram and the streamed sum
+        // The loop over the tiles is compiled four times for each kind of launch, with the mask, the top_k histogram and the streamed sum
         // compiled in or out: a row runs a variant that holds little beyond its own work. (One loop with all
         // three as run-time branches costs the common penalised row 12 % of its launch time, and all eight
         // combinations cost it 3 % again: the size of the code matters, executed or not.)
@@ -1471,25 +1484,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 if (!(kHist && cfg.hist_mode) && collect) {
                     const bool some = tm >= thr;
                     const uint32_t lanes = kAgg ? __ballot_sync(0xffffffffu, some) : 0u;
-                    if (kAgg && __popc(lanes) >= 8) {
-                        // Many lanes have something to keep (a flat row, or the first tiles of any row, before the
-                        // maximum is known): one slot range per warp — a prefix sum over the lanes' counts and one
-                        // atomic — instead of one atomic per element on the same shared-memory word.
+                    if (kAgg && __popc(lanes) >= 2) {
+                        // Many lanes have something to keep (an allowed row, a flat one, or the first tiles of any row,
+                        // before the maximum is known): one slot range a lane instead of one atomic an element.
                         uint32_t mine = 0;
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
                             mine += (w[e] >= thr) ? 1u : 0u;
-                        uint32_t inc = mine;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                            if ((int)lane >= o)
-                                inc += y;
-                        }
-                        uint32_t slot = 0;
-                        if (lane == 31)
-                            slot = atomicAdd(&s.ncand, inc);
-                        slot = __shfl_sync(0xffffffffu, slot, 31) + inc - mine;
+                        uint32_t slot = some ? atomicAdd(&s.ncand, mine) : 0u;
                         if (some) {
 #pragma unroll
                             for (int e = 0; e < kEl; ++e)
@@ -1508,16 +1510,15 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         };
         using T = std::true_type;
         using F = std::false_type;
-        if (!mrow && !cfg.hist_mode && !cfg.need_sum)
-            read_tiles(F{}, F{}, F{}, F{}); // penalties, min_p, greedy: nothing but maximum and bound
-        else if (!mrow && !cfg.need_sum)
-            read_tiles(F{}, T{}, F{}, F{}); // top_k
-        else if (!mrow && a.pass == 1)
-            read_tiles(F{}, F{}, T{}, T{}); // top_p alone, second pass: a third of a flat row is kept
-        else if (!mrow)
-            read_tiles(F{}, T{}, T{}, F{}); // top_p alone (with its first-launch histogram), shard records
+        using M = std::integral_constant<bool, kMasked>;
+        if (!cfg.hist_mode && !cfg.need_sum)
+            read_tiles(M{}, F{}, F{}, M{}); // penalties, min_p, greedy, a pure draw: nothing but maximum and bound
+        else if (!cfg.need_sum)
+            read_tiles(M{}, T{}, F{}, F{}); // top_k
+        else if (a.pass == 1)
+            read_tiles(M{}, F{}, T{}, T{}); // top_p alone, second pass: a third of a flat row is kept
         else
-            read_tiles(T{}, T{}, T{}, F{}); // masked rows: everything, chosen at run time
+            read_tiles(M{}, T{}, T{}, F{}); // top_p alone (with its first-launch histogram), shard records
     }
     __syncthreads();
 
@@ -1665,13 +1666,32 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         // second.
         const uint2* const lists = reinterpret_cast<const uint2*>(row_scratch);
         uint2* const merged = reinterpret_cast<uint2*>(row_scratch + 2u * (size_t)a.scratch_cap);
+        // A warp a slice, or, of few slices, several: 128 elements at a time.
+        constexpr uint32_t kWarps = kThreads / 32;
+        const uint32_t warps_each = max(1u, kWarps / n_slices), at_once = kWarps / warps_each;
+        auto for_each_kept = [&](auto&& f) {
+            for (uint32_t g = warp / warps_each; g < n_slices && warp < at_once * warps_each; g += at_once)
+                for (uint32_t i0 = (warp % warps_each) * 128u; i0 < n_of[g]; i0 += warps_each * 128u) {
+                    uint2 c[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        c[k] = (i0 + k * 32u + lane < n_of[g]) ? __ldcg(&lists[g * a.split_w + i0 + k * 32u + lane])
+                                                               : make_uint2(0xffffffffu, 0u); // a NaN: above no bound
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        if (i0 + k * 32u < n_of[g])
+                            f(c[k], g);
+                }
+        };
         if (cfg.hist_mode) {
-            for (uint32_t g = warp; g < n_slices; g += kThreads / 32)
-                for (uint32_t i = lane; i < n_of[g]; i += 32u) {
-                    const uint32_t bin = hist_bin(__uint_as_float(__ldcg(&lists[g * a.split_w + i]).x));
+            for_each_kept([&](const uint2& c, uint32_t) {
+                const float v = __uint_as_float(c.x);
+                if (v == v) {
+                    const uint32_t bin = hist_bin(v);
                     atomicAdd(&hist2[bin], 1u);
                     atomicMax(&s.hi_group, bin >> 5);
                 }
+            });
             __syncthreads();
             if (warp == 0) {
                 const int found = hist_scan(hist2, s.hi_group, cfg.hist_k);
@@ -1681,20 +1701,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             __syncthreads();
         }
         const float thr = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
-        for (uint32_t g = warp; g < n_slices; g += kThreads / 32)
-            for (uint32_t i0 = 0; i0 < n_of[g]; i0 += 32u) {
-                uint2 c = make_uint2(0xff800000u, 0u);
-                if (i0 + lane < n_of[g])
-                    c = __ldcg(&lists[g * a.split_w + i0 + lane]);
-                const bool in = __uint_as_float(c.x) >= thr;
-                const uint32_t bal = __ballot_sync(0xffffffffu, in);
-                uint32_t at = 0;
-                if (lane == 0 && bal)
-                    at = atomicAdd(&s.ncand, (uint32_t)__popc(bal));
-                at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
-                if (in)
-                    merged[at] = make_uint2(c.x, c.y + g * a.split_w);
-            }
+        for_each_kept([&](const uint2& c, uint32_t g) {
+            const bool in = __uint_as_float(c.x) >= thr;
+            const uint32_t bal = __ballot_sync(0xffffffffu, in);
+            uint32_t at = 0;
+            if (lane == 0 && bal)
+                at = atomicAdd(&s.ncand, (uint32_t)__popc(bal));
+            at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+            if (in)
+                merged[at] = make_uint2(c.x, c.y + g * a.split_w);
+        });
         __syncthreads();
         scratch = merged;
         qrow = reinterpret_cast<float*>(row_scratch);
@@ -2064,30 +2080,38 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         }
         double below = 0.0, exact = 0.0;
         const float c2w = cfg.inv_t * 1.4426950408889634f;
-        for (uint32_t i0 = tid; i0 < n_raw; i0 += 4u * kThreads) {
+        for (uint32_t r0 = tid - lane; r0 < n_raw; r0 += 4u * kThreads) { // a warp's lanes together
             uint2 cv[4]; // four loads in flight
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const uint32_t i = i0 + (uint32_t)k * kThreads;
+                const uint32_t i = r0 + lane + (uint32_t)k * kThreads;
                 cv[k] = (i < n_raw) ? scratch[i] : make_uint2(0xff800000u, 0u); // filler: -inf
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
+                if (r0 + (uint32_t)k * kThreads >= n_raw)
+                    break;
                 const uint2 c = cv[k];
                 const bool in = __uint_as_float(c.x) >= thr_final;
-                if (!in && (!cfg.need_sum || i0 + (uint32_t)k * kThreads >= n_raw))
-                    continue;
-                if (!in && approx_below) {
-                    below += (double)ex2_approx((__uint_as_float(c.x) - m) * c2w);
-                    continue;
+                bool keep = false;
+                float q = 0.0f;
+                if (in || (cfg.need_sum && r0 + lane + (uint32_t)k * kThreads < n_raw)) {
+                    if (!in && approx_below) {
+                        below += (double)ex2_approx((__uint_as_float(c.x) - m) * c2w);
+                    } else {
+                        q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table);
+                        if (q == q)
+                            exact += (double)q;
+                        keep = in && q >= cfg.minp_eff && q > 0.0f;
+                    }
                 }
-                const float x = __fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t);
-                const float q = expf_host_exact(x, s.exp2_table);
-                if (q == q)
-                    exact += (double)q;
-                if (in && q >= cfg.minp_eff && q > 0.0f) {
-                    const uint32_t slot = atomicAdd(&s.nsurv, 1u);
-                    if (slot < (uint32_t)kSortCap)
+                const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+                if (bal) { // one slot range per warp
+                    uint32_t slot = 0;
+                    if (lane == 0)
+                        slot = atomicAdd(&s.nsurv, (uint32_t)__popc(bal));
+                    slot = __shfl_sync(0xffffffffu, slot, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+                    if (keep && slot < (uint32_t)kSortCap)
                         keys[slot] = ((unsigned long long)__float_as_uint(q) << 32) | c.y;
                 }
             }
@@ -2481,15 +2505,14 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     if (e != cudaSuccess)
         return e;
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        e = cudaFuncSetAttribute(row_pipeline_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(row_pipeline_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e != cudaSuccess)
-            return e;
-        e = cudaFuncSetAttribute(row_pipeline_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-        if (e != cudaSuccess)
-            return e;
+        const void* const kernels[] = {(const void*)row_pipeline_kernel<false, false, false>, (const void*)row_pipeline_kernel<false, false, true>,
+                                       (const void*)row_pipeline_kernel<false, true, false>, (const void*)row_pipeline_kernel<false, true, true>,
+                                       (const void*)row_pipeline_kernel<true, false, false>, (const void*)row_pipeline_kernel<true, false, true>};
+        for (const void* k : kernels) {
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+            if (e != cudaSuccess)
+                return e;
+        }
         configured[dev] = true;
     }
     if (batch == 0)
@@ -2509,13 +2532,20 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     RowKernelArgs first = a;
     first.pass = 0;
     const bool spec = a.spec_n_pos != 0u;
-    if (a.split_w != 0u) { // one CTA per (row, slice)
+    auto launch = [&](const RowKernelArgs& x) {
+        if (spec)
+            return x.mask ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false, true>, x)
+                          : cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false, false>, x);
+        if (x.split_w != 0u)
+            return x.mask ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, true, true>, x)
+                          : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, true, false>, x);
+        return x.mask ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false, true>, x)
+                      : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false, false>, x);
+    };
+    if (a.split_w != 0u) // one CTA per (row, slice)
         lc.gridDim = dim3(batch, (a.n_vocab + a.split_w - 1u) / a.split_w);
-        e = cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, true>, first);
-        lc.gridDim = dim3(batch);
-    } else
-        e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, first)
-             : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false>, first);
+    e = launch(first);
+    lc.gridDim = dim3(batch);
     if (e != cudaSuccess)
         return e;
     // top_p alone (make_cfg: need_sum): rows whose nucleus the first launch could not settle are streamed again
@@ -2534,8 +2564,7 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
         RowKernelArgs second = a; // what is left
         second.pass = 1;
         second.split_w = 0;
-        e = spec ? cudaLaunchKernelEx(&lc, row_pipeline_kernel<true, false>, second)
-                 : cudaLaunchKernelEx(&lc, row_pipeline_kernel<false, false>, second);
+        e = launch(second);
     }
     return e;
 }

@@ -24,7 +24,7 @@ struct SplitPart {
     uint32_t bits;               // 1: the row's first column is NaN, 2: a wait ran out
     uint32_t unused;
 };
-constexpr uint32_t kMaxSlices = 64, kSplitMaxRows = 64;
+constexpr uint32_t kMaxSlices = 64, kSplitMaxRows = 148;
 
 struct RowKernelArgs {
     // inputs
