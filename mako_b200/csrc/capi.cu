@@ -166,21 +166,19 @@ bool all_greedy(const mk_rows* r)
 // A few rows leave most of the device idle when each is one CTA. Their columns are split instead, into as many slices as fill
 // the device's 296 places once (of at least a tile of 4096 columns), and the last CTA of a row to arrive draws from what all of
 // them kept. Measured (us a call, split / one CTA a row), 151552 columns: one row top_k 18.5 / 35.6, top_p 20.2 / 42.7, min_p
-// 12.3 / 20.7, greedy 7.0 / 16.9; 64 rows 28 / 36, 76 / 88, 22.3 / 26.0, 10.8 / 17.1; 148 rows 36.6 / 37.5, 99.7 / 103, 29.3 /
-// 27.9, 16.3 / 17.6 — with two slices a row the meeting of the slices is all but what they gain, so above 64 rows only
-// the greedy ones and those under the histogram bound (top_k, top_p alone) are split. Eight tiles (32000 columns): a row under
-// that bound still gains (top_k 14.1 / 17.3, top_p 17.1 / 19.7; 148 rows 21.4 / 23.9, 48 / 45), the others lose a
-// microsecond (min_p 9.4 / 8.0, greedy 6.8 / 6.4), so short rows are split only under it. `set`: which of the two row sets of p/q
-// verification (0 elsewhere).
+// 12.3 / 20.7, greedy 7.0 / 16.9, a mask's 3000 candidates 40 / 67; 148 rows 36 / 37.5, 95 / 101, 26.3 / 27.8, 16.3 / 17.6, 64 / 70
+// (two slices a row; more rows fill the device by themselves). Eight tiles (32000 columns): up to 96 rows under the histogram
+// bound still gain (one row top_k 14.1 / 17.3, top_p 17.1 / 19.7), the others lose a microsecond to the meeting of their
+// slices (min_p 9.4 / 8.0, greedy 6.8 / 6.4) and 128 rows of top_p 2.5, so short rows are split only under that bound. `set`:
+// which of the two row sets of p/q verification (0 elsewhere).
 void split_rows(mk::RowKernelArgs& a, const mk_sampler* s, uint32_t batch, uint32_t set)
 {
     if (!s->split || !s->split_parts || batch == 0 || batch > mk::kSplitMaxRows || s->timing || s->skip_tile != 0xffffffffu)
         return;
     const uint32_t n_tiles = (a.n_vocab + kTile - 1) / kTile;
     const mk_sampling_params& p = a.params;
-    const bool shared = !a.params_dev, greedy = shared && p.temperature <= 0.0f;
-    const bool bound = shared && !greedy && ((p.top_k > 0 && p.top_k < a.n_vocab) || (p.top_p < 1.0f && !(p.min_p > 0.0f)));
-    if (n_tiles < (bound ? 4u : 12u) || (batch > 64u && !bound && !greedy))
+    const bool bound = !a.params_dev && p.temperature > 0.0f && ((p.top_k > 0 && p.top_k < a.n_vocab) || (p.top_p < 1.0f && !(p.min_p > 0.0f)));
+    if (n_tiles < (bound && batch <= 96u ? 4u : 12u))
         return;
     uint32_t slices = kPlaces / batch;
     slices = slices < mk::kMaxSlices ? slices : mk::kMaxSlices;

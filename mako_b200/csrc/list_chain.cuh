@@ -11,6 +11,9 @@
 // binade, or in which the walk could end, is taken element by element by its thread; everything before it stands, and the
 // next round starts behind it with the new unit. A value crosses at most a few dozen binades.
 //
+// Ties are rare: where no run of a round has one, the increments are plain numbers, and as long as their sum stays inside the binade
+// (and, in a walk, above the largest weight) a round is one reduction. The scan is for the others.
+//
 // Rounds are taken by one warp (256 candidates) where the value crosses binades every few candidates — the start of a total,
 // the end of a walk — and by the whole CTA otherwise: what bounds both is the latency and the issue slots of a round's scan,
 // not the number of candidates.
@@ -22,13 +25,14 @@ namespace mk {
 constexpr uint32_t kRun = 8;            // candidates a thread and round
 constexpr uint32_t kUnitCap = 1u << 25; // increments are clamped here: past the binade's end whatever they are
 constexpr uint32_t kHead = 64;          // the first candidates of a total
-constexpr uint32_t kBeside = 32;        // candidates taken element by element at a crossing
+constexpr uint32_t kBeside = 32;        // candidates taken element by element where crossings are close together
 constexpr uint32_t kCleanRounds = 4;    // rounds of one warp without a crossing before the CTA takes over
 constexpr float kChainFloor = 0x1p-100f; // smaller running values are taken element by element: their unit would be a denormal
 
 template <int kThreads>
 struct ChainSmem {
     uint32_t warp0[kThreads / 32], warp1[kThreads / 32]; // increments of whole warps, by starting parity
+    uint32_t sum[2][kThreads / 32], top[2][kThreads / 32]; // by round parity: a warp's units (bit 31: not a plain number), its largest weight
     uint32_t bad[2];       // first thread whose run leaves the binade (or may end the walk), by round parity
     float value;           // the running value and the place it stands at
     uint32_t pos;
@@ -165,17 +169,38 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
             while (pos < n && clean < kCleanRounds && hit == none) {
                 // Taken element by element: the start of a total, where the value doubles every few candidates; where a run
                 // leaves the binade, with the runs behind it (it often leaves the next one soon); and small values.
+                uint32_t stop = pos + kBeside;
                 const bool small = !(value >= kChainFloor && value < __int_as_float(0x7f800000)); // a NaN too
                 if (!small && (kDown || pos >= kHead)) {
                     const Binade<kDown> b(value);
                     uint32_t u0, u1;
                     float top;
                     b.run(q, pos + lane * kRun, n, u0, u1, top);
-                    uint32_t f0 = u0, f1 = u1;
-                    warp_compose(f0, f1);
-                    uint32_t e = __shfl_up_sync(full, (b.k & 1u) ? f1 : f0, 1);
-                    if (lane == 0u)
-                        e = 0u;
+                    uint32_t e = 0u; // the units of the lanes before this one
+                    if (__all_sync(full, u0 == u1)) {
+                        const uint32_t end_all = b.after(b.k, __reduce_add_sync(full, u0));
+                        const float top_all = kDown ? __uint_as_float(__reduce_max_sync(full, __float_as_uint(top))) : 0.0f;
+                        if (!b.bad(end_all, top_all)) {
+                            value = (float)end_all * b.unit;
+                            pos += 32u * kRun;
+                            ++clean;
+                            continue;
+                        }
+                        e = u0;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t y = __shfl_up_sync(full, e, o);
+                            if ((int)lane >= o)
+                                e += y;
+                        }
+                        e -= u0;
+                    } else {
+                        uint32_t f0 = u0, f1 = u1;
+                        warp_compose(f0, f1);
+                        e = __shfl_up_sync(full, (b.k & 1u) ? f1 : f0, 1);
+                        if (lane == 0u)
+                            e = 0u;
+                    }
                     const uint32_t start = b.after(b.k, e), end = b.after(start, (start & 1u) ? u1 : u0);
                     const uint32_t bad = __ballot_sync(full, b.bad(end, top));
                     if (!bad) {
@@ -187,10 +212,10 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
                     const uint32_t f = (uint32_t)__ffs((int)bad) - 1u;
                     value = (float)__shfl_sync(full, start, (int)f) * b.unit;
                     pos += f * kRun;
+                    stop = pos + (f < 4u ? kBeside : kRun);
                     clean = 0;
                 }
-                const uint32_t stop = min(n, pos + kBeside);
-                for (; pos < stop && hit == none; pos += kRun) {
+                for (; pos < min(stop, n) && hit == none; pos += kRun) {
                     float w[kRun];
                     load_run(q, pos, n, w);
                     uint32_t passed;
@@ -221,6 +246,31 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
             uint32_t u0, u1;
             float top;
             b.run(q, i0, n, u0, u1, top);
+            const uint32_t slot = round & 1u;
+            ++round;
+            {
+                const bool plain = __all_sync(full, u0 == u1);
+                const uint32_t sum = min(__reduce_add_sync(full, u0), kUnitCap);
+                const uint32_t largest = kDown ? __reduce_max_sync(full, __float_as_uint(top)) : 0u;
+                if (lane == 0u) {
+                    cs.sum[slot][warp] = sum | (plain ? 0u : 0x80000000u);
+                    cs.top[slot][warp] = largest;
+                }
+            }
+            __syncthreads();
+            if (tid == 0)
+                cs.bad[slot ^ 1u] = (uint32_t)kThreads; // the next round's: everyone is done with the last one's
+            {
+                const uint32_t sum = (lane < kWarps) ? cs.sum[slot][lane] : 0u, largest = (lane < kWarps) ? cs.top[slot][lane] : 0u;
+                if (!__any_sync(full, sum >> 31)) {
+                    const uint32_t end = b.after(b.k, __reduce_add_sync(full, sum));
+                    if (!b.bad(end, kDown ? __uint_as_float(__reduce_max_sync(full, largest)) : 0.0f)) {
+                        value = (float)end * b.unit;
+                        pos += (uint32_t)kThreads * kRun;
+                        continue;
+                    }
+                }
+            }
             uint32_t f0 = u0, f1 = u1;
             warp_compose(f0, f1);
             if (lane == 31u) {
@@ -238,14 +288,10 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
                 before = 0u;
             before = min(before + (((b.k + before) & 1u) ? e1 : e0), 2u * kUnitCap);
             const uint32_t start = b.after(b.k, before), end = b.after(start, (start & 1u) ? u1 : u0);
-            const uint32_t slot = round & 1u;
-            ++round;
             if (b.bad(end, top))
                 atomicMin(&cs.bad[slot], tid);
             else if (tid == (uint32_t)kThreads - 1u)
                 cs.value = (float)end * b.unit;
-            if (tid == 0)
-                cs.bad[slot ^ 1u] = (uint32_t)kThreads;
             __syncthreads();
             const uint32_t f = cs.bad[slot];
             if (f < (uint32_t)kThreads) { // warp 0 goes on at this thread's run
