@@ -28,7 +28,7 @@ struct RowCfg {
 __device__ __forceinline__ unsigned long long global_ns()
 {
     unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)::"memory"); // (stays on its side of a barrier)
     return t;
 }
 

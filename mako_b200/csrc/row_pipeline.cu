@@ -1049,24 +1049,33 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         // The special columns as a bitmap: all the readers need in order to set them aside. The rest of what the
         // reference keeps about the generated tokens (a multiset id -> count, sampler.cpp:15-18) is built by the
         // side warps while the row already streams.
+        // All of a thread's atomics are in flight together; the columns they were the first to mark are listed afterwards, a slot
+        // range a warp (entry by entry, with a look at the bit before each atomic, this took 3.6 us instead of 2.8, most of it now the history on its way).
+        uint32_t firsts = 0u;
 #pragma unroll
-        for (int hi = 0; hi < kHistPerThread; ++hi) {
-            bool mine = false;
+        for (int hi = 0; hi < kHistPerThread; ++hi)
             if (hc[hi] < V) { // unsigned: an id below the row's first column wraps past V
-                const uint32_t col = hc[hi], bit = 1u << (col & 31u);
-                if (!(*(volatile uint32_t*)&bitmap[col >> 5] & bit)) // skip the atomic once the bit is visible
-                    if (!(atomicOr(&bitmap[col >> 5], bit) & bit))
-                        mine = col < span; // exactly one entry per distinct column sees its bit go from 0 to 1
+                const uint32_t bit = 1u << (hc[hi] & 31u);
+                if (!(atomicOr(&bitmap[hc[hi] >> 5], bit) & bit) && hc[hi] < span)
+                    firsts |= 1u << hi; // exactly one entry per distinct column sees its bit go from 0 to 1
             }
-            const uint32_t bal = __ballot_sync(0xffffffffu, mine);
-            if (bal) { // one slot range per warp and round
-                uint32_t at = 0;
-                if (lane == 0)
-                    at = atomicAdd(&s.n_own, (uint32_t)__popc(bal));
-                at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
-                if (mine)
-                    own_list[at] = (uint16_t)hc[hi];
+        {
+            const uint32_t mine = (uint32_t)__popc(firsts);
+            uint32_t inc = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if ((int)lane >= o)
+                    inc += y;
             }
+            uint32_t at = 0;
+            if (lane == 31u && inc)
+                at = atomicAdd(&s.n_own, inc);
+            at = __shfl_sync(0xffffffffu, at, 31) + inc - mine;
+#pragma unroll
+            for (int hi = 0; hi < kHistPerThread; ++hi)
+                if ((firsts >> hi) & 1u)
+                    own_list[at++] = (uint16_t)hc[hi];
         }
         __syncthreads();
         if (a.timing && tid == 0 && !early)
@@ -1141,7 +1150,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         }
         // no search: the list names the column, its rank is one popcount away and indexes the count
         const uint32_t n_own = s.n_own;
-#pragma unroll 2
+#pragma unroll 4
         for (uint32_t i = tid; i < n_own; i += kThreads) {
             const uint32_t c = own_list[i];
             const uint32_t rank = wpre[c >> 5] + __popc(bitmap[c >> 5] & ((1u << (c & 31u)) - 1u));
@@ -1158,7 +1167,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     if (a.timing && tid == 0)
         a.timing[(size_t)row * 64 + 1] = global_ns();
     float seen = -__int_as_float(0x7f800000); // the largest element of the row this warp knows of
-    double sum_acc = 0.0; // need_sum: sum of exp2((l - seen) * c2) over this thread's elements (the uncollected ones)
+    // need_sum: sum of exp2(l * c2 - sref) over this thread's elements (the uncollected ones); sref is seen * c2 rounded to a
+    // float and counts as that float, so that the argument is one fused multiply-add with one rounding
+    double sum_acc = 0.0;
+    float sref = 0.0f;
 
     if (warp == 0) {
         // producer
@@ -1386,10 +1398,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         s.nan0 = 1;
                 }
 
-                float tq[kVec], tm = ninf; // the largest of each four, and of all (NaN is never the larger)
+                float tq[kVec], tm = ninf; // the largest of each four (NaN if all are), and of all (NaN is never the larger)
 #pragma unroll
                 for (int j = 0; j < kVec; ++j) {
-                    tq[j] = fmaxf(fmaxf(fmaxf(w[4 * j], ninf), w[4 * j + 1]), fmaxf(w[4 * j + 2], w[4 * j + 3]));
+                    tq[j] = fmaxf(fmaxf(w[4 * j], w[4 * j + 1]), fmaxf(w[4 * j + 2], w[4 * j + 3]));
                     tm = fmaxf(tm, tq[j]);
                 }
                 // An element that is the row's maximum is at or above all its warp knows of. Only a warp that may hold
@@ -1411,8 +1423,12 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         }
                     }
                     seen = fmaxf(wm, m_run);
-                    if (kSum && cfg.need_sum && seen > before)
-                        sum_acc *= (double)exp2f((before - seen) * c2);
+                    if (kSum && cfg.need_sum && seen > before) {
+                        const float to = __fmul_rn(seen, c2);
+                        if (before > ninf) // (else nothing is summed yet)
+                            sum_acc *= (double)exp2f(sref - to);
+                        sref = to;
+                    }
                 }
                 // Under the histogram bound the distance from the maximum only matters where min_p or a large top_k makes
                 // it the tighter of the two.
@@ -1468,16 +1484,17 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest (and
                     // of a shard record) every element; else of what is NOT collected (`thr` is the bound
                     // the collection used): the collected elements get exact weights in the finish, so only the far tail
-                    // carries the approximation. NaN weighs nothing.
+                    // carries the approximation. (A NaN makes the sum of every
+                    // element one; such a row is left to the second launch.)
                     float p = 0.0f;
-                    if (kHist && sum_all) { // (the maximum with -inf is what a NaN turns into)
+                    if (kHist && sum_all) {
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
-                            p += ex2_approx((fmaxf(w[e], ninf) - seen) * c2);
+                            p += ex2_approx(__fmaf_rn(w[e], c2, -sref));
                     } else {
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
-                            p += w[e] < thr ? ex2_approx((w[e] - seen) * c2) : 0.0f;
+                            p += w[e] < thr ? ex2_approx(__fmaf_rn(w[e], c2, -sref)) : 0.0f;
                     }
                     sum_acc += (double)p;
                 }
@@ -1552,14 +1569,14 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         arg_col = shift;
     }
     // need_sum: weight of the uncollected tail (the whole row for a shard record), relative to the row maximum:
-    // sum over reader threads of sum_acc * exp2((best - m) * c2), fixed order
+    // sum over reader threads of sum_acc * exp2(sref - m * c2), fixed order
     double total_approx = 0.0;
     if (cfg.need_sum) {
         double part = 0.0;
         if (warp > kFixers / 32) {
             const float c2 = cfg.inv_t * 1.4426950408889634f;
-            if (seen > -__int_as_float(0x7f800000) && sum_acc > 0.0)
-                part += sum_acc * exp2((double)(seen - m) * (double)c2);
+            if (seen > -__int_as_float(0x7f800000) && !(sum_acc <= 0.0))
+                part += sum_acc * exp2((double)sref - (double)m * (double)c2);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -1627,8 +1644,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             if (cfg.need_sum)
                 for (uint32_t g = lane; g < n_slices; g += 32u) {
                     const double sg = __ldcg(&parts[g].sum);
-                    if (sg > 0.0)
-                        sum += sg * exp2((double)(__ldcg(&parts[g].m) - mm) * ((double)cfg.inv_t * 1.4426950408889634));
+                    if (!(sg <= 0.0)) // a NaN goes on
+                        sum += sg * exp2((double)(__ldcg(&parts[g].m) - mm) * (double)(cfg.inv_t * 1.4426950408889634f));
                 }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
@@ -1726,51 +1743,65 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // warps wait at one barrier. A one-shot phase waits for its instructions more than for anything else, so this path
     // is short and contiguous; every other row falls through to the general finish below, which recomputes from the
     // collected elements.
-    constexpr uint32_t kFastRaw = 256;
-    if (mode != kModeVpLocal && !cfg.greedy && !s.nan0 && s.ncand <= 2u * kFastRaw && s.ncand <= scratch_cap) {
+    constexpr uint32_t kFastRaw = 512;
+    if (mode != kModeVpLocal && !cfg.greedy && !s.nan0 && s.ncand <= kFastRaw && s.ncand <= scratch_cap &&
+        !(cfg.optimistic && total_approx != total_approx)) {
         // Compiled twice: rows whose total is the candidates' own (nearly all) run code that knows nothing of the
         // row total of top_p alone.
-        auto short_finish = [&](auto row_total_tag) {
-            constexpr bool kRowTotal = decltype(row_total_tag)::value;
-            const uint32_t full = 0xffffffffu;
+        // Every thread takes one collected element, or two: exact weights, and the survivors of the exact filter side by side.
+        double* const fsum = reinterpret_cast<double*>(dyn + kOffKeys + 8u * kWideCand);
+        {
             const uint32_t n_raw = s.ncand;
             const float thr_final = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
             unsigned long long* const fkeys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
-            uint32_t n = 0;
             double sum_kept = 0.0, sum_again = 0.0; // top_p alone: exact weights at or above the bound; what the streamed sum has too much
-            for (uint32_t r0 = 0; r0 < n_raw && n <= kWideCand; r0 += kFastRaw) { // once, for nearly every row
-                uint2 craw[kFastRaw / 32]; // all requested at once: one trip to memory under load, not one per chunk
-#pragma unroll
-                for (uint32_t i = 0; i < kFastRaw / 32; ++i)
-                    craw[i] = (r0 + i * 32u + lane < n_raw) ? scratch[r0 + i * 32u + lane] : make_uint2(0xff800000u, 0u);
-#pragma unroll
-                for (uint32_t i = 0; i < kFastRaw / 32; ++i) {
-                    if (r0 + i * 32u >= n_raw || n > kWideCand)
-                        break;
-                    const uint2 c = craw[i];
-                    float q = 0.0f;
-                    if (__uint_as_float(c.x) >= thr_final) {
-                        q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table);
-                    }
-                    if (kRowTotal) {
-                        // as streamed: of a kept element to be taken out again where the sum took every element, of
-                        // one collected while the bound was lower to be added where it took none of the collected
-                        const bool in = __uint_as_float(c.x) >= thr_final;
-                        const double streamed = (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
-                        if (in && q == q)
-                            sum_kept += (double)q;
-                        if (in == cfg.optimistic && streamed == streamed)
-                            sum_again += in ? streamed : -streamed;
-                    }
-                    const bool ok = q >= cfg.minp_eff && q > 0.0f; // false for NaN
-                    const uint32_t bal = __ballot_sync(full, ok);
-                    const uint32_t pos = n + (uint32_t)__popc(bal & ((1u << lane) - 1u));
+            for (uint32_t r0 = tid - lane; r0 < n_raw; r0 += (uint32_t)kThreads) {
+                const uint2 c = (r0 + lane < n_raw) ? scratch[r0 + lane] : make_uint2(0xff800000u, 0u);
+                const bool in = __uint_as_float(c.x) >= thr_final;
+                const float q = in ? expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table) : 0.0f;
+                if (cfg.need_sum) {
+                    // as streamed: of a kept element to be taken out again where the sum took every element, of one
+                    // collected while the bound was lower to be added where it took none of the collected
+                    const double streamed = (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
+                    if (in && q == q)
+                        sum_kept += (double)q;
+                    if (in == cfg.optimistic && streamed == streamed)
+                        sum_again += in ? streamed : -streamed;
+                }
+                const bool ok = q >= cfg.minp_eff && q > 0.0f; // false for NaN
+                const uint32_t bal = __ballot_sync(0xffffffffu, ok);
+                if (bal) {
+                    uint32_t pos = 0;
+                    if (lane == 0)
+                        pos = atomicAdd(&s.nsurv, (uint32_t)__popc(bal));
+                    pos = __shfl_sync(0xffffffffu, pos, 0) + (uint32_t)__popc(bal & ((1u << lane) - 1u));
                     if (ok && pos < kWideCand)
                         fkeys[pos] = ((unsigned long long)__float_as_uint(q) << 32) | c.y;
-                    n += (uint32_t)__popc(bal);
                 }
             }
-            __syncwarp();
+            if (cfg.need_sum) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    sum_kept += __shfl_xor_sync(0xffffffffu, sum_kept, o);
+                    sum_again += __shfl_xor_sync(0xffffffffu, sum_again, o);
+                }
+                if (lane == 0) {
+                    fsum[warp] = sum_kept;
+                    fsum[kThreads / 32 + warp] = sum_again;
+                }
+            }
+        }
+        __syncthreads();
+        auto short_finish = [&](auto row_total_tag) {
+            constexpr bool kRowTotal = decltype(row_total_tag)::value;
+            const uint32_t full = 0xffffffffu;
+            unsigned long long* const fkeys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
+            uint32_t n = s.nsurv;
+            double sum_kept = 0.0, sum_again = 0.0; // the warps' shares, below
+            if (kRowTotal && lane < (uint32_t)(kThreads / 32)) {
+                sum_kept = fsum[lane];
+                sum_again = fsum[kThreads / 32 + lane];
+            }
             bool done = n <= 32u;
             if (!kRowTotal && n > 32u && n <= kWideCand) {
                 const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
@@ -1961,6 +1992,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         __syncthreads();
         if (s.n_final)
             return;
+        if (tid == 0)
+            s.nsurv = 0; // counted again below
         __syncthreads(); // n_final is written again below
         if (tid == 0)
             s.n_final = 0;
