@@ -783,9 +783,8 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
     // Four head rows per warp and trip, each lane 2 x 4 consecutive floats of a row (128-bit loads; rank a multiple
     // of 4, the rest of a shorter rank reads as zero): 4 KB in flight per warp.
     constexpr uint32_t kRows = 4;
-    const uint32_t warps = gridDim.x * (kPickThreads / 32);
-    for (uint32_t v0 = (blockIdx.x * (kPickThreads / 32) + warp) * kRows; v0 < n_vocab; v0 += warps * kRows) {
-        float4 h[kRows][2];
+    const uint32_t stride = gridDim.x * (kPickThreads / 32) * kRows;
+    auto fetch = [&](uint32_t v0, float4 (&h)[kRows][2]) {
 #pragma unroll
         for (uint32_t r = 0; r < kRows; ++r)
 #pragma unroll
@@ -795,6 +794,33 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
                               ? __ldg(reinterpret_cast<const float4*>(head + (size_t)(v0 + r) * rank + i))
                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
+    };
+    // Several sequences: the next trip's rows, and the logit this lane adds, are on their way while this trip's products are formed
+    // (a trip's loads in front of its products: 51 us for eight sequences of 129280 x 256; so, 33 us).
+    auto fetch_logit = [&](uint32_t v0) -> float {
+        const uint32_t q = lane >> 2, v = v0 + (lane & 3u);
+        return (q < n_seq && v < n_vocab) ? __ldg(logits + (size_t)q * ld + v) : 0.0f;
+    };
+    uint32_t v0 = (blockIdx.x * (kPickThreads / 32) + warp) * kRows;
+    float4 next[kRows][2];
+    float next_logit = 0.0f;
+    if constexpr (kSeq > 1) {
+        fetch(v0, next);
+        next_logit = fetch_logit(v0);
+    }
+    for (; v0 < n_vocab; v0 += stride) {
+        float4 h[kRows][2];
+        float logit = 0.0f;
+        if constexpr (kSeq > 1) {
+#pragma unroll
+            for (uint32_t r = 0; r < kRows; ++r)
+                h[r][0] = next[r][0], h[r][1] = next[r][1];
+            logit = next_logit;
+            fetch(v0 + stride, next);
+            next_logit = fetch_logit(v0 + stride);
+        } else {
+            fetch(v0, h);
+        }
         if constexpr (kSeq == 1) {
     #pragma unroll
             for (int b = 0; b < kSeq; ++b) {
@@ -860,7 +886,7 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
             }
             const uint32_t q = lane >> 2, v = v0 + (lane & 3u);
             if (q < n_seq && v < n_vocab) {
-                const float sc = __ldg(logits + (size_t)q * ld + v) + acc[0];
+                const float sc = logit + acc[0];
                 const unsigned long long key = (sc > -__int_as_float(0x7f800000))
                                                    ? (((unsigned long long)order_key(sc) << 32) | (0xffffffffu - v))
                                                    : 0ull;
@@ -881,20 +907,10 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
     __syncthreads();
     if (tid < n_seq && s_best[tid])
         atomicMax(&best[tid], s_best[tid]);
-    // The CTA that arrives last (a ticket counter behind the maxima) has every CTA's maximum in front of it: it
-    // writes the drafts and the confidences (ds_draft_pick's second half) and leaves maxima and counter clear for the
-    // next call.
-    __shared__ uint32_t s_last;
+    // The confidences (ds_draft_pick's second half) depend on no score: the last CTAs of the grid, which have a trip less, form
+    // one each. (One after the other behind the ticket they were a tail of 12 us for eight sequences.)
     __shared__ float s_part[kPickThreads / 32];
-    __threadfence();
-    __syncthreads();
-    if (tid == 0)
-        s_last = atomicAdd(reinterpret_cast<unsigned int*>(best + kPickMaxSeq), 1u) == gridDim.x - 1u;
-    __syncthreads();
-    if (!s_last)
-        return;
-    __threadfence();
-    for (uint32_t b = 0; b < n_seq; ++b) {
+    for (uint32_t b = gridDim.x - 1u - blockIdx.x; b < n_seq; b += gridDim.x) {
         float d = 0.0f;
         for (uint32_t i = tid; i < dim + rank; i += kPickThreads)
             d = fmaf(__ldg(w + i), i < dim ? __ldg(x + (size_t)b * x_ld + i) : s_e[b][i - dim], d);
@@ -908,12 +924,25 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
             float sum = 0.0f;
             for (int k = 0; k < kPickThreads / 32; ++k)
                 sum += s_part[k];
-            const unsigned long long key = *(volatile unsigned long long*)&best[b];
-            best[b] = 0ull;
-            draft[b] = key ? (int32_t)(0xffffffffu - (uint32_t)(key & 0xffffffffull)) : 0; // nothing comparable: id 0
             conf[b] = 1.0f / (1.0f + expf(-sum));
         }
         __syncthreads();
+    }
+    // The CTA that arrives last (a ticket counter behind the maxima) has every CTA's maximum in front of it: it
+    // writes the drafts and leaves maxima and counter clear for the next call.
+    __shared__ uint32_t s_last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0)
+        s_last = atomicAdd(reinterpret_cast<unsigned int*>(best + kPickMaxSeq), 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last)
+        return;
+    __threadfence();
+    if (tid < n_seq) {
+        const unsigned long long key = *(volatile unsigned long long*)&best[tid];
+        best[tid] = 0ull;
+        draft[tid] = key ? (int32_t)(0xffffffffu - (uint32_t)(key & 0xffffffffull)) : 0; // nothing comparable: id 0
     }
     if (tid == 0)
         *reinterpret_cast<unsigned int*>(best + kPickMaxSeq) = 0u;
