@@ -122,191 +122,225 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
         return;
     }
 
-    // exact weights. The id field of a key carries the shard the candidate came from in its top six bits (ids stay
-    // below 2^26, checked by the caller): shards ascend in id, so the order by id is unchanged, and the count of a
-    // shard's members in the deciding set below needs no knowledge of how the columns were split.
-    if (!nan0) {
-        for (uint32_t e = tid; e < a.n_shards * a.k; e += n_thr) {
-            const uint32_t g = e / a.k, i = e % a.k;
-            const uint32_t ng = s_hdr[g] & 0xffffu;
-            if (i >= ng)
-                continue;
-            const uint2 c = reinterpret_cast<const uint2*>(rec(g) + kVpHeaderBytes)[i];
-            const float x = __fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t);
-            const float q = expf_host_exact(x, s_exp2);
-            if (q >= minp_eff && q > 0.0f) {
-                const uint32_t slot = atomicAdd(&s_n, 1u);
-                keys[slot] = ((unsigned long long)__float_as_uint(q) << 32) | (g << kShardShift) | c.y;
-            }
-        }
-    }
-    __syncthreads();
-    uint32_t n = s_n;
-    if (n == 0) {
-        flags |= MK_FLAG_NO_CANDIDATE;
-        if (tid == 0)
-            keys[0] = ((unsigned long long)__float_as_uint(1.0f) << 32) | arg_shard << kShardShift | arg_id;
-        n = 1;
-        __syncthreads();
-    }
     const bool minp_on = minp_eff > 0.0f;
-    const bool cut_k = prm.top_k > 0 && prm.top_k < n;
     const bool use_topp = prm.top_p < 1.0f;
-    const bool sorted = cut_k || use_topp;
     const bool need_sum = use_topp && !minp_on && !(prm.top_k > 0 && prm.top_k < a.n_vocab_total);
-    uint32_t n2 = 2;
-    while (n2 < n)
-        n2 <<= 1;
-    for (uint32_t i = tid; i < n2; i += n_thr) {
-        unsigned long long key = ~0ull;
-        if (i < n) {
-            const unsigned long long raw = keys[i];
-            const uint32_t qb = (uint32_t)(raw >> 32), id = (uint32_t)(raw & 0xffffffffull);
-            key = sorted ? (((unsigned long long)(~qb) << 32) | id) : (((unsigned long long)id << 32) | qb);
-        }
-        keys[i] = key;
-    }
-    __syncthreads();
-    if (n > 1)
-        sort_keys(keys, n2, n_thr);
-
-    // The rest is sequential by the reference's definition (double sums for top_p, a float total, the walk) or tiny:
-    // one warp runs it, the candidates handed round 32 at a time by shuffles so that no chain waits for a load.
-    if (tid < 32) {
-        const uint32_t lane = tid, full = 0xffffffffu;
-        auto q_at = [&](uint32_t i) -> float {
-            const unsigned long long key = keys[i];
-            return sorted ? __uint_as_float(~(uint32_t)(key >> 32)) : __uint_as_float((uint32_t)(key & 0xffffffffull));
-        };
-        auto tag_at = [&](uint32_t i) -> uint32_t { // shard << kShardShift | token id
-            const unsigned long long key = keys[i];
-            return sorted ? (uint32_t)(key & 0xffffffffull) : (uint32_t)(key >> 32);
-        };
-        // A shard whose whole list is inside the deciding set may hold further members the merge cannot see.
-        uint32_t n_decide = n; // the set whose completeness matters: all candidates when the total is their sum
-        if (cut_k)
-            n = prm.top_k;
-        if (use_topp) {
-            double total = 0.0, band = 0.0;
-            if (need_sum && !(flags & MK_FLAG_NO_CANDIDATE)) {
-                const double c2 = (double)inv_t * 1.4426950408889634;
-                for (uint32_t g0 = 0; g0 < a.n_shards; g0 += 32u) { // the shards' rescaled sums, added in shard order
-                    const uint32_t g = g0 + lane;
-                    double term = 0.0;
-                    if (g < a.n_shards && s_max[g] > ninf && s_sum[g] > 0.0)
-                        term = s_sum[g] * exp2((double)(s_max[g] - m) * c2);
-                    const int cnt = (int)min(32u, a.n_shards - g0);
-                    for (int j = 0; j < cnt; ++j)
-                        total += __shfl_sync(full, term, j);
+    // Top_p alone: the nucleus is a handful of tokens as a rule, so a few of every shard's best are looked at first, 64 in all —
+    // 21 steps of the sort within two warps instead of 45 over eight — and all of them only if the nucleus reaches down to
+    // one that was left out. (1024 rows of eight shards: MERGE_US.)
+    __shared__ uint32_t s_bound, s_settled;
+    if (tid == 0)
+        s_bound = 0u;
+    uint32_t n = 0;
+    bool sorted = false;
+    for (int attempt = 0;; ++attempt) {
+        const uint32_t per = (attempt == 0 && need_sum) ? min(a.k, max(1u, 64u / a.n_shards)) : a.k;
+        flags = 0;
+        if (attempt == 0)
+            __syncthreads();
+        // exact weights. The id field of a key carries the shard the candidate came from in its top six bits (ids stay
+        // below 2^26, checked by the caller): shards ascend in id, so the order by id is unchanged, and the count of a
+        // shard's members in the deciding set below needs no knowledge of how the columns were split.
+        if (!nan0) {
+            for (uint32_t e = tid; e < a.n_shards * per; e += n_thr) {
+                const uint32_t g = e / per, i = e % per;
+                const uint32_t ng = s_hdr[g] & 0xffffu;
+                if (i >= ng)
+                    continue;
+                const uint2 c = reinterpret_cast<const uint2*>(rec(g) + kVpHeaderBytes)[i];
+                const float x = __fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t);
+                const float q = expf_host_exact(x, s_exp2);
+                if (q >= minp_eff && q > 0.0f) {
+                    const uint32_t slot = atomicAdd(&s_n, 1u);
+                    keys[slot] = ((unsigned long long)__float_as_uint(q) << 32) | (g << kShardShift) | c.y;
                 }
-                band = 1e-5 * total;
             }
-            // prefix sums in double, a run of candidates a lane (their rounding is far inside `band`)
-            const uint32_t len = (n + 31u) / 32u, r0 = min(lane * len, n), r1 = min(r0 + len, n);
-            double mine = 0.0;
-            for (uint32_t i = r0; i < r1; ++i)
-                mine += (double)q_at(i);
-            double inc = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double y = __shfl_up_sync(full, inc, o);
-                if ((int)lane >= o)
-                    inc += y;
+        }
+        if (per < a.k && tid < a.n_shards && !nan0 && (s_hdr[tid] & 0xffffu) > per) { // the best of what is left out
+            const uint2 c = reinterpret_cast<const uint2*>(rec(tid) + kVpHeaderBytes)[per];
+            const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t), s_exp2);
+            if (q > 0.0f)
+                atomicMax(&s_bound, __float_as_uint(q));
+        }
+        __syncthreads();
+        n = s_n;
+        if (n == 0) {
+            flags |= MK_FLAG_NO_CANDIDATE;
+            if (tid == 0)
+                keys[0] = ((unsigned long long)__float_as_uint(1.0f) << 32) | arg_shard << kShardShift | arg_id;
+            n = 1;
+            __syncthreads();
+        }
+        const bool cut_k = prm.top_k > 0 && prm.top_k < n;
+        sorted = cut_k || use_topp;
+        uint32_t n2 = 2;
+        while (n2 < n)
+            n2 <<= 1;
+        for (uint32_t i = tid; i < n2; i += n_thr) {
+            unsigned long long key = ~0ull;
+            if (i < n) {
+                const unsigned long long raw = keys[i];
+                const uint32_t qb = (uint32_t)(raw >> 32), id = (uint32_t)(raw & 0xffffffffull);
+                key = sorted ? (((unsigned long long)(~qb) << 32) | id) : (((unsigned long long)id << 32) | qb);
             }
-            const double list_total = __shfl_sync(full, inc, 31);
-            if (!(need_sum && !(flags & MK_FLAG_NO_CANDIDATE))) {
-                total = list_total;
-                band = 0x1p-40 * total;
+            keys[i] = key;
+        }
+        __syncthreads();
+        if (n > 1)
+            sort_keys(keys, n2, n_thr);
+
+        // The rest is sequential by the reference's definition (double sums for top_p, a float total, the walk) or tiny:
+        // one warp runs it, the candidates handed round 32 at a time by shuffles so that no chain waits for a load.
+        if (tid < 32) {
+            const uint32_t lane = tid, full = 0xffffffffu;
+            auto q_at = [&](uint32_t i) -> float {
+                const unsigned long long key = keys[i];
+                return sorted ? __uint_as_float(~(uint32_t)(key >> 32)) : __uint_as_float((uint32_t)(key & 0xffffffffull));
+            };
+            auto tag_at = [&](uint32_t i) -> uint32_t { // shard << kShardShift | token id
+                const unsigned long long key = keys[i];
+                return sorted ? (uint32_t)(key & 0xffffffffull) : (uint32_t)(key >> 32);
+            };
+            bool settled = true;
+            // A shard whose whole list is inside the deciding set may hold further members the merge cannot see.
+            uint32_t n_decide = n; // the set whose completeness matters: all candidates when the total is their sum
+            if (cut_k)
+                n = prm.top_k;
+            if (use_topp) {
+                double total = 0.0, band = 0.0;
+                if (need_sum && !(flags & MK_FLAG_NO_CANDIDATE)) {
+                    const double c2 = (double)inv_t * 1.4426950408889634;
+                    for (uint32_t g0 = 0; g0 < a.n_shards; g0 += 32u) { // the shards' rescaled sums, added in shard order
+                        const uint32_t g = g0 + lane;
+                        double term = 0.0;
+                        if (g < a.n_shards && s_max[g] > ninf && s_sum[g] > 0.0)
+                            term = s_sum[g] * exp2((double)(s_max[g] - m) * c2);
+                        const int cnt = (int)min(32u, a.n_shards - g0);
+                        for (int j = 0; j < cnt; ++j)
+                            total += __shfl_sync(full, term, j);
+                    }
+                    band = 1e-5 * total;
+                }
+                // prefix sums in double, a run of candidates a lane (their rounding is far inside `band`)
+                const uint32_t len = (n + 31u) / 32u, r0 = min(lane * len, n), r1 = min(r0 + len, n);
+                double mine = 0.0;
+                for (uint32_t i = r0; i < r1; ++i)
+                    mine += (double)q_at(i);
+                double inc = mine;
+    #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double y = __shfl_up_sync(full, inc, o);
+                    if ((int)lane >= o)
+                        inc += y;
+                }
+                const double list_total = __shfl_sync(full, inc, 31);
+                if (!(need_sum && !(flags & MK_FLAG_NO_CANDIDATE))) {
+                    total = list_total;
+                    band = 0x1p-40 * total;
+                }
+                const double want = (double)prm.top_p * total;
+                double run = inc - mine, prev = run;
+                uint32_t k = 0xffffffffu; // candidates taken: the first count whose sum is not below `want`
+                for (uint32_t i = r0; i < r1; ++i) {
+                    prev = run;
+                    run += (double)q_at(i);
+                    if (!(run < want)) {
+                        k = i + 1u;
+                        break;
+                    }
+                }
+                const uint32_t k_all = __reduce_min_sync(full, k);
+                if (k_all != 0xffffffffu) {
+                    const int owner = __ffs((int)__ballot_sync(full, k == k_all)) - 1;
+                    run = __shfl_sync(full, run, owner);
+                    prev = __shfl_sync(full, prev, owner);
+                    k = k_all;
+                } else { // the list ends first
+                    run = list_total;
+                    prev = list_total - (double)q_at(n - 1u);
+                    k = n;
+                }
+                // of a few of every shard's best: settled if the nucleus ends above all that were left out
+                if (per < a.k)
+                    settled = k_all != 0xffffffffu && __float_as_uint(q_at(k - 1u)) > s_bound;
+                if (need_sum && run < want)
+                    flags |= MK_FLAG_VP_TRUNCATED;
+                if (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))
+                    flags |= MK_FLAG_GUARD_BAND;
+                n = max(k, 1u);
+                if (need_sum)
+                    n_decide = n;
             }
-            const double want = (double)prm.top_p * total;
-            double run = inc - mine, prev = run;
-            uint32_t k = 0xffffffffu; // candidates taken: the first count whose sum is not below `want`
-            for (uint32_t i = r0; i < r1; ++i) {
-                prev = run;
-                run += (double)q_at(i);
-                if (!(run < want)) {
-                    k = i + 1u;
+            if (lane == 0)
+                s_settled = settled ? 1u : 0u;
+            if (settled) {
+            if (cut_k && !use_topp)
+                n_decide = n;
+            else if (cut_k)
+                n_decide = min(n_decide, prm.top_k);
+            // count members per shard among the deciding set
+            for (uint32_t i = lane; i < n_decide; i += 32u)
+                atomicAdd(&s_shard_in[tag_at(i) >> kShardShift], 1u);
+            __syncwarp();
+            bool cut_short = false;
+            for (uint32_t g = lane; g < a.n_shards && g < 64u; g += 32u) {
+                const uint32_t hdr = s_hdr[g];
+                const uint32_t ng = hdr & 0xffffu;
+                const bool more = (hdr & 0x40000000u) != 0;
+                cut_short = cut_short || (hdr & 0x80000000u) || (more && ng > 0 && s_shard_in[g] >= ng);
+            }
+            if (__any_sync(full, cut_short))
+                flags |= MK_FLAG_VP_TRUNCATED;
+            // 32 candidates a step, lanes past the end of the list holding zeros (which change nothing and never win): the
+            // shuffles do not depend on the chains, which then run at the adder's latency
+            float total = 0.0f;
+            for (uint32_t base = 0; base < n; base += 32u) {
+                const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
+    #pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    total = __fadd_rn(total, __shfl_sync(full, q, j));
+            }
+            float r = __fmul_rn(a.u[row], total);
+            const float eps = 1e-6f * total;
+            uint32_t hit = n - 1u;
+            float q_hit = q_at(n - 1u);
+            for (uint32_t base = 0; base < n; base += 32u) {
+                const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
+                uint32_t short_of = 0u;
+                float rr = r;
+    #pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const float qj = __shfl_sync(full, q, j);
+                    short_of |= (rr < qj) ? (1u << j) : 0u;
+                    rr = __fsub_rn(rr, qj);
+                }
+                if (short_of) { // the first candidate the draw falls short of; the remainder in front of it, once more
+                    const int jh = __ffs((int)short_of) - 1;
+                    for (int j = 0; j < jh; ++j)
+                        r = __fsub_rn(r, __shfl_sync(full, q, j));
+                    hit = base + (uint32_t)jh;
+                    q_hit = __shfl_sync(full, q, jh);
+                    if ((hit > 0 && r < eps) || (hit + 1 < n && __fsub_rn(q_hit, r) < eps))
+                        flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
                     break;
                 }
+                r = rr;
             }
-            const uint32_t k_all = __reduce_min_sync(full, k);
-            if (k_all != 0xffffffffu) {
-                const int owner = __ffs((int)__ballot_sync(full, k == k_all)) - 1;
-                run = __shfl_sync(full, run, owner);
-                prev = __shfl_sync(full, prev, owner);
-                k = k_all;
-            } else { // the list ends first
-                run = list_total;
-                prev = list_total - (double)q_at(n - 1u);
-                k = n;
+            if (lane == 0) {
+                if (a.token) a.token[row] = (int32_t)(tag_at(hit) & kIdMask);
+                if (a.prob) a.prob[row] = __fdiv_rn(q_hit, total);
+                if (a.flags) a.flags[row] = flags;
+                if (a.n_cand) a.n_cand[row] = n;
+                s_nfinal = n;
             }
-            if (need_sum && run < want)
-                flags |= MK_FLAG_VP_TRUNCATED;
-            if (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))
-                flags |= MK_FLAG_GUARD_BAND;
-            n = max(k, 1u);
-            if (need_sum)
-                n_decide = n;
-        }
-        if (cut_k && !use_topp)
-            n_decide = n;
-        else if (cut_k)
-            n_decide = min(n_decide, prm.top_k);
-        // count members per shard among the deciding set
-        for (uint32_t i = lane; i < n_decide; i += 32u)
-            atomicAdd(&s_shard_in[tag_at(i) >> kShardShift], 1u);
-        __syncwarp();
-        bool cut_short = false;
-        for (uint32_t g = lane; g < a.n_shards && g < 64u; g += 32u) {
-            const uint32_t hdr = s_hdr[g];
-            const uint32_t ng = hdr & 0xffffu;
-            const bool more = (hdr & 0x40000000u) != 0;
-            cut_short = cut_short || (hdr & 0x80000000u) || (more && ng > 0 && s_shard_in[g] >= ng);
-        }
-        if (__any_sync(full, cut_short))
-            flags |= MK_FLAG_VP_TRUNCATED;
-        // 32 candidates a step, lanes past the end of the list holding zeros (which change nothing and never win): the
-        // shuffles do not depend on the chains, which then run at the adder's latency
-        float total = 0.0f;
-        for (uint32_t base = 0; base < n; base += 32u) {
-            const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                total = __fadd_rn(total, __shfl_sync(full, q, j));
-        }
-        float r = __fmul_rn(a.u[row], total);
-        const float eps = 1e-6f * total;
-        uint32_t hit = n - 1u;
-        float q_hit = q_at(n - 1u);
-        for (uint32_t base = 0; base < n; base += 32u) {
-            const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-            uint32_t short_of = 0u;
-            float rr = r;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float qj = __shfl_sync(full, q, j);
-                short_of |= (rr < qj) ? (1u << j) : 0u;
-                rr = __fsub_rn(rr, qj);
             }
-            if (short_of) { // the first candidate the draw falls short of; the remainder in front of it, once more
-                const int jh = __ffs((int)short_of) - 1;
-                for (int j = 0; j < jh; ++j)
-                    r = __fsub_rn(r, __shfl_sync(full, q, j));
-                hit = base + (uint32_t)jh;
-                q_hit = __shfl_sync(full, q, jh);
-                if ((hit > 0 && r < eps) || (hit + 1 < n && __fsub_rn(q_hit, r) < eps))
-                    flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
-                break;
-            }
-            r = rr;
         }
-        if (lane == 0) {
-            if (a.token) a.token[row] = (int32_t)(tag_at(hit) & kIdMask);
-            if (a.prob) a.prob[row] = __fdiv_rn(q_hit, total);
-            if (a.flags) a.flags[row] = flags;
-            if (a.n_cand) a.n_cand[row] = n;
-            s_nfinal = n;
-        }
+        __syncthreads();
+        if (s_settled)
+            break;
+        if (tid == 0)
+            s_n = 0;
+        __syncthreads();
     }
     __syncthreads();
     if (a.cand_ids || a.cand_q) {

@@ -1168,7 +1168,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         a.timing[(size_t)row * 64 + 1] = global_ns();
     float seen = -__int_as_float(0x7f800000); // the largest element of the row this warp knows of
     // need_sum: sum of exp2(l * c2 - sref) over this thread's elements (the uncollected ones); sref is seen * c2 rounded to a
-    // float and counts as that float, so that the argument is one fused multiply-add with one rounding
+    // float and counts as that float, so that the argument is one fused multiply-add with one rounding.
     double sum_acc = 0.0;
     float sref = 0.0f;
 
@@ -1298,8 +1298,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         const float c2 = cfg.inv_t * 1.4426950408889634f;
         const float ninf = -__int_as_float(0x7f800000);
         const bool collect = !cfg.greedy || mode == kModeVpLocal;
-        // A nucleus that is to be found among the few largest, or a shard record: the streamed sum takes every element.
-        const bool sum_all = mode == kModeVpLocal || cfg.optimistic;
+        // A nucleus that is to be found among the few largest: the streamed sum takes every element.
+        const bool sum_all = cfg.optimistic;
         const bool hist_bound_alone = !(cfg.minp_eff > 0.0f) && cfg.hist_k <= kVpMaxK + 1u;
         // What a thread keeps of its elements, four at a time: it is rarely more than one.
         auto keep_fours = [&](const float (&tq)[kVec], const float (&w)[kEl], float thr, uint32_t base) {
@@ -1481,8 +1481,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         keep_fours(tq, w, thr, base);
                 }
                 if (kSum && cfg.need_sum && seen > ninf) {
-                    // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest (and
-                    // of a shard record) every element; else of what is NOT collected (`thr` is the bound
+                    // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest
+                    // every element; else of what is NOT collected (`thr` is the bound
                     // the collection used): the collected elements get exact weights in the finish, so only the far tail
                     // carries the approximation. (A NaN makes the sum of every
                     // element one; such a row is left to the second launch.)
@@ -2016,14 +2016,23 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         unsigned long long* keys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
         const uint32_t n_all = min(s.ncand, scratch_cap);
         const float thr_final = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
+        double exact = 0.0; // the collected elements' weights; the streamed sum has the others
         for (uint32_t i = tid; i < n_all; i += kThreads) {
             const uint2 c = scratch[i];
+            const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table);
+            if (q == q)
+                exact += (double)q;
             if (__uint_as_float(c.x) >= thr_final) {
                 const uint32_t slot = atomicAdd(&s.nsurv, 1u);
                 if (slot < (uint32_t)kSortCap)
                     keys[slot] = ((unsigned long long)(~order_key(__uint_as_float(c.x))) << 32) | c.y;
             }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            exact += __shfl_xor_sync(0xffffffffu, exact, o);
+        if (lane == 0)
+            s.warp_sum[warp] = exact;
         __syncthreads();
         const uint32_t n_raw = min(s.nsurv, (uint32_t)kSortCap);
         const bool over = s.nsurv > (uint32_t)kSortCap || s.ncand > scratch_cap;
@@ -2058,6 +2067,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             uint32_t* hu = reinterpret_cast<uint32_t*>(rec);
             hf[0] = m;
             hu[1] = n_out | (over ? 0x80000000u : 0u) | ((n_cols > a.vp_k) ? 0x40000000u : 0u);
+            for (int i = 0; i < kThreads / 32; ++i)
+                total_approx += s.warp_sum[i];
             *reinterpret_cast<double*>(rec + 8) = total_approx;
         }
         for (uint32_t i = tid; i < a.vp_k; i += kThreads) {
