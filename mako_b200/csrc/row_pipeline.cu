@@ -68,6 +68,7 @@ constexpr uint32_t kBarSort = 3;         // named barrier of the sorting warps
 #endif
 constexpr int kPrefixTiles = MK_PREFIX_TILES;  // tiles all warps edit before the stream starts (their columns fit 16 bits)
 constexpr int kBins = 2048;     // bins of the top_k histogram (see hist_bin)
+constexpr uint32_t kHistWords = kBins + kBins / 32; // ... and the counts of their groups of 32
 
 // Shared memory of a CTA: this fixed head, then kDynBytes laid out per row. While the row streams: the tables the
 // row needs (generated-column bitmap, per-word ranks, counts; the top_k histogram) and, in all that is left, the
@@ -84,7 +85,6 @@ struct __align__(128) Smem {
     uint32_t nsurv;                 // candidates surviving the exact filter
     uint32_t abort_flag;
     uint32_t nan0;                  // column 0 (token id 0) is NaN: the reference's max_element keeps it
-    uint32_t hi_group;              // highest non-empty group of 32 histogram bins
     uint32_t first_tile_warps;      // reader warps whose first-tile maxima are in the histogram
     uint32_t n_final;
     uint32_t flags;
@@ -102,7 +102,7 @@ constexpr uint32_t kOffFinOrd = kOffFinWpre + kBmWords * 2u;      // kSortCap 16
 constexpr uint32_t kOffChain = kOffFinOrd + kSortCap * 2u;        // what the chains of a long list share
 using RowChain = ChainSmem<kThreads>;
 static_assert(kOffChain + sizeof(RowChain) <= kDynBytes, "finish layout fits");
-static_assert(kBins * 4u <= kBmWords * 4u, "mass histogram fits the finish bitmap area");
+static_assert(kHistWords <= (uint32_t)kBmWords, "the histogram fits the finish bitmap area");
 
 // Bins of the histogram that bounds the k-th largest element of a row: monotone in the float order, fine where
 // logits live — 32 bins per octave for magnitudes from 2^-10 to 2^8 (a bin is 2.2 % wide), everything smaller or
@@ -138,26 +138,46 @@ __device__ __forceinline__ float hist_bin_floor(uint32_t b)
     return -__uint_as_float((((q >> 5) + 117u) << 23) | ((q & 31u) << 18));
 }
 
-// The highest bin in which the count from the top reaches k, or -1: by one warp, 32 bins at a time from group `hi_group` down.
-__device__ __forceinline__ int hist_scan(const volatile uint32_t* hist, uint32_t hi_group, uint32_t k)
+// One element into the histogram: its bin, then the group of 32 bins it lies in (counts behind the bins).
+__device__ __forceinline__ void hist_enter(uint32_t* hist, float v)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t cum = 0;
-    int found = -1;
-    for (int g = (int)hi_group; g >= 0 && found < 0; --g) {
-        uint32_t suf = hist[g * 32 + lane]; // suffix sum over lanes >= lane
+    const uint32_t bin = hist_bin(v);
+    atomicAdd(&hist[bin], 1u);
+    atomicAdd(&hist[kBins + (bin >> 5)], 1u);
+}
+
+// The highest bin in which the count from the top reaches k, or -1. One warp: a suffix scan over the 64 groups, two a lane, then
+// one over the bins of the group found. (Group by group from the top, without their counts, it was 250 cycles a group and a dozen
+// of them: as much as reading the tile.) While others still enter elements the groups' counts may run ahead of the bins';
+// the answer is then -1 or a bin that holds its k elements all the same.
+__device__ __forceinline__ int hist_scan(const volatile uint32_t* hist, uint32_t k)
+{
+    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
+    const uint32_t low = hist[kBins + 2u * lane], high = hist[kBins + 2u * lane + 1u];
+    uint32_t suf = low + high; // lanes >= lane
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_down_sync(0xffffffffu, suf, o);
-            if ((int)lane + o < 32)
-                suf += y;
-        }
-        const uint32_t hit = __ballot_sync(0xffffffffu, cum + suf >= k);
-        if (hit)
-            found = g * 32 + (31 - __clz(hit));
-        cum += __shfl_sync(0xffffffffu, suf, 0);
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_down_sync(full, suf, o);
+        if ((int)lane + o < 32)
+            suf += y;
     }
-    return found;
+    const uint32_t reach = __ballot_sync(full, suf >= k);
+    if (!reach)
+        return -1;
+    const int top = 31 - __clz((int)reach);
+    uint32_t cum = suf - low - high; // above this lane's groups
+    const bool in_high = cum + high >= k;
+    const uint32_t g = __shfl_sync(full, 2u * lane + (in_high ? 1u : 0u), top);
+    cum = __shfl_sync(full, in_high ? cum : cum + high, top);
+    suf = hist[g * 32u + lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_down_sync(full, suf, o);
+        if ((int)lane + o < 32)
+            suf += y;
+    }
+    const uint32_t hit = __ballot_sync(full, cum + suf >= k);
+    return hit ? (int)(g * 32u) + 31 - __clz((int)hit) : -1;
 }
 
 __device__ __forceinline__ float warp_max(float v)
@@ -968,7 +988,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     uint32_t* const counts = reinterpret_cast<uint32_t*>(dyn + off); // by rank: occurrences, two per word
     off += use_table ? (uint32_t)kHistCap * 2u : 0u;
     uint32_t* const hist = reinterpret_cast<uint32_t*>(dyn + off);
-    off += cfg.hist_mode ? (uint32_t)kBins * 4u : 0u;
+    off += cfg.hist_mode ? kHistWords * 4u : 0u;
     off = (off + 127u) & ~127u;
     float* const ring = reinterpret_cast<float*>(dyn + off);
     const uint32_t n_stages = min((uint32_t)kMaxStages, (kDynBytes - off) / ((uint32_t)kTile * 4u)); // >= 4
@@ -989,7 +1009,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         s.nsurv = 0;
         s.abort_flag = 0;
         s.nan0 = 0;
-        s.hi_group = 0;
         s.first_tile_warps = 0;
         s.n_final = 0;
         s.flags = 0;
@@ -1002,7 +1021,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         for (uint32_t i = tid; i < kTile / 2; i += kThreads)
             cnt[i] = 0;
     if (cfg.hist_mode)
-        for (uint32_t i = tid; i < kBins; i += kThreads)
+        for (uint32_t i = tid; i < kHistWords; i += kThreads)
             hist[i] = 0;
     if (use_table) { // bitmap, ranks and counts are contiguous and 16-byte aligned: cleared with 128-bit stores
         uint4* const z = reinterpret_cast<uint4*>(bitmap);
@@ -1444,10 +1463,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     // a thread's 16 columns).
                     thr = fmaxf(thr, key_to_float(*(volatile uint32_t*)&s.thr_topk_key));
                     if (tm >= thr) {
-                        const uint32_t bin = hist_bin(tm);
-                        atomicAdd(&hist[bin], 1u);
-                        if ((bin >> 5) > *(volatile uint32_t*)&s.hi_group)
-                            atomicMax(&s.hi_group, bin >> 5);
+                        hist_enter(hist, tm);
                     }
                     __syncwarp();
                     // The first tile would be kept whole (no bound exists while it is read), so its 256 thread maxima
@@ -1465,10 +1481,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     }
                     // One reader warp rescans the histogram and raises the bound, after every tile while the row is young and
                     // then after every fourth (the bound of t tiles lets k / t elements of a later tile through; a scan is
-                    // a chain of a dozen dependent shared loads and shuffle rounds); nobody waits for it. Counts only grow and every count is an element at or above its bin's edge, so a bound read from a
+                    // two chains of five shuffles); nobody waits for it. Counts only grow and every count is an element at or above its bin's edge, so a bound read from a
                     // histogram that other warps are still adding to has its k elements all the same.
                     if (t == 0 || (rwarp == (t % (kReaders / 32)) && (t < 8 || (t & 3u) == 0u))) {
-                        const int found = hist_scan(hist, *(volatile uint32_t*)&s.hi_group, cfg.hist_k);
+                        const int found = hist_scan(hist, cfg.hist_k);
                         // the lowest key of a bin is its smallest float; bin 0 (NaN keys) is never a bound
                         if (lane == 0 && found > 0)
                             atomicMax(&s.thr_topk_key, order_key(hist_bin_floor((uint32_t)found)));
@@ -1625,7 +1641,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         uint32_t* const n_of = reinterpret_cast<uint32_t*>(dyn + kOffFinOrd);
         uint32_t* const hist2 = reinterpret_cast<uint32_t*>(dyn + kOffFinBitmap);
         if (cfg.hist_mode)
-            for (uint32_t i = tid; i < (uint32_t)kBins; i += kThreads)
+            for (uint32_t i = tid; i < kHistWords; i += kThreads)
                 hist2[i] = 0u;
         if (warp == 0) {
             unsigned long long best_key = 0ull;
@@ -1656,7 +1672,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 s.abort_flag = bits & 2u;
                 s.warp_sum[0] = sum;
                 s.ncand = 0u;
-                s.hi_group = 0u;
                 s.thr_topk_key = order_key(-FLT_MAX);
                 s.n_final = 0u;
                 again[0] = 0u;
@@ -1703,15 +1718,12 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         if (cfg.hist_mode) {
             for_each_kept([&](const uint2& c, uint32_t) {
                 const float v = __uint_as_float(c.x);
-                if (v == v) {
-                    const uint32_t bin = hist_bin(v);
-                    atomicAdd(&hist2[bin], 1u);
-                    atomicMax(&s.hi_group, bin >> 5);
-                }
+                if (v == v)
+                    hist_enter(hist2, v);
             });
             __syncthreads();
             if (warp == 0) {
-                const int found = hist_scan(hist2, s.hi_group, cfg.hist_k);
+                const int found = hist_scan(hist2, cfg.hist_k);
                 if (lane == 0 && found > 0)
                     s.thr_topk_key = order_key(hist_bin_floor((uint32_t)found));
             }
