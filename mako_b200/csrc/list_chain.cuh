@@ -5,18 +5,16 @@
 // Why that is possible: while the running value stays within one binade [2^e, 2^(e+1)) it is a whole number k of units
 // u = 2^(e-23), and rounding k*u + q to the nearest unit adds a whole number of units that depends on q alone — except
 // for an exact tie, which goes to the even neighbour and so depends on the parity of k as well. A run of candidates is
-// therefore a function of the parity it starts with: two increments. Such functions compose, so a scan over the threads
-// gives every thread the value its run starts with. The increments come from the float adder itself, by adding the run to
+// therefore a function of the parity it starts with: two increments. Such functions compose, so a scan over the lanes of
+// a warp gives every lane the value its run starts with. The increments come from the float adder itself, by adding the run to
 // the smallest even and the smallest odd value of the binade (the largest two for the walk). A run that leaves the
-// binade, or in which the walk could end, is taken element by element by its thread; everything before it stands, and the
-// next round starts behind it with the new unit. A value crosses at most a few dozen binades.
+// binade, or in which the walk could end, is taken element by element; everything before it stands, and the next round
+// starts behind it with the new unit. A value crosses at most a few dozen binades.
 //
 // Ties are rare: where no run of a round has one, the increments are plain numbers, and as long as their sum stays inside the binade
-// (and, in a walk, above the largest weight) a round is one reduction. The scan is for the others.
-//
-// Rounds are taken by one warp (256 candidates) where the value crosses binades every few candidates — the start of a total,
-// the end of a walk — and by the whole CTA otherwise: what bounds both is the latency and the issue slots of a round's scan,
-// not the number of candidates.
+// (and, in a walk, above the largest weight) a round is one reduction. Such rounds are taken by the whole CTA, up to the first
+// warp's share that is not like that; one warp takes the others (256 candidates). What bounds both is a round's latency, not
+// the number of candidates.
 #pragma once
 #include <cstdint>
 
@@ -31,13 +29,12 @@ constexpr float kChainFloor = 0x1p-100f; // smaller running values are taken ele
 
 template <int kThreads>
 struct ChainSmem {
-    uint32_t warp0[kThreads / 32], warp1[kThreads / 32]; // increments of whole warps, by starting parity
     uint32_t sum[2][kThreads / 32], top[2][kThreads / 32]; // by round parity: a warp's units (bit 31: not a plain number), its largest weight
-    uint32_t bad[2];       // first thread whose run leaves the binade (or may end the walk), by round parity
     float value;           // the running value and the place it stands at
     uint32_t pos;
     uint32_t hit;          // the walk's end
     float r_hit, q_hit;
+    uint32_t first, last;  // for the caller: the list's ends that could win
 };
 
 // 2^e as a float, for -126 <= e <= 127.
@@ -157,10 +154,8 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
     constexpr uint32_t kWarps = kThreads / 32, none = 0xffffffffu;
     const uint32_t full = 0xffffffffu, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint32_t pos = 0, round = 0;
-    if (tid == 0) {
-        cs.bad[0] = cs.bad[1] = (uint32_t)kThreads;
+    if (tid == 0)
         cs.hit = none;
-    }
     __syncthreads();
     while (pos < n) {
         if (warp == 0) { // every lane knows value and pos
@@ -238,71 +233,42 @@ __device__ __forceinline__ float chain(ChainSmem<kThreads>& cs, const float* q, 
         __syncthreads();
         value = cs.value;
         pos = cs.pos;
-        // rounds of the whole CTA, until one of them crosses a binade; each has a barrier between the reads above and its
-        // first write to the same places
+        // Rounds of the whole CTA, a barrier each, for as long as no warp's runs cross a binade or hold a tie; warp 0 goes on
+        // at the first that does.
         while (pos < n && value >= kChainFloor) {
             const Binade<kDown> b(value);
-            const uint32_t i0 = pos + tid * kRun;
             uint32_t u0, u1;
             float top;
-            b.run(q, i0, n, u0, u1, top);
+            b.run(q, pos + tid * kRun, n, u0, u1, top);
             const uint32_t slot = round & 1u;
             ++round;
-            {
-                const bool plain = __all_sync(full, u0 == u1);
-                const uint32_t sum = min(__reduce_add_sync(full, u0), kUnitCap);
-                const uint32_t largest = kDown ? __reduce_max_sync(full, __float_as_uint(top)) : 0u;
-                if (lane == 0u) {
-                    cs.sum[slot][warp] = sum | (plain ? 0u : 0x80000000u);
-                    cs.top[slot][warp] = largest;
-                }
+            const bool plain = __all_sync(full, u0 == u1);
+            const uint32_t own = min(__reduce_add_sync(full, u0), kUnitCap);
+            const uint32_t largest = kDown ? __reduce_max_sync(full, __float_as_uint(top)) : 0u;
+            if (lane == 0u) {
+                cs.sum[slot][warp] = own | (plain ? 0u : 0x80000000u);
+                cs.top[slot][warp] = largest;
             }
             __syncthreads();
-            if (tid == 0)
-                cs.bad[slot ^ 1u] = (uint32_t)kThreads; // the next round's: everyone is done with the last one's
-            {
-                const uint32_t sum = (lane < kWarps) ? cs.sum[slot][lane] : 0u, largest = (lane < kWarps) ? cs.top[slot][lane] : 0u;
-                if (!__any_sync(full, sum >> 31)) {
-                    const uint32_t end = b.after(b.k, __reduce_add_sync(full, sum));
-                    if (!b.bad(end, kDown ? __uint_as_float(__reduce_max_sync(full, largest)) : 0.0f)) {
-                        value = (float)end * b.unit;
-                        pos += (uint32_t)kThreads * kRun;
-                        continue;
-                    }
-                }
+            // lane w: warp w's units, and where they take the value
+            const uint32_t entry = (lane < kWarps) ? cs.sum[slot][lane] : 0u, units = entry & 0x7fffffffu;
+            const float top_w = (kDown && lane < kWarps) ? __uint_as_float(cs.top[slot][lane]) : 0.0f;
+            uint32_t inc = units;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(full, inc, o);
+                if ((int)lane >= o)
+                    inc += y;
             }
-            uint32_t f0 = u0, f1 = u1;
-            warp_compose(f0, f1);
-            if (lane == 31u) {
-                cs.warp0[warp] = f0;
-                cs.warp1[warp] = f1;
-            }
-            uint32_t e0 = __shfl_up_sync(full, f0, 1), e1 = __shfl_up_sync(full, f1, 1);
-            if (lane == 0u)
-                e0 = e1 = 0u;
-            __syncthreads();
-            uint32_t w0 = (lane < kWarps) ? cs.warp0[lane] : 0u, w1 = (lane < kWarps) ? cs.warp1[lane] : 0u;
-            warp_compose(w0, w1);
-            uint32_t before = __shfl_sync(full, (b.k & 1u) ? w1 : w0, (int)((warp + 31u) & 31u));
-            if (warp == 0u)
-                before = 0u;
-            before = min(before + (((b.k + before) & 1u) ? e1 : e0), 2u * kUnitCap);
-            const uint32_t start = b.after(b.k, before), end = b.after(start, (start & 1u) ? u1 : u0);
-            if (b.bad(end, top))
-                atomicMin(&cs.bad[slot], tid);
-            else if (tid == (uint32_t)kThreads - 1u)
-                cs.value = (float)end * b.unit;
-            __syncthreads();
-            const uint32_t f = cs.bad[slot];
-            if (f < (uint32_t)kThreads) { // warp 0 goes on at this thread's run
-                if (tid == f)
-                    cs.value = (float)start * b.unit;
-                pos += f * kRun;
-                __syncthreads();
-                value = cs.value;
+            const uint32_t start = b.after(b.k, inc - units), end = b.after(b.k, inc);
+            const uint32_t stops = __ballot_sync(full, (entry >> 31) || b.bad(end, top_w));
+            if (stops) {
+                const int f = __ffs((int)stops) - 1;
+                value = (float)__shfl_sync(full, start, f) * b.unit;
+                pos += (uint32_t)f * 32u * kRun;
                 break;
             }
-            value = cs.value;
+            value = (float)__shfl_sync(full, end, 31) * b.unit;
             pos += (uint32_t)kThreads * kRun;
         }
         __syncthreads(); // everyone has read the round's results before warp 0 writes there again

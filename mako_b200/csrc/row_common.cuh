@@ -178,23 +178,23 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, float* q, uin
     // the first and the last candidate that could win: the edges of the CDF have no neighbour beyond them
     __syncthreads();
     if (threadIdx.x == 0) {
-        cs.warp0[0] = none;
-        cs.warp1[0] = 0u;
+        cs.first = none;
+        cs.last = 0u;
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += kThreads)
         if (q[i] > 0.0f) {
-            atomicMin(&cs.warp0[0], i);
+            atomicMin(&cs.first, i);
             break;
         }
     for (uint32_t i = threadIdx.x; i < n; i += kThreads)
         if (q[n - 1u - i] > 0.0f) {
-            atomicMax(&cs.warp1[0], n - 1u - i);
+            atomicMax(&cs.last, n - 1u - i);
             break;
         }
     __syncthreads();
-    first = cs.warp0[0];
-    last = cs.warp1[0];
+    first = cs.first;
+    last = cs.last;
     if (threadIdx.x != 0)
         return;
     if (tok == -2) {

@@ -1334,7 +1334,25 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         }
                 }
         };
-        // The loop over the tiles is compiled four times for each kind of launch, with the mask, the top_k histogram and the streamed sum
+        // Where several lanes have something to keep (an allowed row, a flat one, or the first tiles of any row, before its bound is
+        // known), the fours of all of them would be run through one after the other, each waiting for its own slot: there a
+        // lane counts its elements and takes their slots at once.
+        auto keep_many = [&](const float (&w)[kEl], float thr, uint32_t base) {
+            uint32_t bits = 0u;
+#pragma unroll
+            for (int e = 0; e < kEl; ++e)
+                bits |= (w[e] >= thr) ? 1u << e : 0u;
+            const uint32_t mine = (uint32_t)__popc(bits), slot = atomicAdd(&s.ncand, mine);
+            if (slot + mine <= scratch_cap) {
+                uint2* at = scratch + slot;
+                const uint32_t col = base + rt * 4;
+#pragma unroll
+                for (int e = 0; e < kEl; ++e)
+                    if ((bits >> e) & 1u)
+                        *at++ = make_uint2(__float_as_uint(w[e]), col + (e >> 2) * 1024 + (e & 3));
+            }
+        };
+        // The loop over the tiles is compiled five times for each kind of launch, with the mask, the top_k histogram and the streamed sum
         // compiled in or out: a row runs a variant that holds little beyond its own work. (One loop with all
         // three as run-time branches costs the common penalised row 12 % of its launch time, and all eight
         // combinations cost it 3 % again: the size of the code matters, executed or not.)
@@ -1493,8 +1511,13 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             thr = fmaxf(thr, key_to_float(*(volatile uint32_t*)&s.thr_topk_key));
                         }
                     }
-                    if (collect && tm >= thr)
+                    const uint32_t lanes = kAgg ? __ballot_sync(0xffffffffu, collect && tm >= thr) : 0u;
+                    if (kAgg && __popc(lanes) >= 3) {
+                        if (tm >= thr)
+                            keep_many(w, thr, base);
+                    } else if (collect && tm >= thr) {
                         keep_fours(tq, w, thr, base);
+                    }
                 }
                 if (kSum && cfg.need_sum && seen > ninf) {
                     // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest
@@ -1517,24 +1540,9 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 if (!(kHist && cfg.hist_mode) && collect) {
                     const bool some = tm >= thr;
                     const uint32_t lanes = kAgg ? __ballot_sync(0xffffffffu, some) : 0u;
-                    if (kAgg && __popc(lanes) >= 2) {
-                        // Many lanes have something to keep (an allowed row, a flat one, or the first tiles of any row,
-                        // before the maximum is known): one slot range a lane instead of one atomic an element.
-                        uint32_t mine = 0;
-#pragma unroll
-                        for (int e = 0; e < kEl; ++e)
-                            mine += (w[e] >= thr) ? 1u : 0u;
-                        uint32_t slot = some ? atomicAdd(&s.ncand, mine) : 0u;
-                        if (some) {
-#pragma unroll
-                            for (int e = 0; e < kEl; ++e)
-                                if (w[e] >= thr) {
-                                    if (slot < scratch_cap)
-                                        scratch[slot] = make_uint2(__float_as_uint(w[e]),
-                                                                   base + (e >> 2) * 1024 + rt * 4 + (e & 3));
-                                    ++slot;
-                                }
-                        }
+                    if (kAgg && __popc(lanes) >= 3) {
+                        if (some)
+                            keep_many(w, thr, base);
                     } else if (some) {
                         keep_fours(tq, w, thr, base);
                     }
@@ -1545,13 +1553,15 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         using F = std::false_type;
         using M = std::integral_constant<bool, kMasked>;
         if (!cfg.hist_mode && !cfg.need_sum)
-            read_tiles(M{}, F{}, F{}, M{}); // penalties, min_p, greedy, a pure draw: nothing but maximum and bound
+            read_tiles(M{}, F{}, F{}, T{}); // penalties, min_p, greedy, a pure draw: nothing but maximum and bound
         else if (!cfg.need_sum)
-            read_tiles(M{}, T{}, F{}, F{}); // top_k
+            read_tiles(M{}, T{}, F{}, T{}); // top_k
         else if (a.pass == 1)
             read_tiles(M{}, F{}, T{}, T{}); // top_p alone, second pass: a third of a flat row is kept
+        else if (!kSplit && mode == kModeVpLocal)
+            read_tiles(M{}, T{}, T{}, T{}); // shard records
         else
-            read_tiles(M{}, T{}, T{}, F{}); // top_p alone (with its first-launch histogram), shard records
+            read_tiles(M{}, T{}, T{}, F{}); // top_p alone, with its first launch's histogram: keeps few, and loses 2 % to the code
     }
     __syncthreads();
 
