@@ -26,7 +26,7 @@ namespace {
 constexpr int kFlatThreads = 1024;
 constexpr uint32_t kFlatWarps = kFlatThreads / 32;
 constexpr uint32_t kClasses = 512;          // weight classes: sixteenths of an octave below the maximum's weight
-constexpr uint32_t kSpecialCap = 4096;      // generated and biased columns of a row (history entries + bias entries)
+constexpr uint32_t kSpecialCap = kFlatMaxEdits; // generated and biased columns of a row (history entries + bias entries)
 constexpr uint32_t kFlatVocab = 163840;
 constexpr uint32_t kFlatBmWords = kFlatVocab / 32 + 2;
 constexpr uint32_t kMaxBuckets = 8192;
@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
         s.exp2_table[tid] = kExp2Tab[tid];
     uint32_t seen = 0; // marked rows of earlier chunks
     for (uint32_t chunk = 0; chunk < batch; chunk += (uint32_t)kFlatThreads) {
-        // which marked rows of this chunk are this CTA's
+        // Which marked rows of this chunk are this CTA's. Every CTA counts the marks itself, whenever it comes to run, so they
+        // stand until the next call's first launch.
         const uint32_t r_mine = chunk + tid;
         bool marked = false;
         if (r_mine < batch)
@@ -207,8 +208,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             const int32_t* __restrict__ hrow = a.history ? a.history + (size_t)row * a.history_ld : nullptr;
             const float u_row = a.u ? __ldg(a.u + row) : 0.0f, u2_row = a.u2 ? __ldg(a.u2 + row) : 0.0f;
             const int32_t draft_row = a.draft ? __ldg(a.draft + row) : -1;
-            if (hlen + nb > kSpecialCap)
-                continue; // stays marked: the row pipeline's own second launch takes it
+            if (!flat_row_takes(a, hlen, nb))
+                continue; // the row pipeline's own second launch takes it
             const bool special = hlen > 0u || nb > 0u;
             // Four places of the row: fetched (nothing is, for a group that reaches past the row's ends), and edited; those that
             // are not the row's own, not allowed, or edited apart read as -inf.
@@ -715,9 +716,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                               a.cand_cap, a.id_offset, a.timing, a.mode};
             draw_long<kFlatThreads>(s.chain, q, n_take, n_take, draft_idx, row, flags, u_row, u2_row, draft_row, o,
                                     [&](uint32_t i) -> uint32_t { return (uint32_t)(keys[i] & 0xffffffffull); });
-            if (tid == 0)
-                state[0] = 0u;
-            __syncthreads();
+            __syncthreads(); // (the mark stays: CTAs that start later count it too)
         }
     }
 }

@@ -975,7 +975,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             return;
         }
     }
-    if (a.pass == 1 && again[0] == 0u)
+    if (a.pass == 1 && (again[0] == 0u || flat_row_takes(a, hlen, nb)))
         return;
     // ---- shared-memory layout of the streaming phase ---------------------------------------------------------------
     const uint32_t bm_words = (V + 31u) / 32u;
@@ -2597,6 +2597,7 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     lc.numAttrs = a.overlap != MK_OVERLAP_OFF ? 1u : 0u;
     RowKernelArgs first = a;
     first.pass = 0;
+    first.flat_take = flat_rows_take(a);
     const bool spec = a.spec_n_pos != 0u;
     auto launch = [&](const RowKernelArgs& x) {
         if (spec)
@@ -2621,13 +2622,12 @@ cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream
     const bool host_need_sum = !(p.temperature <= 0.0f) && p.top_p < 1.0f && !(minp_eff > 0.0f) &&
                                !(p.top_k > 0 && p.top_k < a.n_vocab);
     if (a.mode != kModeVpLocal && kNucleusGuess < a.n_vocab && (a.params_dev || host_need_sum)) {
-        const int take = flat_rows_take(a);
-        if (take) {
-            e = launch_flat_rows(a, batch, stream);
-            if (e != cudaSuccess || take == 2)
+        if (first.flat_take) {
+            e = launch_flat_rows(first, batch, stream);
+            if (e != cudaSuccess || first.flat_take == 2)
                 return e;
         }
-        RowKernelArgs second = a; // what is left
+        RowKernelArgs second = first; // what is left
         second.pass = 1;
         second.split_w = 0;
         e = launch(second);

@@ -64,6 +64,7 @@ struct RowKernelArgs {
     unsigned long long* timing; // optional [batch][64] ns timestamps (slots: see mk_debug_set_timing)
     int mode;
     int pass;              // 0: first launch; 1: second pass, only the rows that asked for it (set by launch_row_kernel)
+    int flat_take;         // which marked rows the flat rows' kernel takes (flat_rows_take; set by launch_row_kernel)
     int overlap;           // MK_OVERLAP_*: launch behind the previous kernel of the stream programmatically
     // a speculative round: row = sequence * spec_n_pos + position (0: off); history and history_len are per sequence
     uint32_t spec_n_pos;
@@ -79,15 +80,22 @@ struct RowKernelArgs {
 };
 
 // Words of handle scratch per row: 4 per column of capacity, then 4 of per-row state (word 0: the row asks for the
-// second pass; with it word 1 its maximum, words 2-3 its total weight as a double).
+// second launch; with it word 1 its maximum, words 2-3 its total weight as a double). The first launch writes word 0 on every
+// call, for every row; the launches behind it only read it: the flat rows' CTAs each count the marks for themselves.
 __host__ __device__ inline size_t row_scratch_words(uint32_t cap) { return 4ull * cap + 4ull; }
 
 size_t row_kernel_smem_bytes();
 cudaError_t launch_row_kernel(const RowKernelArgs& a, uint32_t batch, cudaStream_t stream);
 
 // The rows of `a` that the first launch marked (top_p alone, nucleus not settled), one CTA of 1024 threads each.
-// flat_rows_take says which rows that can be: 2 all, 1 those whose history is short enough (the others stay marked), 0 none.
+// flat_rows_take says which rows that can be: 2 all, 1 those with few enough edits (the row pipeline's own second launch takes
+// the others), 0 none; flat_row_takes which row it is.
+constexpr uint32_t kFlatMaxEdits = 4096; // history entries and bias entries of a row
 int flat_rows_take(const RowKernelArgs& a);
+__host__ __device__ inline bool flat_row_takes(const RowKernelArgs& a, uint32_t n_history, uint32_t n_bias)
+{
+    return a.flat_take != 0 && n_history + n_bias <= kFlatMaxEdits;
+}
 cudaError_t launch_flat_rows(const RowKernelArgs& a, uint32_t batch, cudaStream_t stream);
 
 struct VpMergeArgs {

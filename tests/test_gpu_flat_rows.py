@@ -60,3 +60,60 @@ def test_flat_rows_equal_the_reference(gpu_sampler_factory, ref, name):
         if not ver.flags[b].item() & 0x2:
             want = ref.verify(p, inp.logits[b], int(draft[b]), inp.u2[b], inp.u3[b], **inp.row_kwargs(b))
             assert (ver.token[b].item(), bool(ver.accepted[b].item())) == (want[0], bool(want[1])), f"row {b}"
+
+
+def _flat_inputs(seed, batch, v, settled_every):
+    """Rows of nuclei of some thousand tokens, with a peaked one (settled by the first launch) after every few of them."""
+    inp = Inputs(seed, batch, v, n_spikes=0, sigma=0.4)
+    if settled_every:
+        inp.logits[::settled_every, 7] = 25.0
+    return inp
+
+
+@pytest.mark.parametrize("batch,settled_every", [(149, 0), (320, 3), (1025, 0), (2100, 5)])
+def test_every_marked_row_is_taken_once(gpu_sampler_factory, ref, batch, settled_every):
+    """More marked rows than CTAs, and more rows than a CTA looks at in one go: each is drawn, none twice, call after call."""
+    import torch
+    v, p = 4099, SamplingParams(temperature=1.0, top_p=0.9)
+    inp = _flat_inputs(9000 + batch, batch, v, settled_every)
+    g = inp.to_gpu()
+    s = gpu_sampler_factory(v, batch, 16)
+    want = oracle_sample_rows(ref, p, inp, cap=16)
+    assert sum(w["n_cand"] > 1000 for w in want) >= batch // 2
+    for call in range(3):
+        s.token.fill_(-7)
+        s.n_cand.zero_()
+        res = s.sample(g["logits"], p, g["u"])
+        torch.cuda.synchronize()
+        tok, n, flags = res.token.cpu().numpy(), res.n_cand.cpu().numpy(), res.flags.cpu().numpy()
+        ids, qs = res.cand_ids.cpu().numpy(), res.cand_q.cpu().numpy()
+        assert (tok >= 0).all()
+        for b, w in enumerate(want):
+            if flags[b] & 0x2:
+                continue
+            k = min(w["n_cand"], 16)
+            assert (tok[b], n[b]) == (w["token"], w["n_cand"]), f"call {call} row {b}"
+            assert np.array_equal(ids[b, :k], w["cand_ids"][:k]), f"call {call} row {b}"
+            assert np.array_equal(qs[b, :k].view(np.uint32), w["cand_q"][:k].view(np.uint32)), f"call {call} row {b}"
+
+
+def test_two_sets_of_marked_rows_side_by_side(gpu_sampler_factory, ref):
+    """p/q verification of flat rows: the drafter's and the target's marked rows are taken by two grids that compete for the
+    device, so the later CTAs of one start when its first rows are done."""
+    import torch
+    from mako_b200 import synth
+    v, batch, p = 4099, 320, SamplingParams(temperature=1.0, top_p=0.9)
+    inp = _flat_inputs(9400, batch, v, 0)
+    lq = synth.add_noise(9400, inp.logits, v, sigma=0.3)
+    g, lq_dev = inp.to_gpu(), torch.from_numpy(lq).cuda()
+    s = gpu_sampler_factory(v, batch, 16)
+    want = [ref.verify_pq(p, inp.logits[b], lq[b], inp.u[b], inp.u2[b], inp.u3[b]) for b in range(batch)]
+    for call in range(3):
+        res = s.verify_pq(g["logits"], lq_dev, p, g["u"], g["u2"], g["u3"])
+        torch.cuda.synchronize()
+        d, acc, tok, flags = (t.cpu().numpy() for t in (res.draft_token, res.accepted, res.token, res.flags))
+        assert not (flags & 0x50).any() and (tok >= 0).all()
+        for b in range(batch):
+            if not flags[b] & 0x2:
+                assert (d[b], bool(acc[b]), tok[b]) == want[b], f"call {call} row {b}"
+    assert 0 < sum(w[1] for w in want) < batch
