@@ -87,6 +87,7 @@ struct __align__(128) Smem {
     uint32_t nan0;                  // column 0 (token id 0) is NaN: the reference's max_element keeps it
     uint32_t first_tile_warps;      // reader warps whose first-tile maxima are in the histogram
     uint32_t n_final;
+    uint32_t last_slice;            // split launch: this CTA arrived last and goes on with the row
     uint32_t flags;
     uint32_t n_distinct;            // distinct special columns (generated or biased)
     uint32_t n_own;                 // generated columns within the first tiles (edited by all warps)
@@ -1640,12 +1641,12 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             parts[blockIdx.y] = p;
             __threadfence();
             const uint32_t ticket = atomicAdd(&a.tickets[row], 1u);
-            s.n_final = (ticket == n_slices - 1u) ? 1u : 0u;
-            if (s.n_final)
+            s.last_slice = (ticket == n_slices - 1u) ? 1u : 0u;
+            if (s.last_slice)
                 a.tickets[row] = 0u; // for the next launch
         }
         __syncthreads();
-        if (!s.n_final)
+        if (!s.last_slice) // (written nowhere else: a warp that reads late finds the same)
             return;
         __threadfence();
         uint32_t* const n_of = reinterpret_cast<uint32_t*>(dyn + kOffFinOrd);
@@ -1683,7 +1684,6 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 s.warp_sum[0] = sum;
                 s.ncand = 0u;
                 s.thr_topk_key = order_key(-FLT_MAX);
-                s.n_final = 0u;
                 again[0] = 0u;
             }
         }

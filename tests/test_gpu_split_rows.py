@@ -1,6 +1,7 @@
 """Rows split over several CTAs give what one CTA per row gives, for every kind of bound the slices keep their elements by, on
 slices of one tile and of several, call after call on one handle (the slices' tickets start over by themselves)."""
 import pytest
+import torch
 
 from helpers import Inputs
 from mako_b200.sampler import SamplingParams
@@ -21,7 +22,6 @@ KINDS = {
 @pytest.mark.parametrize("batch", [1, 9, 40, 64])
 @pytest.mark.parametrize("masked", [False, True])
 def test_split_rows_equal_whole_rows(gpu_sampler_factory, batch, masked):
-    import torch
     v, cap = 100003, 64  # 25 tiles, rows on every alignment
     inp = Inputs(500 + batch, batch, v, n_history=700, n_bias=16, with_mask=masked)
     g = inp.to_gpu()
@@ -46,3 +46,82 @@ def test_split_rows_equal_whole_rows(gpu_sampler_factory, batch, masked):
             sure = (banded == 0).view(-1, *([1] * (a.dim() - 1))).expand_as(a)
             assert torch.equal(a[sure], b[sure]), name
             assert torch.equal(a, c), name
+
+
+def _copies(r):
+    """A result's values as they are now (its tensors are views of the handle's buffers, which the next call writes again)."""
+    keep = None if r.cand_ids is None else torch.arange(r.cand_ids.shape[1], device="cuda") < r.n_cand[:, None]
+    return [r.token.clone(), r.prob.clone(), r.n_cand.clone()] + ([] if keep is None else [r.cand_ids * keep, r.cand_q * keep])
+
+
+def _same_where_sure(a, b, sure, what):
+    for x, y in zip(a, b):
+        at = sure.view(-1, *([1] * (x.dim() - 1))).expand_as(x)
+        assert torch.equal(x[at], y[at]), what
+
+
+@pytest.mark.parametrize("overlap", [1, 2])
+def test_split_rows_behind_one_another(overlap):
+    """Launches that follow one another programmatically share the handle's tickets and parts: 60 in a row, of other shapes in
+    turn, each equal to whole rows in plain stream order."""
+    from mako_b200 import BatchSampler
+    v, cap = 100003, 64
+    sets = [(Inputs(800 + b, b, v, n_history=300), b) for b in (1, 5, 48)]
+    gs = [i.to_gpu() for i, _ in sets]
+    whole, split = BatchSampler(v, 48, 0, cap), BatchSampler(v, 48, 0, cap)
+    whole.set_split(False)
+    split.set_overlap(overlap)
+    for name in ("top_k_40", "min_p", "top_p"):
+        want = []
+        for g in gs:
+            r = whole.sample(g["logits"], KINDS[name], g["u"], **g["kw"])
+            want.append((_copies(r), r.flags.clone()))
+        torch.cuda.synchronize()
+        got = []
+        for call in range(60):
+            g = gs[call % 3]
+            r = split.sample(g["logits"], KINDS[name], g["u"], **g["kw"])
+            got.append((_copies(r), r.flags.clone()))
+        torch.cuda.synchronize()
+        for call, (g, f) in enumerate(got):
+            w, wf = want[call % 3]
+            _same_where_sure(g, w, ((f | wf) & 0x2) == 0, f"{name}, call {call}")
+
+
+def test_split_rows_with_parameters_of_their_own(gpu_sampler_factory):
+    from mako_b200.sampler import pack_params
+    v, cap, batch = 100003, 64, 14
+    inp = Inputs(860, batch, v, n_history=700, n_bias=16)
+    g = inp.to_gpu()
+    ps = list(KINDS.values())
+    params = torch.from_numpy(pack_params([ps[b % len(ps)] for b in range(batch)])).cuda()
+    s = gpu_sampler_factory(v, 64, cap)
+    got = []
+    for on in (True, False):
+        s.set_split(on)
+        r = s.sample(g["logits"], params, g["u"], **g["kw"])
+        got.append((_copies(r), r.flags.clone()))
+    s.set_split(True)
+    _same_where_sure(got[0][0], got[1][0], ((got[0][1] | got[1][1]) & 0x2) == 0, "per-row parameters")
+
+
+@pytest.mark.parametrize("batch", [1, 24, 148])
+@pytest.mark.parametrize("kind", ["top_k_40", "top_p"])
+def test_split_rows_of_both_distributions(gpu_sampler_factory, batch, kind):
+    """p/q verification splits two row sets at a time, each with tickets of its own."""
+    from mako_b200 import synth
+    v = 100003
+    inp = Inputs(870 + batch, batch, v)
+    g = inp.to_gpu()
+    lq = torch.from_numpy(synth.add_noise(870, inp.logits, v, sigma=1.0)).cuda()
+    s = gpu_sampler_factory(v, 148, 0)
+    got = []
+    for on in (True, False, True):
+        s.set_split(on)
+        r = s.verify_pq(g["logits"], lq, KINDS[kind], g["u"], g["u2"], g["u3"])
+        got.append(([r.draft_token.clone(), r.accepted.clone(), r.token.clone()], r.flags.clone()))
+    s.set_split(True)
+    sure = ((got[0][1] | got[1][1] | got[2][1]) & 0x2) == 0
+    assert sure.any()
+    _same_where_sure(got[0][0], got[1][0], sure, "split against whole")
+    _same_where_sure(got[0][0], got[2][0], sure, "split again")
