@@ -293,10 +293,15 @@ int mk_sampler_create(mk_sampler** out, int device, uint32_t n_vocab, uint32_t m
             at += up(x.bytes);
         }
         s->split_tickets = reinterpret_cast<uint32_t*>(s->pick_best + mk::kDraftPickMaxSeq + 1);
-        e = cudaMemset(s->pick_best, 0, zero_bytes);
     }
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking);
+    // The counters are zero before the handle is handed out: a memset of the default stream would wait for what is queued there, and
+    // a caller's own stream would not wait for it.
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(s->pick_best, 0, zero_bytes, s->own_stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(s->own_stream);
     if (e == cudaSuccess)
         e = cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess)

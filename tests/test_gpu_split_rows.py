@@ -125,3 +125,25 @@ def test_split_rows_of_both_distributions(gpu_sampler_factory, batch, kind):
     assert sure.any()
     _same_where_sure(got[0][0], got[1][0], sure, "split against whole")
     _same_where_sure(got[0][0], got[2][0], sure, "split again")
+
+
+def test_a_new_handle_is_ready_on_any_stream(ref):
+    """Created while the default stream is busy, on memory that was something else before, and used at once on a stream that does
+    not wait for the default one: the first call's tickets are zero all the same."""
+    from mako_b200 import BatchSampler
+    from helpers import oracle_sample_rows
+    v, batch, p = 151552, 4, KINDS["top_k_40"]
+    inp = Inputs(880, batch, v)
+    g = inp.to_gpu()
+    want = [w["token"] for w in oracle_sample_rows(ref, p, inp)]
+    junk = torch.full((1 << 28,), -1, dtype=torch.int32, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    del junk
+    torch.cuda.empty_cache()
+    torch.cuda._sleep(200_000_000)  # the default stream is busy for some 100 ms
+    with torch.cuda.stream(side):
+        s = BatchSampler(v, batch, 0)
+        tok = s.sample(g["logits"], p, g["u"]).token.clone()
+    side.synchronize()
+    assert tok.tolist() == want
