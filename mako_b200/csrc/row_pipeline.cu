@@ -1318,11 +1318,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
         const float c2 = cfg.inv_t * 1.4426950408889634f;
         const float ninf = -__int_as_float(0x7f800000);
         const bool collect = !cfg.greedy || mode == kModeVpLocal;
-        // A nucleus that is to be found among the few largest: the streamed sum takes every element.
-        const bool sum_all = cfg.optimistic;
         const bool hist_bound_alone = !(cfg.minp_eff > 0.0f) && cfg.hist_k <= kVpMaxK + 1u;
-        // What a thread keeps of its elements, four at a time: it is rarely more than one.
-        auto keep_fours = [&](const float (&tq)[kVec], const float (&w)[kEl], float thr, uint32_t base) {
+        // What a thread keeps of its elements, four at a time: it is rarely more than one. `take_out`: the kept ones read as -inf
+        // afterwards, which weighs nothing in a sum over all sixteen.
+        auto keep_fours = [&](const float (&tq)[kVec], float (&w)[kEl], float thr, uint32_t base, auto take_out) {
 #pragma unroll
             for (int j = 0; j < kVec; ++j)
                 if (tq[j] >= thr) {
@@ -1332,6 +1331,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             const uint32_t slot = atomicAdd(&s.ncand, 1u);
                             if (slot < scratch_cap)
                                 scratch[slot] = make_uint2(__float_as_uint(w[4 * j + c]), base + j * 1024 + rt * 4 + c);
+                            if (decltype(take_out)::value)
+                                w[4 * j + c] = ninf;
                         }
                 }
         };
@@ -1353,6 +1354,8 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         *at++ = make_uint2(__float_as_uint(w[e]), col + (e >> 2) * 1024 + (e & 3));
             }
         };
+        using T = std::true_type;
+        using F = std::false_type;
         // The loop over the tiles is compiled five times for each kind of launch, with the mask, the top_k histogram and the streamed sum
         // compiled in or out: a row runs a variant that holds little beyond its own work. (One loop with all
         // three as run-time branches costs the common penalised row 12 % of its launch time, and all eight
@@ -1517,17 +1520,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         if (tm >= thr)
                             keep_many(w, thr, base);
                     } else if (collect && tm >= thr) {
-                        keep_fours(tq, w, thr, base);
+                        keep_fours(tq, w, thr, base, std::integral_constant<bool, kSum && !kAgg>{});
                     }
                 }
                 if (kSum && cfg.need_sum && seen > ninf) {
-                    // Approximate weights, relative to the largest element seen. Of a row that keeps the few largest
-                    // every element; else of what is NOT collected (`thr` is the bound
-                    // the collection used): the collected elements get exact weights in the finish, so only the far tail
-                    // carries the approximation. (A NaN makes the sum of every
-                    // element one; such a row is left to the second launch.)
+                    // Approximate weights, relative to the largest element seen, of what is NOT collected (`thr` is the bound the
+                    // collection used): the collected elements get exact weights in the finish, so only the far tail
+                    // carries the approximation. Where few are kept they have been taken out already, and all sixteen are
+                    // summed without a choice each. (A NaN makes that sum one; such a row is left to the second launch.)
                     float p = 0.0f;
-                    if (kHist && sum_all) {
+                    if (kHist && !kAgg && cfg.hist_mode) {
 #pragma unroll
                         for (int e = 0; e < kEl; ++e)
                             p += ex2_approx(__fmaf_rn(w[e], c2, -sref));
@@ -1545,13 +1547,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                         if (some)
                             keep_many(w, thr, base);
                     } else if (some) {
-                        keep_fours(tq, w, thr, base);
+                        keep_fours(tq, w, thr, base, F{});
                     }
                 }
             }
         };
-        using T = std::true_type;
-        using F = std::false_type;
         using M = std::integral_constant<bool, kMasked>;
         if (!cfg.hist_mode && !cfg.need_sum)
             read_tiles(M{}, F{}, F{}, T{}); // penalties, min_p, greedy, a pure draw: nothing but maximum and bound
@@ -1740,8 +1740,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             __syncthreads();
         }
         const float thr = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
+        double dropped = 0.0; // top_p alone: what the slices kept and the row does not joins the streamed sum
         for_each_kept([&](const uint2& c, uint32_t g) {
             const bool in = __uint_as_float(c.x) >= thr;
+            if (cfg.need_sum && __uint_as_float(c.x) < thr)
+                dropped += (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
             const uint32_t bal = __ballot_sync(0xffffffffu, in);
             uint32_t at = 0;
             if (lane == 0 && bal)
@@ -1751,6 +1754,16 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                 merged[at] = make_uint2(c.x, c.y + g * a.split_w);
         });
         __syncthreads();
+        if (cfg.need_sum) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                dropped += __shfl_xor_sync(0xffffffffu, dropped, o);
+            if (lane == 0)
+                s.warp_sum[warp] = dropped;
+            __syncthreads();
+            for (uint32_t i = 0; i < kWarps; ++i)
+                total_approx += s.warp_sum[i];
+        }
         scratch = merged;
         qrow = reinterpret_cast<float*>(row_scratch);
     }
@@ -1766,29 +1779,29 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // is short and contiguous; every other row falls through to the general finish below, which recomputes from the
     // collected elements.
     constexpr uint32_t kFastRaw = 512;
-    if (mode != kModeVpLocal && !cfg.greedy && !s.nan0 && s.ncand <= kFastRaw && s.ncand <= scratch_cap &&
-        !(cfg.optimistic && total_approx != total_approx)) {
+    const bool weighed = mode != kModeVpLocal && !cfg.greedy && !s.nan0 && s.ncand <= kFastRaw && s.ncand <= scratch_cap &&
+                         !(cfg.optimistic && total_approx != total_approx);
+    double* const fsum = reinterpret_cast<double*>(dyn + kOffKeys + 8u * kWideCand); // the warps' sums of what was collected
+    if (weighed) {
         // Compiled twice: rows whose total is the candidates' own (nearly all) run code that knows nothing of the
         // row total of top_p alone.
         // Every thread takes one collected element, or two: exact weights, and the survivors of the exact filter side by side.
-        double* const fsum = reinterpret_cast<double*>(dyn + kOffKeys + 8u * kWideCand);
         {
             const uint32_t n_raw = s.ncand;
             const float thr_final = fmaxf(keep_threshold(cfg, m), key_to_float(s.thr_topk_key));
             unsigned long long* const fkeys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
-            double sum_kept = 0.0, sum_again = 0.0; // top_p alone: exact weights at or above the bound; what the streamed sum has too much
+            double sum_kept = 0.0, sum_rest = 0.0; // top_p alone: exact weights at or above the bound, the others
             for (uint32_t r0 = tid - lane; r0 < n_raw; r0 += (uint32_t)kThreads) {
                 const uint2 c = (r0 + lane < n_raw) ? scratch[r0 + lane] : make_uint2(0xff800000u, 0u);
                 const bool in = __uint_as_float(c.x) >= thr_final;
                 const float q = in ? expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), cfg.inv_t), s.exp2_table) : 0.0f;
                 if (cfg.need_sum) {
-                    // as streamed: of a kept element to be taken out again where the sum took every element, of one
-                    // collected while the bound was lower to be added where it took none of the collected
-                    const double streamed = (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
-                    if (in && q == q)
-                        sum_kept += (double)q;
-                    if (in == cfg.optimistic && streamed == streamed)
-                        sum_again += in ? streamed : -streamed;
+                    if (in) {
+                        if (q == q)
+                            sum_kept += (double)q;
+                    } else if (r0 + lane < n_raw) { // collected while the bound was lower: part of the row total, never a candidate
+                        sum_rest += (double)ex2_approx((__uint_as_float(c.x) - m) * (cfg.inv_t * 1.4426950408889634f));
+                    }
                 }
                 const bool ok = q >= cfg.minp_eff && q > 0.0f; // false for NaN
                 const uint32_t bal = __ballot_sync(0xffffffffu, ok);
@@ -1805,11 +1818,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     sum_kept += __shfl_xor_sync(0xffffffffu, sum_kept, o);
-                    sum_again += __shfl_xor_sync(0xffffffffu, sum_again, o);
+                    sum_rest += __shfl_xor_sync(0xffffffffu, sum_rest, o);
                 }
                 if (lane == 0) {
                     fsum[warp] = sum_kept;
-                    fsum[kThreads / 32 + warp] = sum_again;
+                    fsum[kThreads / 32 + warp] = sum_rest;
                 }
             }
         }
@@ -1819,10 +1832,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             const uint32_t full = 0xffffffffu;
             unsigned long long* const fkeys = reinterpret_cast<unsigned long long*>(dyn + kOffKeys);
             uint32_t n = s.nsurv;
-            double sum_kept = 0.0, sum_again = 0.0; // the warps' shares, below
+            double sum_kept = 0.0, sum_rest = 0.0; // the warps' shares, below
             if (kRowTotal && lane < (uint32_t)(kThreads / 32)) {
                 sum_kept = fsum[lane];
-                sum_again = fsum[kThreads / 32 + lane];
+                sum_rest = fsum[kThreads / 32 + lane];
             }
             bool done = n <= 32u;
             if (!kRowTotal && n > 32u && n <= kWideCand) {
@@ -1885,19 +1898,18 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                             inc += y;
                     }
                     double total_d = 0.0, band;
-                    // top_p alone: the total covers every column — exact weights of what was kept, and of the streamed
-                    // sum what lies beside them — and carries the margin of the approximate part and, where the kept
-                    // elements' shares had to be taken out of it, of the rounding of the streamed sum's terms
+                    // top_p alone: the total covers every column — exact weights of what was kept, the streamed sum
+                    // and the approximations above for the rest — and carries the margin of the approximate part
                     const bool row_total = kRowTotal && !(fl & MK_FLAG_NO_CANDIDATE);
                     if (row_total) {
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) {
                             sum_kept += __shfl_xor_sync(full, sum_kept, o);
-                            sum_again += __shfl_xor_sync(full, sum_again, o);
+                            sum_rest += __shfl_xor_sync(full, sum_rest, o);
                         }
-                        const double rest = fmax(total_approx - sum_again, 0.0);
+                        const double rest = total_approx + sum_rest;
                         total_d = sum_kept + rest;
-                        band = 1e-5 * rest + (cfg.optimistic ? 2e-6 * sum_kept : 0x1p-40 * total_d);
+                        band = 1e-5 * rest + 0x1p-40 * total_d;
                     } else {
                         total_d = __shfl_sync(full, inc, (int)n - 1);
                         band = 0x1p-40 * total_d;
@@ -2024,7 +2036,22 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // Top_p alone, and what was kept does not hold the nucleus, or holds too much to tell here: the row is left to the second
     // launch, with its maximum and total. (Where no weight can exist there is nothing to look for.)
     if (cfg.optimistic && !s.nan0 && !cfg.force_none && fabsf(m) < __int_as_float(0x7f800000)) {
+        if (!weighed) { // what was collected is not in the streamed sum
+            double collected = 0.0;
+            for (uint32_t i = tid; i < min(s.ncand, scratch_cap); i += kThreads)
+                collected += (double)ex2_approx((__uint_as_float(scratch[i].x) - m) * (cfg.inv_t * 1.4426950408889634f));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                collected += __shfl_xor_sync(0xffffffffu, collected, o);
+            if (lane == 0) {
+                fsum[warp] = collected;
+                fsum[kThreads / 32 + warp] = 0.0;
+            }
+            __syncthreads();
+        }
         if (tid == 0) {
+            for (int i = 0; i < 2 * (kThreads / 32); ++i)
+                total_approx += fsum[i];
             again[0] = 1u;
             again[1] = __float_as_uint(m);
             *reinterpret_cast<double*>(again + 2) = total_approx;

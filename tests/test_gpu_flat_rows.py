@@ -117,3 +117,46 @@ def test_two_sets_of_marked_rows_side_by_side(gpu_sampler_factory, ref):
             if not flags[b] & 0x2:
                 assert (d[b], bool(acc[b]), tok[b]) == want[b], f"call {call} row {b}"
     assert 0 < sum(w[1] for w in want) < batch
+
+
+def _top_p_beside(q, k, delta):
+    """The float nearest to (mass of the k heaviest) * (1 + delta), and how far off that mass it is, relative to the total."""
+    q = np.sort(q)[::-1]
+    share = q[:k].sum() / q.sum()
+    p = np.float32(share * (1.0 + delta))
+    return float(p), abs(float(p) - share)
+
+
+def test_the_first_launch_settles_what_its_margin_allows(gpu_sampler_factory, ref):
+    """A dozen heavy tokens over a rest of 1.4 %: the row's total is the kept tokens' exact weights and an approximate rest, so a
+    nucleus that ends a millionth of the total beside its bound is further off than the margin (1e-5 of the rest) and decided by the
+    first launch: no flag, and no stamp of the flat rows' kernel."""
+    import torch
+    from mako_b200 import lib
+    from mako_b200.sampler import pack_params
+    v, batch, cap = 50000, 16, 32
+    rng = np.random.default_rng(77)
+    rows = rng.normal(0, 0.5, size=(batch, v)).astype(np.float32)
+    ps = []
+    for b in range(batch):
+        cols = rng.choice(v, size=12, replace=False)
+        rows[b, cols] = (14.0 - 0.35 * np.arange(12) + rng.uniform(0, 0.05, 12)).astype(np.float32)
+        q = np.exp(rows[b].astype(np.float64) - float(rows[b].max()))
+        top_p, off = _top_p_beside(q, 3 + b % 7, -1e-6 if b % 2 else 1e-6)
+        rest = (q.sum() - np.sort(q)[::-1][:12].sum()) / q.sum()
+        assert 2e-5 * rest < off < 1.5e-6 and rest < 0.02
+        ps.append(SamplingParams(temperature=1.0, top_p=top_p))
+    u = np.linspace(0.01, 0.99, batch).astype(np.float32)
+    s = gpu_sampler_factory(v, batch, cap)
+    stamps = torch.zeros((batch, 64), dtype=torch.int64, device="cuda")
+    assert lib.mk_debug_set_timing(s._h, stamps.data_ptr()) == 0
+    try:
+        res = s.sample(torch.from_numpy(rows).cuda(), torch.from_numpy(pack_params(ps)).cuda(), torch.from_numpy(u).cuda())
+        torch.cuda.synchronize()
+    finally:
+        lib.mk_debug_set_timing(s._h, None)
+    assert not (res.flags.cpu().numpy() & 0x2).any()
+    assert (stamps[:, 14] == 0).all() and (stamps[:, 3] != 0).all()
+    for b in range(batch):
+        w = ref.sample(ps[b], rows[b], u[b], cap=cap)
+        assert (res.token[b].item(), res.n_cand[b].item()) == (w["token"], w["n_cand"]), f"row {b}"
