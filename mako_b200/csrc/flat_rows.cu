@@ -5,9 +5,10 @@
 // One CTA of 1024 threads takes a marked row; the others return. What the first launch leaves is the row's maximum and its
 // total weight (exact for what it kept, approximate for the rest), so the cut is known before the row is read again:
 //   sample    an eighth of the columns counted by weight class (sixteenths of an octave) says below which weight the elements
-//             sum up to a little less than the mass top_p leaves out;
+//             sum up to a little less than the mass top_p leaves out; where the bound that cannot be too tight leaves no more
+//             than a few thousand elements, that bound is the cut, and all of them get exact weights;
 //   collect   one pass over the row keeps everything above that weight — the nucleus and a few per cent more — and sums
-//             the approximate weights of the rest;
+//             the approximate weights of the rest, one by one in double;
 //   order     exact weights; the list is dealt into buckets of about eight, of equal counts rather than equal widths, each whose
 //             members rank themselves, a lane each (a warp or the CTA sorts where equal weights crowd a bucket);
 //   draw      double prefix sums for top_p, then the float total and the walk as scans (list_chain.cuh).
@@ -32,6 +33,7 @@ constexpr uint32_t kFlatBmWords = kFlatVocab / 32 + 2;
 constexpr uint32_t kMaxBuckets = 8192;
 constexpr uint32_t kWarpSort = 4096;        // a bucket of more than 32 and up to this size is sorted by one warp
 constexpr uint32_t kBigBuckets = 1024;
+constexpr uint32_t kKeepWhole = 6144;       // elements above the loose bound that are not cut further (see the cut)
 
 // Shared memory: the tables of the edits while the row is read, the list and its buckets afterwards.
 constexpr uint32_t kOffBitmap = 0;
@@ -53,7 +55,7 @@ struct FlatSmem {
     double sum[2][kFlatWarps];
     uint32_t wsum[kFlatWarps];
     uint32_t rows[16], n_rows;
-    uint32_t n_list, n_big, n_take, n_special;
+    uint32_t n_list, n_big, n_take, n_above;
     float cut;
     double run, prev;
 };
@@ -99,6 +101,14 @@ __device__ __forceinline__ double block_sum(FlatSmem& s, double v, int slot)
         t += __shfl_xor_sync(0xffffffffu, t, o);
     __syncthreads();
     return t;
+}
+
+// A float that is zero or normal, not negative, as a double: three integer instructions, where a conversion takes as long as the
+// exponential before it. (Zero comes out as 2^-127, which is nothing beside a total of at least one.)
+__device__ __forceinline__ double widen(float x)
+{
+    const uint32_t b = __float_as_uint(x);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
 }
 
 // Four mask bits from column c on (c may be negative: columns in front of the row read as not allowed by the caller's test).
@@ -319,9 +329,14 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             // class is never taken for less than the sample says. An eighth of a long row is counted, in runs of 128 columns.
             for (uint32_t i = tid; i < kClasses; i += kFlatThreads)
                 cls[i] = 0u;
+            if (tid == 0)
+                s.n_above = 0u;
             __syncthreads();
             const uint32_t every = n4 >= 24576u ? 8u : n4 >= 8192u ? 4u : 1u;
+            const float loose = fmaxf(keep_threshold(cfg, m), -FLT_MAX);
+            uint32_t above = 0; // the sample's elements above the loose bound
             auto enter = [&](float w, uint32_t n) {
+                above += w >= loose ? n : 0u;
                 const float x = (m - w) * (c2 * 16.0f);
                 if (x < (float)kClasses) // false for NaN and for what is not there
                     atomicAdd(&cls[min((uint32_t)fmaxf(x, 0.0f), kClasses - 1u)], n);
@@ -341,8 +356,10 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             }
             for (uint32_t r = tid; r < n_special; r += kFlatThreads)
                 enter(sval[r], 1u);
+            above = __reduce_add_sync(full, above);
+            if (lane == 0 && above)
+                atomicAdd(&s.n_above, above);
             __syncthreads();
-            const float loose = fmaxf(keep_threshold(cfg, m), -FLT_MAX);
             if (warp == 0) { // lane l holds classes 16 l .. 16 l + 15; mass from the light end
                 float sum = 0.0f, sq = 0.0f;
                 for (uint32_t j = 16u; j-- > 0u;) {
@@ -376,9 +393,11 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 }
                 cut = __reduce_min_sync(full, cut);
                 if (lane == 0) {
-                    // place of the class's heavy edge as a logit, a rounding below
+                    // Place of the class's heavy edge as a logit, a rounding below. Lists of up to 4096 elements above the loose
+                    // bound are kept whole, so that all of them count with their exact weights; the sample's own count of an eighth
+                    // is off by 170 or so there, a clustered one by more.
                     const float t = m - ((float)cut * 0.0625f) / c2;
-                    s.cut = cut < kClasses ? fmaxf(loose, t - fabsf(m) * 1e-6f - fabsf(t) * 1e-6f) : loose;
+                    s.cut = cut < kClasses && s.n_above > kKeepWhole ? fmaxf(loose, t - fabsf(m) * 1e-6f - fabsf(t) * 1e-6f) : loose;
                 }
             }
             __syncthreads();
@@ -405,16 +424,16 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     for (uint32_t k = 0; k < 4u; ++k)
                         edit4(g0 + k * 32u + lane, v[k], w[k]);
                     uint32_t keep = 0u; // one bit an element; nothing below branches on an element's own value
-                    float part = 0.0f;
+                    double part[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
                     for (uint32_t k = 0; k < 4u; ++k)
 #pragma unroll
                         for (uint32_t j = 0; j < 4u; ++j) {
                             keep |= w[k][j] >= thr ? 1u << (4u * k + j) : 0u;
                             const float e = ex2_approx((w[k][j] - m) * c2); // (not w * c2 - m * c2: that rounds m * c2)
-                            part += w[k][j] < thr ? e : 0.0f; // a NaN is neither
+                            part[j] += widen(w[k][j] < thr ? e : 0.0f); // a NaN is neither
                         }
-                    tail += (double)part;
+                    tail += (part[0] + part[1]) + (part[2] + part[3]);
                     const uint32_t mine = (uint32_t)__popc(keep);
                     if (__any_sync(full, mine != 0u)) {
                         uint32_t inc = mine;

@@ -160,3 +160,28 @@ def test_the_first_launch_settles_what_its_margin_allows(gpu_sampler_factory, re
     for b in range(batch):
         w = ref.sample(ps[b], rows[b], u[b], cap=cap)
         assert (res.token[b].item(), res.n_cand[b].item()) == (w["token"], w["n_cand"]), f"row {b}"
+
+
+def test_short_lists_are_decided_by_exact_weights(gpu_sampler_factory, ref):
+    """Rows of 4000 columns and nuclei of hundreds: every column above the loose bound counts with its exact weight, so a nucleus that
+    ends a few ten-millionths of the total beside its bound is decided without a guard band."""
+    import torch
+    from mako_b200.sampler import pack_params
+    v, batch, cap = 4000, 24, 64
+    rows = np.random.default_rng(78).normal(0, 1.0, size=(batch, v)).astype(np.float32)
+    ps, n_close = [], 0
+    for b in range(batch):
+        q = np.exp(rows[b].astype(np.float64) - float(rows[b].max()))
+        top_p, off = _top_p_beside(q, 300 + 61 * b, -2e-7 if b % 2 else 2e-7)
+        n_close += 1e-8 < off < 5e-7
+        ps.append(SamplingParams(temperature=1.0, top_p=top_p))
+    assert n_close >= batch - 4
+    u = np.linspace(0.01, 0.99, batch).astype(np.float32)
+    s = gpu_sampler_factory(v, batch, cap)
+    res = s.sample(torch.from_numpy(rows).cuda(), torch.from_numpy(pack_params(ps)).cuda(), torch.from_numpy(u).cuda())
+    torch.cuda.synchronize()
+    assert not (res.flags.cpu().numpy() & 0x2).any()
+    for b in range(batch):
+        w = ref.sample(ps[b], rows[b], u[b], cap=cap)
+        assert (res.token[b].item(), res.n_cand[b].item()) == (w["token"], w["n_cand"]), f"row {b}"
+        assert w["n_cand"] > 100
