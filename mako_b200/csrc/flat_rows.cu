@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
             const uint32_t row = s.rows[slot0 + ri];
             // ---- the row -------------------------------------------------------------------------------------------
             const mk_sampling_params prm = a.params_dev ? a.params_dev[row] : a.params;
-            const RowCfg cfg = make_cfg(prm, V, a.mode, a.vp_k, 1);
+            const RowCfg cfg = make_cfg(prm, V, a.mode, a.vp_k, 1, true);
             uint32_t* const row_scratch = a.scratch + (size_t)row * row_scratch_words(a.scratch_cap);
             uint2* const list = reinterpret_cast<uint2*>(row_scratch);
             uint32_t* const state = row_scratch + 4ull * a.scratch_cap;

@@ -12,8 +12,10 @@
 namespace mk {
 
 // top_p alone, first launch: the largest elements kept. The bound that keeps them is the edge of a histogram bin and lets
-// about 1.4 times as many through; the one-warp finish takes 32.
-constexpr uint32_t kNucleusGuess = 20;
+// about 1.4 times as many through; the one-warp finish takes 32. Rows that the flat rows' kernel does not take pay for a longer
+// nucleus with a second stream of the row: they keep a few more, and the general finish has a look at what the one-warp finish
+// could not settle; of the others that goes to the flat rows' kernel at once. (hist_k says which of the two a row is.)
+constexpr uint32_t kNucleusGuess = 20, kNucleusGuessAlone = 24;
 
 struct RowCfg {
     float temperature, inv_t, minp_eff, top_p;
@@ -32,7 +34,8 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-__device__ __forceinline__ RowCfg make_cfg(const mk_sampling_params& p, uint32_t n_vocab, int mode, uint32_t vp_k, int pass)
+// `flat`: whether the flat rows' kernel takes this row, should it be marked.
+__device__ __forceinline__ RowCfg make_cfg(const mk_sampling_params& p, uint32_t n_vocab, int mode, uint32_t vp_k, int pass, bool flat)
 {
     RowCfg c;
     c.temperature = p.temperature;
@@ -54,13 +57,14 @@ __device__ __forceinline__ RowCfg make_cfg(const mk_sampling_params& p, uint32_t
     // The float total over "all candidates" is only needed when top_p is the only truncation.
     c.need_sum = !c.greedy && c.use_topp && !minp_on && !c.hist_mode;
     c.force_none = !c.greedy && (!(c.inv_t < __int_as_float(0x7f800000)) || !(c.inv_t == c.inv_t));
-    // top_p alone: the first launch bets that the nucleus lies within the kNucleusGuess largest elements and keeps
+    // top_p alone: the first launch bets that the nucleus lies within the largest few elements and keeps
     // only those (the top_k histogram bound, with no top_k cut afterwards); a row whose nucleus does not close within
-    // what was kept asks for the second pass, which keeps everything the mass bound allows.
-    c.optimistic = c.need_sum && pass == 0 && mode != kModeVpLocal && kNucleusGuess < n_vocab;
+    // what was kept asks for a second launch, which keeps everything the mass bound allows.
+    const uint32_t guess = flat ? kNucleusGuess : kNucleusGuessAlone;
+    c.optimistic = c.need_sum && pass == 0 && mode != kModeVpLocal && guess < n_vocab;
     if (c.optimistic) {
         c.hist_mode = true;
-        c.hist_k = kNucleusGuess;
+        c.hist_k = guess;
     }
     if (mode == kModeVpLocal) {
         c.hist_mode = vp_k < n_vocab;

@@ -508,7 +508,7 @@ __device__ __noinline__ uint32_t wide_top_p(Smem& s, const unsigned long long* k
     }
     __syncthreads();
     const double run = s.warp_sum[0], prev = s.warp_sum[1];
-    const bool unsure = (need_sum && run < want) ||
+    const bool unsure = (need_sum && !(run >= want)) ||
                         (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)));
     return k | (unsure ? 0x80000000u : 0u);
 }
@@ -693,6 +693,22 @@ __device__ __noinline__ const unsigned long long* long_sort(Smem& s, unsigned lo
         P = src;
     }
     return P;
+}
+
+// Approximate weights of a row's collected elements, a sum a warp (and as many zeros behind them). Whole CTA.
+__device__ __noinline__ void weigh_collected(const uint2* scratch, uint32_t n, float m, float inv_t, double* sums)
+{
+    double collected = 0.0;
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads)
+        collected += (double)ex2_approx((__uint_as_float(scratch[i].x) - m) * (inv_t * 1.4426950408889634f));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        collected += __shfl_xor_sync(0xffffffffu, collected, o);
+    if ((threadIdx.x & 31u) == 0u) {
+        sums[threadIdx.x >> 5] = collected;
+        sums[kThreads / 32 + (threadIdx.x >> 5)] = 0.0;
+    }
+    __syncthreads();
 }
 
 constexpr uint32_t kWideCand = 64;
@@ -952,7 +968,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             hc[i] = (j < hlen) ? (uint32_t)hist_at(j) - (uint32_t)id_off : 0xffffffffu;
         }
     }
-    const RowCfg cfg = make_cfg(prm, a.n_vocab, mode, a.vp_k, a.pass);
+    const RowCfg cfg = make_cfg(prm, a.n_vocab, mode, a.vp_k, a.pass, flat_row_takes(a, hlen, nb));
     const uint32_t* __restrict__ mrow = (kMasked && a.mask) ? a.mask + (size_t)row * a.mask_ld + (col0 >> 5) : nullptr;
     // Per-row scratch, 16 bytes per column: scratch_cap raw candidates (logit bits, column) — sorted in place as
     // 64-bit keys by the large sorted-list path — then as much again: the merge sort's second buffer, or (large
@@ -2033,22 +2049,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             s.n_final = 0;
     }
 
-    // Top_p alone, and what was kept does not hold the nucleus, or holds too much to tell here: the row is left to the second
-    // launch, with its maximum and total. (Where no weight can exist there is nothing to look for.)
-    if (cfg.optimistic && !s.nan0 && !cfg.force_none && fabsf(m) < __int_as_float(0x7f800000)) {
-        if (!weighed) { // what was collected is not in the streamed sum
-            double collected = 0.0;
-            for (uint32_t i = tid; i < min(s.ncand, scratch_cap); i += kThreads)
-                collected += (double)ex2_approx((__uint_as_float(scratch[i].x) - m) * (cfg.inv_t * 1.4426950408889634f));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                collected += __shfl_xor_sync(0xffffffffu, collected, o);
-            if (lane == 0) {
-                fsum[warp] = collected;
-                fsum[kThreads / 32 + warp] = 0.0;
-            }
-            __syncthreads();
-        }
+    // Top_p alone, and what was kept does not hold the nucleus, or holds too much to tell here: the row is left to the flat rows'
+    // kernel, with its maximum and total. (Where no weight can exist there is nothing to look for.)
+    if (cfg.optimistic && cfg.hist_k == kNucleusGuess && !s.nan0 && !cfg.force_none && fabsf(m) < __int_as_float(0x7f800000)) {
+        if (!weighed) // what was collected is not in the streamed sum
+            weigh_collected(scratch, min(s.ncand, scratch_cap), m, cfg.inv_t, fsum);
         if (tid == 0) {
             for (int i = 0; i < 2 * (kThreads / 32); ++i)
                 total_approx += fsum[i];
@@ -2385,7 +2390,11 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
 
     if (a.timing && tid == 0)
         a.timing[(size_t)row * 64 + 13] = global_ns();
+    // A first launch of top_p alone that has come this far (the flat rows' kernel does not take the row) leaves what it cannot settle to
+    // the row pipeline's own second launch, which writes every output again.
     if (!short_list) {
+        if ((flags & MK_FLAG_GUARD_BAND) && cfg.optimistic && tid == 0)
+            again[0] = 1u;
         const RowOut o = {a.token, a.prob, a.flags, a.n_cand, a.accepted, a.total_out, a.cand_ids, a.cand_q,
                           a.cand_cap, id_off, a.timing, mode};
         // the weights in order go behind the keys where there is room, else to the half of the scratch the list is not in
@@ -2434,9 +2443,12 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
                     }
                 }
             }
-            if ((cfg.need_sum && run < want) ||
-                (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band))))
+            if ((cfg.need_sum && !(run >= want)) || // (also where a NaN in the row has made its total one)
+                (k >= 1 && (fabs(run - want) <= band || (k >= 2 && fabs(prev - want) <= band)))) {
                 flags |= MK_FLAG_GUARD_BAND;
+                if (cfg.optimistic && lane == 0)
+                    again[0] = 1u;
+            }
             n = max(k, 1u);
         }
         float total = 0.0f, q_draft = 0.0f;

@@ -185,3 +185,48 @@ def test_short_lists_are_decided_by_exact_weights(gpu_sampler_factory, ref):
         w = ref.sample(ps[b], rows[b], u[b], cap=cap)
         assert (res.token[b].item(), res.n_cand[b].item()) == (w["token"], w["n_cand"]), f"row {b}"
         assert w["n_cand"] > 100
+
+
+@pytest.mark.parametrize("kind", ["speculative round", "long history", "wide vocabulary"])
+def test_rows_the_flat_kernel_does_not_take(gpu_sampler_factory, ref, kind):
+    """Their second launch streams the row again, so the first one settles a nucleus of up to 24 tokens by itself: the count of
+    collected elements that the general finish leaves in the stamps is then a few dozen at most, not a second launch's
+    thousands. A row with a NaN and a flat one among them do take the second launch."""
+    import torch
+    from mako_b200 import lib
+    v, batch, cap = (170000 if kind == "wide vocabulary" else 50000), 12, 64
+    p = SamplingParams(temperature=1.0, top_p=0.88, frequency_penalty=0.01)
+    rng = np.random.default_rng(79)
+    rows = rng.normal(0, 0.5, size=(batch, v)).astype(np.float32)
+    for b in range(batch - 1):
+        rows[b, 10000 + rng.choice(v - 10000, size=26, replace=False)] = rng.uniform(13.4, 14.6, 26)
+    rows[2, 17] = np.nan
+    hist = np.zeros((batch, 4200 if kind == "long history" else 8), dtype=np.int32)  # (id 0, over and over)
+    u = rng.uniform(0.01, 0.99, batch).astype(np.float32)
+    s = gpu_sampler_factory(v, batch, cap)
+    stamps = torch.zeros((batch, 64), dtype=torch.int64, device="cuda")
+    lg, hist_dev = torch.from_numpy(rows).cuda(), torch.from_numpy(hist).cuda()
+    assert lib.mk_debug_set_timing(s._h, stamps.data_ptr()) == 0
+    try:
+        if kind == "speculative round":  # rounds of a bonus row alone
+            us = torch.from_numpy(np.stack([u, u], 1)).cuda()
+            res = s.spec_round(lg, p, torch.zeros((batch, 0), dtype=torch.int32, device="cuda"), us, history=hist_dev)[2]
+        else:
+            res = s.sample(lg, p, torch.from_numpy(u).cuda(), history=hist_dev)
+        torch.cuda.synchronize()
+    finally:
+        lib.mk_debug_set_timing(s._h, None)
+    collected, flags = stamps[:, 9].tolist(), res.flags.cpu().numpy()
+    n_within = 0
+    for b in range(batch):
+        w = ref.sample(p, rows[b], u[b], cap=cap, history=hist[b])
+        assert not flags[b] & 0x52
+        k = min(w["n_cand"], cap)
+        assert (res.token[b].item(), res.n_cand[b].item()) == (w["token"], w["n_cand"]), f"row {b}"
+        assert np.array_equal(res.cand_ids[b, :k].cpu().numpy(), w["cand_ids"][:k]), f"row {b}"
+        if b in (2, batch - 1):
+            assert collected[b] > 512
+        elif w["n_cand"] <= 24:
+            assert collected[b] <= 512, f"row {b}"
+            n_within += w["n_cand"] > 20
+    assert n_within >= 4

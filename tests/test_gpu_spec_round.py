@@ -42,7 +42,8 @@ def _cpu_round(ref, p, logits, drafts, forced, u, hist):
                     frequency_penalty=0.3), False),
     (SamplingParams(temperature=0.7, top_k=40, top_p=0.95, repetition_penalty=1.3), True),
     (SamplingParams(temperature=0.0), True),
-], ids=["penalised", "nucleus+forced", "greedy+forced"])
+    (SamplingParams(temperature=1.0, top_p=0.9, repetition_penalty=1.1, frequency_penalty=0.2), True),
+], ids=["penalised", "nucleus+forced", "greedy+forced", "top_p alone+forced"])
 @pytest.mark.parametrize("v,n_seq", [(40003, 64), (129280, 24)], ids=["ragged_rows", "aligned_rows"])
 def test_rounds_of_four_drafts_and_a_bonus_row(gpu_sampler_factory, ref, params, with_forced, v, n_seq):
     """Rows of 40003 columns are not 16-byte aligned and take the kernel's plain-load path, rows of 129280 columns
@@ -60,6 +61,7 @@ def test_rounds_of_four_drafts_and_a_bonus_row(gpu_sampler_factory, ref, params,
     kept_total = 0
     for rnd in range(rounds):
         logits, spikes = synth.logits(500 + rnd, n_seq * n_pos, v)
+        logits[3::7] *= 0.5  # some rows are flat: under top_p alone their nucleus is read for in a second launch
         # drafts: mostly the row's strongest tokens (often kept), sometimes a random one (rejected), sometimes a repeat
         drafts = np.empty((n_seq, n_drafts), dtype=np.int32)
         for i in range(n_seq):
