@@ -143,14 +143,15 @@ struct RowOut {
 
 // What the draw leaves behind once its chains are known (sampler.cpp:64-73, 80-83, 100-106), for a list of n weights q in draw
 // order (16-byte aligned; zeros, the gaps of a list laid out by column, never win; a rejected draft's weight is zeroed).
-// col_of(i) names a weight's column; n_out is the number of candidates. Whole CTA; the caller synchronises before.
+// col_of(i) names a weight's column; n_out is the number of candidates; in front of place `from`, a multiple of eight, there are
+// only zeros. Whole CTA; the caller synchronises before.
 template <int kThreads, class Col>
 __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, float* q, uint32_t n, uint32_t n_out, uint32_t draft_idx,
                                           uint32_t row, uint32_t flags, float u_row, float u2_row, int32_t draft_row,
-                                          const RowOut& o, Col&& col_of)
+                                          const RowOut& o, Col&& col_of, uint32_t from = 0u)
 {
     const uint32_t none = 0xffffffffu;
-    const float total = chain<kThreads, false>(cs, q, n, 0.0f);
+    const float total = chain<kThreads, false>(cs, q, n, 0.0f, from);
     const float q_draft = (draft_idx != none) ? q[draft_idx] : 0.0f;
     int32_t tok = -1, acc = 0;
     float prob = 0.0f, walk_total = total;
@@ -174,7 +175,7 @@ __device__ __forceinline__ void draw_long(ChainSmem<kThreads>& cs, float* q, uin
                 q[draft_idx] = 0.0f;
             __syncthreads();
         }
-        chain<kThreads, true>(cs, q, n, __fmul_rn((o.mode == kModeVerify) ? u2_row : u_row, walk_total));
+        chain<kThreads, true>(cs, q, n, __fmul_rn((o.mode == kModeVerify) ? u2_row : u_row, walk_total), from);
         hit = cs.hit;
         r_hit = cs.r_hit;
         q_hit = cs.q_hit;

@@ -370,19 +370,27 @@ __device__ __noinline__ void wide_id_ordered(Smem& s, RowChain& cs, const uint2*
     const uint32_t tid = threadIdx.x;
     for (uint32_t i = tid; i < V; i += kThreads)
         qrow[i] = 0.0f;
+    if (tid == 0)
+        cs.first = V;
     __syncthreads();
+    uint32_t lowest = V; // of this thread's columns
     for (uint32_t i = tid; i < n_raw; i += kThreads) {
         const uint2 c = scratch[i];
         if (!(__uint_as_float(c.x) >= thr_final))
             continue;
         const float q = expf_host_exact(__fmul_rn(__fsub_rn(__uint_as_float(c.x), m), inv_t), s.exp2_table);
-        if (q >= minp_eff && q > 0.0f)
+        if (q >= minp_eff && q > 0.0f) {
             qrow[c.y] = q;
+            lowest = min(lowest, c.y);
+        }
     }
+    atomicMin(&cs.first, lowest);
     __syncthreads();
+    const uint32_t from = cs.first & ~7u;
+    __syncthreads(); // (the draw writes there again)
     if ((o.cand_ids || o.cand_q) && tid < 32u) { // the candidate list, as far as the caller wants it
         uint32_t at = 0;
-        for (uint32_t c0 = 0; c0 < V && at < o.cand_cap; c0 += 32u) {
+        for (uint32_t c0 = from; c0 < V && at < o.cand_cap; c0 += 32u) {
             const float q = (c0 + tid < V) ? qrow[c0 + tid] : 0.0f;
             const uint32_t have = __ballot_sync(0xffffffffu, q > 0.0f);
             const uint32_t slot = at + (uint32_t)__popc(have & ((1u << tid) - 1u));
@@ -395,7 +403,7 @@ __device__ __noinline__ void wide_id_ordered(Smem& s, RowChain& cs, const uint2*
     }
     const int64_t d = (int64_t)draft_row - o.id_offset;
     const uint32_t draft_idx = (o.mode == kModeVerify && draft_row >= 0 && d >= 0 && d < (int64_t)V) ? (uint32_t)d : 0xffffffffu;
-    draw_long<kThreads>(cs, qrow, V, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, [](uint32_t i) -> uint32_t { return i; });
+    draw_long<kThreads>(cs, qrow, V, n, draft_idx, row, flags, u_row, u2_row, draft_row, o, [](uint32_t i) -> uint32_t { return i; }, from);
 }
 
 // How a long list names its candidates.
