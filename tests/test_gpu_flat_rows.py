@@ -230,3 +230,24 @@ def test_rows_the_flat_kernel_does_not_take(gpu_sampler_factory, ref, kind):
             assert collected[b] <= 512, f"row {b}"
             n_within += w["n_cand"] > 20
     assert n_within >= 4
+
+
+@pytest.mark.parametrize("v", [4096, 100000])
+def test_a_min_p_that_is_no_number(gpu_sampler_factory, ref, v):
+    """No weight is at least NaN: there is no candidate, whatever top_p would have kept, and the first maximum is returned."""
+    import torch
+    p, batch = SamplingParams(temperature=1.0, top_p=0.9, min_p=float("nan")), 3
+    rows = np.zeros((batch, v), dtype=np.float32)  # (all equal: more than the one-warp finish looks at)
+    rows[1] = np.random.default_rng(80).normal(0, 0.4, v)
+    rows[2, 77] = 9.0
+    u = np.full(batch, 0.7, dtype=np.float32)
+    s = gpu_sampler_factory(v, batch, 16)
+    for split in (True, False):
+        s.set_split(split)
+        res = s.sample(torch.from_numpy(rows).cuda(), p, torch.from_numpy(u).cuda())
+        torch.cuda.synchronize()
+        want = [ref.sample(p, rows[b], u[b], cap=16) for b in range(batch)]
+        assert [w["token"] for w in want] == rows.argmax(1).tolist()
+        assert res.token.tolist() == [w["token"] for w in want] and res.n_cand.tolist() == [1] * batch
+        assert all(f & 0x4 for f in res.flags.tolist())
+    s.set_split(True)
