@@ -34,6 +34,11 @@ def _stream_ptr(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index)
 
 
+def _first(t: torch.Tensor, b: int) -> torch.Tensor:
+    """The first b rows, as a tensor of its own for each call (of a whole one: 0.5 us, a slice takes 1.4)."""
+    return t.detach() if t.shape[0] == b else t[:b]
+
+
 class Sampler:
     """One row at a time, as the reference: Sampler(params, n_vocab, seed); sample(); verify(); accept()."""
 
@@ -106,7 +111,6 @@ class BatchSampler:
         check(lib.mk_sampler_create(C.byref(self._h), device, n_vocab, max_batch))
         self.n_vocab, self.max_batch, self.cand_cap = n_vocab, max_batch, cand_cap
         d = self.device
-        self._views = (-1, ())
         self.token = torch.empty(max_batch, dtype=torch.int32, device=d)
         self.prob = torch.empty(max_batch, dtype=torch.float32, device=d)
         self.flags = torch.zeros(max_batch, dtype=torch.int32, device=d)
@@ -136,12 +140,14 @@ class BatchSampler:
     # -- argument marshalling -----------------------------------------------------------------------------------
     def _rows(self, logits: torch.Tensor, params, history=None, history_len=None, mask=None, bias=None,
               n_vocab=None, id_offset: int = 0) -> RowsC:
-        assert logits.is_cuda and logits.dtype == torch.float32 and logits.dim() == 2 and logits.stride(1) == 1
+        assert logits.is_cuda and logits.dtype == torch.float32 and logits.dim() == 2
+        (ld, unit), (batch, columns) = logits.stride(), logits.shape
+        assert unit == 1
         r = RowsC()
         r.logits = logits.data_ptr()
-        r.ld = logits.stride(0)
-        r.batch = logits.shape[0]
-        r.n_vocab = n_vocab if n_vocab is not None else logits.shape[1]
+        r.ld = ld
+        r.batch = batch
+        r.n_vocab = n_vocab if n_vocab is not None else columns
         r.id_offset = id_offset
         if history is not None:
             assert history.is_cuda and history.dtype == torch.int32 and history.dim() == 2 and history.stride(1) == 1
@@ -162,10 +168,13 @@ class BatchSampler:
             r.bias = bias.data_ptr()
             r.n_bias = bias.shape[1]
         if isinstance(params, torch.Tensor):
-            assert params.is_cuda and params.dtype == torch.int32 and params.shape == (logits.shape[0], 7)
+            assert params.is_cuda and params.dtype == torch.int32 and params.shape == (batch, 7)
             r.params_dev = params.data_ptr()
-        else:
-            r.params = params.to_c()
+        else:  # field by field: a structure of its own to copy from takes three times as long
+            p = r.params
+            p.temperature, p.top_k, p.top_p, p.min_p = params.temperature, params.top_k, params.top_p, params.min_p
+            p.presence_penalty, p.frequency_penalty = params.presence_penalty, params.frequency_penalty
+            p.repetition_penalty = params.repetition_penalty
         return r
 
     def _out(self, batch: int) -> SampleOutC:
@@ -181,10 +190,9 @@ class BatchSampler:
         return o
 
     def _result(self, b: int, **kw) -> SampleResult:
-        if self._views[0] != b:  # the outputs' first rows: slicing them anew was a quarter of a call's host time
-            self._views = (b, (self.token[:b], self.prob[:b], self.flags[:b], self.n_cand[:b],
-                               self.cand_ids[:b] if self.cand_cap else None, self.cand_q[:b] if self.cand_cap else None))
-        return SampleResult(*self._views[1], **kw)
+        return SampleResult(_first(self.token, b), _first(self.prob, b), _first(self.flags, b), _first(self.n_cand, b),
+                            _first(self.cand_ids, b) if self.cand_cap else None,
+                            _first(self.cand_q, b) if self.cand_cap else None, **kw)
 
     # -- the operations -----------------------------------------------------------------------------------------
     def sample(self, logits, params, u=None, *, history=None, history_len=None, mask=None, bias=None) -> SampleResult:
