@@ -173,7 +173,7 @@ bool all_greedy(const mk_rows* r)
 // which of the two row sets of p/q verification (0 elsewhere).
 void split_rows(mk::RowKernelArgs& a, const mk_sampler* s, uint32_t batch, uint32_t set)
 {
-    if (!s->split || !s->split_parts || batch == 0 || batch > mk::kSplitMaxRows || s->timing || s->skip_tile != 0xffffffffu)
+    if (!s->split || !s->split_parts || batch == 0 || batch > mk::kSplitMaxRows || s->timing)
         return;
     const uint32_t n_tiles = (a.n_vocab + kTile - 1) / kTile;
     const mk_sampling_params& p = a.params;

@@ -933,6 +933,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     // Probes a wait for a tile makes before it gives up (each parks the thread for up to 20 us): seconds normally, a
     // few milliseconds with the test hook that withholds a tile.
     const uint32_t wait_probes = a.debug_wait_probes ? a.debug_wait_probes : (1u << 17);
+    const uint32_t skip_tile = a.debug_skip_tile - col0 / (uint32_t)kTile; // (counted from the row's first tile)
     if (!early)
         griddep_wait();
     const mk_sampling_params prm = a.params_dev ? a.params_dev[row] : a.params;
@@ -1066,7 +1067,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     const uint32_t tiles_early = (list_owners && tiles_issued == n_stages) ? n_stages - 1u : tiles_issued;
     auto fill_ring = [&](uint32_t t0, uint32_t t1) {
         for (uint32_t t = t0; t < t1; ++t) {
-            if (t == a.debug_skip_tile)
+            if (t == skip_tile)
                 continue; // test hook: this tile's copy is never requested, so that the waits for it run out
             const uint32_t n_t = min((uint32_t)kTile, V - t * kTile);
             const uint32_t bytes = (n_t * 4u) & ~15u;
@@ -1241,7 +1242,7 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
             }
             if (*(volatile uint32_t*)&s.abort_flag)
                 break;
-            if (t == a.debug_skip_tile)
+            if (t == skip_tile)
                 continue;
             if (lane == 0) {
                 fence_proxy_async();

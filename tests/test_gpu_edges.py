@@ -260,20 +260,23 @@ def test_overlap_modes_give_the_same_tokens(gpu_sampler_factory, ref):
     s.set_overlap(0)
 
 
+@pytest.mark.parametrize("split", [False, True], ids=["whole rows", "split rows"])
 @pytest.mark.parametrize("with_history", [True, False], ids=["fix-up warps wait", "readers wait"])
-def test_a_wait_that_runs_out_ends_the_row_in_good_order(ref, with_history):
+def test_a_wait_that_runs_out_ends_the_row_in_good_order(ref, with_history, split):
     """Every wait in the kernel is bounded. With the test hook that never requests one tile's copy, the waits for
     that tile run out after a few milliseconds: each row returns token -1 with MK_FLAG_TIMEOUT, nothing traps or
-    hangs, and the same handle samples correctly right afterwards."""
+    hangs, and the same handle samples correctly right afterwards. (Of a split row one slice's CTA runs into it, and the last
+    to arrive reports it.)"""
     import torch
     from mako_b200 import BatchSampler, lib
-    v, b = 40003, 6
+    v, b = 100003 if split else 40003, 6
     inp = Inputs(411, b, v, n_history=600 if with_history else 0)
     p = SamplingParams(temperature=0.8, top_p=0.9, min_p=0.05, repetition_penalty=1.1, presence_penalty=0.5,
                        frequency_penalty=0.3)
     g = inp.to_gpu()
     s = BatchSampler(v, b, 0)
-    assert lib.mk_debug_withhold_tile(s._h, 7, 100) == 0          # tile 7 of 10 never arrives; 100 probes of <= 20 us
+    s.set_split(split)
+    assert lib.mk_debug_withhold_tile(s._h, 7, 100) == 0          # the row's tile 7 never arrives; 100 probes of <= 20 us
     res = s.sample(g["logits"], p, g["u"], **g["kw"])
     torch.cuda.synchronize()
     assert res.token.cpu().tolist() == [-1] * b
