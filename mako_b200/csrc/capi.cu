@@ -165,27 +165,72 @@ bool all_greedy(const mk_rows* r)
 
 // A few rows leave most of the device idle when each is one CTA. Their columns are split instead, into as many slices as fill
 // the device's 296 places once (of at least a tile of 4096 columns), and the last CTA of a row to arrive draws from what all of
-// them kept. Measured (us a call, split / one CTA a row), 151552 columns: one row top_k 18.5 / 35.6, top_p 20.2 / 42.7, min_p
-// 12.3 / 20.7, greedy 7.0 / 16.9, a mask's 3000 candidates 40 / 67; 148 rows 36 / 37.5, 95 / 101, 26.3 / 27.8, 16.3 / 17.6, 64 / 70
-// (two slices a row; more rows fill the device by themselves). Eight tiles (32000 columns): up to 96 rows under the histogram
-// bound still gain (one row top_k 14.1 / 17.3, top_p 17.1 / 19.7), the others lose a microsecond to the meeting of their
-// slices (min_p 9.4 / 8.0, greedy 6.8 / 6.4) and 128 rows of top_p 2.5, so short rows are split only under that bound. `set`:
-// which of the two row sets of p/q verification (0 elsewhere).
-void split_rows(mk::RowKernelArgs& a, const mk_sampler* s, uint32_t batch, uint32_t set)
+// them kept. That pays for the meeting of the slices (1 to 4 us) where a row streams for long enough and the device has room, so
+// the line is a number of tiles that rises with the number of rows, and lies the higher the faster such rows stream. Measured
+// in graphs, the whole rows' time over the split rows' time (151552 columns are 37 tiles):
+//   rows                 top_k                      top_p alone           mask, penalties       min_p, neither         greedy
+//    1    4 / 8 / 37     0.86 / 1.10 / 1.85         0.95 / 1.08 / 1.76     - / 1.06 / 1.76       0.86 / 1.00 / 1.59     0.75 / 0.94 / 2.14
+//   16    8 / 12 / 37    1.10 / 1.44 / 1.64         1.03 / 1.08 / 1.61    1.06 / 1.11 / 1.49    1.00 / 1.07 / 1.48     0.85 / 0.97 / 1.82
+//   48    8 / 12 / 37    1.00 / 1.31 / 1.32         0.99 / 1.03 / 1.30    0.99 / 1.05 / 1.27    0.97 / 1.00 / 1.22     0.78 / 0.87 / 1.44
+//   96    12 / 20 / 37   1.12 / 1.19 / 1.15         0.98 / 1.03 / 1.13    0.99 / 1.03 / 1.14    0.94 / 0.99 / 1.10     0.80 / 0.89 / 1.08
+//   148   12 / 28 / 37   1.02 / 1.08 / 1.02         0.94 / 1.00 / 1.04    0.93 / 1.01 / 1.04    0.91 / 0.89 / 0.99     0.76 / 0.82 / 0.87
+// (`mask, penalties`: the slower of a masked draw and penalised min_p rows.) Rows with parameters of their own, greedy ones among
+// them: 16 rows 1.04 at 8 tiles, 48 rows 1.05 at 10, 64 rows 1.15 at 12, 128 rows 1.04 / 1.26 / 1.07 at 16 / 20 / 24 but 96 rows
+// 0.94 at 37 and 148 rows 0.82; with histories 48 rows 1.01 at 8, 64 rows 1.03 at 12, 96 rows 1.01 at 16, 80 rows 1.04 at 37 and 128
+// rows 0.96 to 0.97 everywhere. The two row sets of p/q verification share the device: under top_k or top_p 8 rows 1.18 and
+// 1.02 at 10 tiles, 16 rows 1.17 and 1.03 at 16, 32 rows 1.04 and 1.07 at 32, 48 rows 0.91 and 0.99 at 37, 148 rows 0.71 and 0.90;
+// under neither 16 rows 1.05 at 32 and 148 rows 0.83. More rows than 148 fill the device by themselves.
+struct SplitLine {
+    uint32_t tiles, rows; // from so many tiles on, calls of up to so many rows
+};
+
+template <size_t N>
+uint32_t split_max_rows(const SplitLine (&lines)[N], uint32_t n_tiles)
 {
+    uint32_t rows = 0;
+    for (const SplitLine& l : lines)
+        if (n_tiles >= l.tiles)
+            rows = l.rows;
+    return rows;
+}
+
+// `set`: which of the two row sets of p/q verification, or -1.
+void split_rows(mk::RowKernelArgs& a, const mk_sampler* s, uint32_t batch, int set)
+{
+    static const SplitLine top_k[] = {{8, 32}, {10, 148}}, slow[] = {{8, 16}, {10, 48}, {12, 64}, {20, 96}, {28, 148}},
+                           fast[] = {{10, 16}, {12, 32}, {16, 64}, {20, 80}, {37, 96}, {40, 148}},
+                           greedy[] = {{14, 16}, {20, 48}, {28, 64}, {32, 80}, {37, 96}}, own[] = {{8, 16}, {10, 48}, {12, 64}, {16, 128}, {32, 64}},
+                           own_history[] = {{8, 48}, {12, 64}, {16, 96}, {37, 80}}, pq_bound[] = {{10, 8}, {16, 16}, {32, 32}},
+                           pq[] = {{20, 4}, {32, 16}};
     if (!s->split || !s->split_parts || batch == 0 || batch > mk::kSplitMaxRows || s->timing)
         return;
     const uint32_t n_tiles = (a.n_vocab + kTile - 1) / kTile;
     const mk_sampling_params& p = a.params;
-    const bool bound = !a.params_dev && p.temperature > 0.0f && ((p.top_k > 0 && p.top_k < a.n_vocab) || (p.top_p < 1.0f && !(p.min_p > 0.0f)));
-    if (n_tiles < (bound && batch <= 96u ? 4u : 12u))
+    const bool shared = !a.params_dev, by_top_k = shared && p.top_k > 0 && p.top_k < a.n_vocab,
+               by_top_p = shared && p.top_p < 1.0f && !(p.min_p > 0.0f),
+               penalties = a.history && !(p.repetition_penalty == 1.0f && p.presence_penalty == 0.0f && p.frequency_penalty == 0.0f);
+    uint32_t rows;
+    if (shared && p.temperature <= 0.0f)
+        rows = set < 0 ? split_max_rows(greedy, n_tiles) : 0u;
+    else if (set >= 0)
+        rows = by_top_k || by_top_p ? split_max_rows(pq_bound, n_tiles) : split_max_rows(pq, n_tiles);
+    else if (!shared)
+        rows = a.history ? split_max_rows(own_history, n_tiles) : split_max_rows(own, n_tiles);
+    else if (by_top_k)
+        rows = split_max_rows(top_k, n_tiles);
+    else if (by_top_p || a.mask || penalties)
+        rows = split_max_rows(slow, n_tiles);
+    else
+        rows = split_max_rows(fast, n_tiles);
+    if (batch > rows)
         return;
     uint32_t slices = kPlaces / batch;
     slices = slices < mk::kMaxSlices ? slices : mk::kMaxSlices;
     const uint32_t per = (n_tiles + slices - 1) / slices; // tiles per slice
     a.split_w = per * kTile;
-    a.parts = s->split_parts + (size_t)set * mk::kSplitMaxRows * mk::kMaxSlices;
-    a.tickets = s->split_tickets + (size_t)set * mk::kSplitMaxRows;
+    const size_t own_part = set > 0 ? 1u : 0u;
+    a.parts = s->split_parts + own_part * mk::kSplitMaxRows * mk::kMaxSlices;
+    a.tickets = s->split_tickets + own_part * mk::kSplitMaxRows;
 }
 
 } // namespace
@@ -346,7 +391,7 @@ int mk_sampler_sample_batch(mk_sampler* s, const mk_rows* rows, const float* u, 
     fill_out(a, out);
     a.u = u;
     a.mode = mk::kModeSample;
-    split_rows(a, s, rows->batch, 0);
+    split_rows(a, s, rows->batch, -1);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, (cudaStream_t)stream));
     return MK_OK;
 }
@@ -417,7 +462,7 @@ int mk_sampler_verify_batch(mk_sampler* s, const mk_rows* rows, const int32_t* d
     a.draft = draft;
     a.accepted = accepted;
     a.mode = mk::kModeVerify;
-    split_rows(a, s, rows->batch, 0);
+    split_rows(a, s, rows->batch, -1);
     MK_CUDA(mk::launch_row_kernel(a, rows->batch, (cudaStream_t)stream));
     return MK_OK;
 }
