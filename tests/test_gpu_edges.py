@@ -119,7 +119,7 @@ def test_long_history_and_heavy_repeats(gpu_sampler_factory, ref):
     compare_sample(res, want, cap=1024)
 
 
-def test_unaligned_rows_take_the_plain_load_path(gpu_sampler_factory, ref):
+def test_unaligned_rows(gpu_sampler_factory, ref):
     import torch
     v, b = 10001, 5
     inp = Inputs(121, b, v, ld=v + 2)            # ld % 4 != 0: rows are not 16-byte aligned
@@ -198,7 +198,7 @@ def test_lists_a_little_longer_than_the_on_chip_sort(gpu_sampler_factory, ref, p
 
 
 def test_second_pass_only_for_rows_that_ask(gpu_sampler_factory, ref):
-    """top_p alone: the first launch keeps the 24 largest elements per row; rows whose nucleus is longer stream a
+    """top_p alone: the first launch keeps the 20 largest elements per row; rows whose nucleus is longer are read a
     second time. Flat and peaked rows share a batch, with histories and a mask, and the same handle is then used for
     a batch in which no row asks for the second pass: marks left by one call must not leak into the next."""
     v, b, cap = 50021, 8, 4096

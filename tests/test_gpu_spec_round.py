@@ -46,8 +46,8 @@ def _cpu_round(ref, p, logits, drafts, forced, u, hist):
 ], ids=["penalised", "nucleus+forced", "greedy+forced", "top_p alone+forced"])
 @pytest.mark.parametrize("v,n_seq", [(40003, 64), (129280, 24)], ids=["ragged_rows", "aligned_rows"])
 def test_rounds_of_four_drafts_and_a_bonus_row(gpu_sampler_factory, ref, params, with_forced, v, n_seq):
-    """Rows of 40003 columns are not 16-byte aligned and take the kernel's plain-load path, rows of 129280 columns
-    the bulk-copy path: the round's bookkeeping is the same on both."""
+    """Rows of 40003 columns start at any float and are taken from the 16-byte boundary before it, rows of 129280 columns lie on
+    one: the round's bookkeeping is the same for both."""
     import torch
     n_drafts, cap, rounds = 4, 256, 3
     n_pos = n_drafts + 1
