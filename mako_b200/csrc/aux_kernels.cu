@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
                 for (uint32_t i = r0; i < r1; ++i)
                     mine += (double)q_at(i);
                 double inc = mine;
-    #pragma unroll
+#pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const double y = __shfl_up_sync(full, inc, o);
                     if ((int)lane >= o)
@@ -274,65 +274,65 @@ __global__ void __launch_bounds__(kMergeThreadsFew) vp_merge_kernel(const VpMerg
             if (lane == 0)
                 s_settled = settled ? 1u : 0u;
             if (settled) {
-            if (cut_k && !use_topp)
-                n_decide = n;
-            else if (cut_k)
-                n_decide = min(n_decide, prm.top_k);
-            // count members per shard among the deciding set
-            for (uint32_t i = lane; i < n_decide; i += 32u)
-                atomicAdd(&s_shard_in[tag_at(i) >> kShardShift], 1u);
-            __syncwarp();
-            bool cut_short = false;
-            for (uint32_t g = lane; g < a.n_shards && g < 64u; g += 32u) {
-                const uint32_t hdr = s_hdr[g];
-                const uint32_t ng = hdr & 0xffffu;
-                const bool more = (hdr & 0x40000000u) != 0;
-                cut_short = cut_short || (hdr & 0x80000000u) || (more && ng > 0 && s_shard_in[g] >= ng);
-            }
-            if (__any_sync(full, cut_short))
-                flags |= MK_FLAG_VP_TRUNCATED;
-            // 32 candidates a step, lanes past the end of the list holding zeros (which change nothing and never win): the
-            // shuffles do not depend on the chains, which then run at the adder's latency
-            float total = 0.0f;
-            for (uint32_t base = 0; base < n; base += 32u) {
-                const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-    #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    total = __fadd_rn(total, __shfl_sync(full, q, j));
-            }
-            float r = __fmul_rn(a.u[row], total);
-            const float eps = 1e-6f * total;
-            uint32_t hit = n - 1u;
-            float q_hit = q_at(n - 1u);
-            for (uint32_t base = 0; base < n; base += 32u) {
-                const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
-                uint32_t short_of = 0u;
-                float rr = r;
-    #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const float qj = __shfl_sync(full, q, j);
-                    short_of |= (rr < qj) ? (1u << j) : 0u;
-                    rr = __fsub_rn(rr, qj);
+                if (cut_k && !use_topp)
+                    n_decide = n;
+                else if (cut_k)
+                    n_decide = min(n_decide, prm.top_k);
+                // count members per shard among the deciding set
+                for (uint32_t i = lane; i < n_decide; i += 32u)
+                    atomicAdd(&s_shard_in[tag_at(i) >> kShardShift], 1u);
+                __syncwarp();
+                bool cut_short = false;
+                for (uint32_t g = lane; g < a.n_shards && g < 64u; g += 32u) {
+                    const uint32_t hdr = s_hdr[g];
+                    const uint32_t ng = hdr & 0xffffu;
+                    const bool more = (hdr & 0x40000000u) != 0;
+                    cut_short = cut_short || (hdr & 0x80000000u) || (more && ng > 0 && s_shard_in[g] >= ng);
                 }
-                if (short_of) { // the first candidate the draw falls short of; the remainder in front of it, once more
-                    const int jh = __ffs((int)short_of) - 1;
-                    for (int j = 0; j < jh; ++j)
-                        r = __fsub_rn(r, __shfl_sync(full, q, j));
-                    hit = base + (uint32_t)jh;
-                    q_hit = __shfl_sync(full, q, jh);
-                    if ((hit > 0 && r < eps) || (hit + 1 < n && __fsub_rn(q_hit, r) < eps))
-                        flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
-                    break;
+                if (__any_sync(full, cut_short))
+                    flags |= MK_FLAG_VP_TRUNCATED;
+                // 32 candidates a step, lanes past the end of the list holding zeros (which change nothing and never win): the
+                // shuffles do not depend on the chains, which then run at the adder's latency
+                float total = 0.0f;
+                for (uint32_t base = 0; base < n; base += 32u) {
+                    const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        total = __fadd_rn(total, __shfl_sync(full, q, j));
                 }
-                r = rr;
-            }
-            if (lane == 0) {
-                if (a.token) a.token[row] = (int32_t)(tag_at(hit) & kIdMask);
-                if (a.prob) a.prob[row] = __fdiv_rn(q_hit, total);
-                if (a.flags) a.flags[row] = flags;
-                if (a.n_cand) a.n_cand[row] = n;
-                s_nfinal = n;
-            }
+                float r = __fmul_rn(a.u[row], total);
+                const float eps = 1e-6f * total;
+                uint32_t hit = n - 1u;
+                float q_hit = q_at(n - 1u);
+                for (uint32_t base = 0; base < n; base += 32u) {
+                    const float q = (base + lane < n) ? q_at(base + lane) : 0.0f;
+                    uint32_t short_of = 0u;
+                    float rr = r;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const float qj = __shfl_sync(full, q, j);
+                        short_of |= (rr < qj) ? (1u << j) : 0u;
+                        rr = __fsub_rn(rr, qj);
+                    }
+                    if (short_of) { // the first candidate the draw falls short of; the remainder in front of it, once more
+                        const int jh = __ffs((int)short_of) - 1;
+                        for (int j = 0; j < jh; ++j)
+                            r = __fsub_rn(r, __shfl_sync(full, q, j));
+                        hit = base + (uint32_t)jh;
+                        q_hit = __shfl_sync(full, q, jh);
+                        if ((hit > 0 && r < eps) || (hit + 1 < n && __fsub_rn(q_hit, r) < eps))
+                            flags |= MK_FLAG_NEAR_CDF_BOUNDARY;
+                        break;
+                    }
+                    r = rr;
+                }
+                if (lane == 0) {
+                    if (a.token) a.token[row] = (int32_t)(tag_at(hit) & kIdMask);
+                    if (a.prob) a.prob[row] = __fdiv_rn(q_hit, total);
+                    if (a.flags) a.flags[row] = flags;
+                    if (a.n_cand) a.n_cand[row] = n;
+                    s_nfinal = n;
+                }
             }
         }
         __syncthreads();
@@ -856,13 +856,13 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
             fetch(v0, h);
         }
         if constexpr (kSeq == 1) {
-    #pragma unroll
+#pragma unroll
             for (int b = 0; b < kSeq; ++b) {
                 if ((uint32_t)b >= n_seq)
                     break;
                 const float4 e0 = *reinterpret_cast<const float4*>(&s_e[b][4u * lane]);
                 const float4 e1 = *reinterpret_cast<const float4*>(&s_e[b][4u * lane + 128u]);
-    #pragma unroll
+#pragma unroll
                 for (uint32_t r = 0; r < kRows; ++r) {
                     float acc = h[r][0].x * e0.x;
                     acc = fmaf(h[r][0].y, e0.y, acc);
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(kPickThreads, kSeq == 1 ? 4 : 2) draft_score_k
                     acc = fmaf(h[r][1].y, e1.y, acc);
                     acc = fmaf(h[r][1].z, e1.z, acc);
                     acc = fmaf(h[r][1].w, e1.w, acc);
-    #pragma unroll
+#pragma unroll
                     for (int o = 16; o > 0; o >>= 1)
                         acc += __shfl_xor_sync(0xffffffffu, acc, o);
                     const uint32_t v = v0 + r;

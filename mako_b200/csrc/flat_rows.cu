@@ -9,7 +9,7 @@
 //             than a few thousand elements, that bound is the cut, and all of them get exact weights;
 //   collect   one pass over the row keeps everything above that weight — the nucleus and a few per cent more — and sums
 //             the approximate weights of the rest, one by one in double;
-//   order     exact weights; the list is dealt into buckets of about eight, of equal counts rather than equal widths, each whose
+//   order     exact weights; the list is dealt into buckets of about six, of equal counts rather than equal widths, whose
 //             members rank themselves, a lane each (a warp or the CTA sorts where equal weights crowd a bucket);
 //   draw      double prefix sums for top_p, then the float total and the walk as scans (list_chain.cuh).
 // A cut that proves too tight (a list that ends before the nucleus does) is replaced by the bound that cannot be, and the row
@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 }
                 const double rest = block_sum(s, tail, 0);
                 n = s.n_list;
-            if (a.timing && tid == 0)
-                a.timing[(size_t)row * 64 + 17] = global_ns();
+                if (a.timing && tid == 0)
+                    a.timing[(size_t)row * 64 + 17] = global_ns();
                 // exact weights, in place of the logits; their sum; how many there are in each class of the float's own octaves
                 for (uint32_t i = tid; i < kClasses; i += kFlatThreads)
                     cls2[i] = make_uint2(0u, 0u);
@@ -493,8 +493,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 const double sum = block_sum(s, exact, 1);
                 const double total = sum + rest;
                 const double band = 1e-5 * rest + 0x1p-36 * total, want = (double)cfg.top_p * total;
-            if (a.timing && tid == 0)
-                a.timing[(size_t)row * 64 + 18] = global_ns();
+                if (a.timing && tid == 0)
+                    a.timing[(size_t)row * 64 + 18] = global_ns();
                 // buckets: each class gets as many as its count asks for
                 uint32_t in_class = tid < kClasses ? cls2[tid].y : 0u, n_in, n_buckets;
                 block_exclusive(s, in_class, n_in);
@@ -566,8 +566,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                                 ((unsigned long long)(c[k].x + ~0x3f800000u) << 32) | c[k].y; // pack_by_weight's key
                 }
                 __syncthreads();
-            if (a.timing && tid == 0)
-                a.timing[(size_t)row * 64 + 19] = global_ns();
+                if (a.timing && tid == 0)
+                    a.timing[(size_t)row * 64 + 19] = global_ns();
                 for (uint32_t b = tid; b < n_buckets; b += kFlatThreads)
                     if (ends[b] - (b ? ends[b - 1u] : 0u) > 32u) {
                         const uint32_t at_big = atomicAdd(&s.n_big, 1u);
@@ -626,8 +626,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                     }
                     __syncthreads();
                 }
-            if (a.timing && tid == 0)
-                a.timing[(size_t)row * 64 + 20] = global_ns();
+                if (a.timing && tid == 0)
+                    a.timing[(size_t)row * 64 + 20] = global_ns();
                 // ---- top_p (sampler.cpp:44-61): the shortest prefix whose double sum is not below `want` --------------------
                 auto q_key = [&](uint32_t i) -> float { return __uint_as_float(~(uint32_t)(keys[i] >> 32)); };
                 const uint32_t run_len = ((n_in + kFlatThreads - 1u) / kFlatThreads) | 1u;

@@ -51,10 +51,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
     return ok != 0;
 }
 
-// Bounded wait: gives up after `limit` probes and reports false, so that a lost copy or a logic error ends the
-// kernel with a status instead of hanging the GPU. (2^17 probes of up to 20 us each: a few seconds at most.)
-// The same wait by polling (no suspension): for the one lane whose reaction time is on a ring stage's round trip.
-// Bounded like the other: about a million probes.
+// The wait below by polling (no suspension): for the one lane whose reaction time is on a ring stage's round trip.
+// Bounded like the other: four million probes.
 __device__ __forceinline__ bool mbar_wait_poll(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22))
 {
     for (uint32_t i = 0; i < limit; ++i) {
@@ -72,6 +70,8 @@ __device__ __forceinline__ bool mbar_wait_poll(uint64_t* bar, uint32_t parity, u
     return false;
 }
 
+// Bounded wait: gives up after `limit` probes and reports false, so that a lost copy or a logic error ends the
+// kernel with a status instead of hanging the GPU. (2^17 probes of up to 20 us each: a few seconds at most.)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 17))
 {
     for (uint32_t i = 0; i < limit; ++i)

@@ -21,14 +21,17 @@
 //                 collection of every element that can still become a candidate: the keep thresholds of min_p,
 //                 top_k and top_p are all lower-bounded by a function of the running maximum (or, for top_k, of a
 //                 histogram of the reader threads' maxima) that only rises while the row streams, so filtering with
-//                 the current bound keeps a superset of the final candidates. The loop exists in five variants.
+//                 the current bound keeps a superset of the final candidates. The loop exists in five variants, each
+//                 with and without a mask.
 //   finish        exact weights q = expf((l - max) * inv_t) for the few collected elements with the host library's
 //                 float exponential (device_expf.cuh), min_p, top_k, top_p, and the sequential float total and walk
 //                 of the draw — in the reference's precision and order, because token ids depend on both. Up to 64
 //                 candidates: one warp, in registers. Steps only unusual rows need (long lists) live in functions of
 //                 their own.
-//   second pass   top_p alone: the first launch keeps the 24 largest elements; a row whose nucleus that does not
-//                 settle marks itself, and a second launch of this kernel streams the marked rows again.
+//   second pass   top_p alone: the first launch keeps the 20 largest elements; a row whose nucleus that does not
+//                 settle marks itself, and a second launch reads the marked rows again: the flat rows' kernel (flat_rows.cu), or,
+//                 for the rows that one does not take (speculative rounds, more than 4096 edits, vocabularies above 163840
+//                 columns; of these the first launch keeps 24), this kernel with the loose bound.
 //   split launch  a few rows: a second grid dimension over slices of the columns; every CTA keeps what its slice's bounds
 //                 leave, the last one of a row to arrive narrows that to the row's own bounds and finishes.
 //

@@ -133,8 +133,8 @@ class BatchSampler:
         check(lib.mk_sampler_set_overlap(self._h, int(mode)))
 
     def set_split(self, on: bool) -> None:
-        """Whether a small batch (at most 8 rows, shared parameters, drawing under a top_k of at most 64) has every
-        row split over many CTAs and merged (the default) or runs as one CTA per row (mk_sampler_set_split)."""
+        """Whether a call of at most 148 rows may have every row's columns split over up to 64 CTAs, the last of which draws
+        (the default, where it is faster), or runs as one CTA per row (mk_sampler_set_split)."""
         check(lib.mk_sampler_set_split(self._h, 1 if on else 0))
 
     # -- argument marshalling -----------------------------------------------------------------------------------
