@@ -24,7 +24,7 @@ struct RowCfg {
     float rep, presence, frequency;
     bool greedy, hist_mode, need_sum, use_topp, pen_active, optimistic;
     float delta_w;      // keep elements with l >= running max - delta_w
-    bool force_none;    // inv_t is inf/NaN, or min_p a NaN: no weight can be a candidate's
+    bool force_none;    // inv_t is inf/NaN: no finite weight can exist
 };
 
 __device__ __forceinline__ unsigned long long global_ns()
@@ -56,8 +56,7 @@ __device__ __forceinline__ RowCfg make_cfg(const mk_sampling_params& p, uint32_t
     const bool minp_on = c.minp_eff > 0.0f;
     // The float total over "all candidates" is only needed when top_p is the only truncation.
     c.need_sum = !c.greedy && c.use_topp && !minp_on && !c.hist_mode;
-    c.force_none = !c.greedy && (!(c.inv_t < __int_as_float(0x7f800000)) || !(c.inv_t == c.inv_t) ||
-                                 (mode != kModeVpLocal && c.minp_eff != c.minp_eff));
+    c.force_none = !c.greedy && (!(c.inv_t < __int_as_float(0x7f800000)) || !(c.inv_t == c.inv_t));
     // top_p alone: the first launch bets that the nucleus lies within the largest few elements and keeps
     // only those (the top_k histogram bound, with no top_k cut afterwards); a row whose nucleus does not close within
     // what was kept asks for a second launch, which keeps everything the mass bound allows.

@@ -2062,8 +2062,10 @@ __global__ void __launch_bounds__(kThreads, 2) row_pipeline_kernel(const RowKern
     }
 
     // Top_p alone, and what was kept does not hold the nucleus, or holds too much to tell here: the row is left to the flat rows'
-    // kernel, with its maximum and total. (Where no weight can exist there is nothing to look for.)
-    if (cfg.optimistic && cfg.hist_k == kNucleusGuess && !s.nan0 && !cfg.force_none && fabsf(m) < __int_as_float(0x7f800000)) {
+    // kernel, with its maximum and total. (Where no weight can exist, or none be at least a min_p that is a NaN, there is nothing to
+    // look for.)
+    if (cfg.optimistic && cfg.hist_k == kNucleusGuess && !s.nan0 && !cfg.force_none && cfg.minp_eff == cfg.minp_eff &&
+        fabsf(m) < __int_as_float(0x7f800000)) {
         if (!weighed) // what was collected is not in the streamed sum
             weigh_collected(scratch, min(s.ncand, scratch_cap), m, cfg.inv_t, fsum);
         if (tid == 0) {
