@@ -492,6 +492,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) flat_row_kernel(const RowKern
                 }
                 const double sum = block_sum(s, exact, 1);
                 const double total = sum + rest;
+                // (an approximate weight: ex2.approx takes 2^-22, its argument's rounding 4e-8 an octave below the maximum: 2e-6 at most
+                // where a weight still counts; the sum is double)
                 const double band = 1e-5 * rest + 0x1p-36 * total, want = (double)cfg.top_p * total;
                 if (a.timing && tid == 0)
                     a.timing[(size_t)row * 64 + 18] = global_ns();

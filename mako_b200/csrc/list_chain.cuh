@@ -14,7 +14,8 @@
 // Ties are rare: where no run of a round has one, the increments are plain numbers, and as long as their sum stays inside the binade
 // (and, in a walk, above the largest weight) a round is one reduction. Such rounds are taken by the whole CTA, up to the first
 // warp's share that is not like that; one warp takes the others (256 candidates). What bounds both is a round's latency, not
-// the number of candidates.
+// the number of candidates. (128 masked rows of 3000 candidates: 61.9 us with a scan over the CTA's threads in every round, 60.3 so; lists
+// of tens of thousands take the same either way.)
 #pragma once
 #include <cstdint>
 
